@@ -88,6 +88,9 @@ struct HItem {
   const int32_t* st_n;
   double* H;
   long long blk0, nblk;
+  // the first Z column of each initial slot (column colI of a slot follows
+  // colI later); null: column colI * nslotI + slot
+  const int32_t* slotcol;
 };
 // One unit's Y rows of a batched digit build (split_build_y_digits' arguments):
 // rows [row0, row0 + rows) of the round's Y.
@@ -98,6 +101,27 @@ struct YItem {
   const double* rep;
   int ld, ndeg, Ntot, nslot;
   long long row0, rows;
+};
+// The default split scheme (split8.cu): one column group of the half-line-
+// strength GEMM, nI * ndeg columns of one (unit, slot).
+struct YItem8 {
+  const double* vecs;
+  const int32_t* ivec;
+  const int32_t* ys;     // Basis::d_ys, d_yc from the slot on (d_yc: from the
+  const double* yc;      // first degenerate component wanted)
+  const int32_t* vlist;  // [32 nk] function at each K position of the group's band
+  uint8_t* out;          // the band's first B tile
+  int32_t* e_out;        // the band's column exponents
+  int ld, ndeg, nent, nk;
+  long long nsv;         // nslot * N
+  int col0;              // first column within the band
+  int rows;              // columns
+  long long blk0;        // first grid block
+};
+// One 128-row tile of a GEMM's A operand and where its rows go in C.
+struct ATile {
+  int32_t tile, rows;
+  int64_t coff;
 };
 // The column norms of several H in one launch: item k's columns are
 // [col0, col0 + ncol) of the grid.
@@ -160,6 +184,19 @@ struct Basis {
   // (slot, v) -> roots CSR; depends on the dipole size N
   int y_N = -1;
   DevArray<int32_t> d_yptr, d_yroot;
+  // most symmetrised functions with a non-zero coefficient on one root, per
+  // gamma, and most roots on one (slot, v)
+  std::vector<int32_t> root_ent;
+  int32_t y_mult = 0;
+  // Y as a table (default split scheme), per gamma (made on first use): entry
+  // e < E of (slot, v) is coefficient c[(d * E + e) * nslot * N + slot * N + v] of
+  // symmetrised function s[e * nslot * N + slot * N + v], in the CSR's order;
+  // absent entries are 0, 0.  E = root_ent * y_mult.
+  std::vector<DevArray<int32_t>> d_ys;
+  std::vector<DevArray<double>> d_yc;
+  // row of Z of each root in the order of a VibPlan (split8.h), and that plan
+  uint64_t z_uid = 0;
+  DevArray<int32_t> d_root_z;
   // largest iroot_correlat_j0 (checked against N without a pass over the roots)
   int32_t iroot_max = -1;
   // device copies of the key -> slot map and of the half-line-strength terms
@@ -210,6 +247,8 @@ struct Level {
 };
 
 struct SplitState;  // split-precision state (split.cu)
+struct Split8;      // the default scheme's (split8.cu)
+struct HlsPlan8;    // gi_half_ls in the default scheme: tables of a call shape (host.cu)
 struct Server;      // serving loop (serve.cu)
 struct TroveMeta;   // level descriptors of a TROVE job (trove.cu)
 struct DipoleStream;  // dipole kept in host memory, streamed in panels (stream.cu)
@@ -226,6 +265,7 @@ struct JobSel {
 
 struct Ctx {
   SplitState* split = nullptr;
+  Split8* split8 = nullptr;
   int tune_mode = 0;          // split GEMM autotuner (gi_set_tuning)
   std::string tune_path;
   Ctx* parent = nullptr;      // a serving worker shares its parent's model state
@@ -329,6 +369,7 @@ struct Ctx {
   };
   std::vector<HlsGraph> hls_graphs;  // most recently used first
   uint64_t hls_last_sig = 0;         // the last call run eagerly
+  std::vector<std::shared_ptr<HlsPlan8>> hls_plans8;  // most recently used first, at most 8
   DevArray<int32_t> hls_iv;
   DevArray<double> w_y, w_z, w_h, w_t, w_EI;
   DevArray<unsigned long long> w_counter;
@@ -342,6 +383,13 @@ struct Ctx {
   DevArray<long long> w_hfirst; // their first grid blocks, contiguous for the lookup
   DevArray<NormItem> w_nitems; // the H column norms of every group
   DevArray<YItem> w_yitems;    // the Y digit builds of every round (one launch per round)
+  // the default split scheme's tables of a run: column groups of Y and the
+  // first one of every 64 columns, K slice and function lists of the bands, row
+  // tiles of the bands, first Z columns of every unit's slots
+  DevArray<YItem8> w_yitems8;
+  DevArray<int32_t> w_ytile8, w_vl8, w_slotcol;
+  DevArray<uint16_t> w_kl8;
+  DevArray<ATile> w_at8;
   DevArray<RefineRec> w_rec;   // lines handed to the exact re-evaluation
   int64_t refine_max = 0;      // doubtful lines re-evaluated per run (gi_set_refine)
   DevArray<int32_t> w_stencil_n, w_levelI, w_levelF;
@@ -428,10 +476,16 @@ int dipole_panel_rows(const Ctx* c);
 cudaError_t launch_build_y(const double* vecs, int ld, const int32_t* ivec, int nI, int ndeg,
                            const Basis& b, int gamma, int degen, int N, int Kp, double* Y,
                            cudaStream_t s, int d0 = 0);
+// out[r] = zpos[root_v[r]].
+cudaError_t launch_root_z(const Basis& b, const int32_t* zpos, int32_t* out, cudaStream_t s);
+// Basis::d_ys / d_yc of gamma (E entries per position) from its CSR.
+cudaError_t launch_y_table(const Basis& b, int gamma, int degen, int N, int E, int32_t* ys,
+                           double* yc, cudaStream_t s);
 cudaError_t launch_build_h(const double* Z, size_t zstride_c, int ldz, int nslotI, int ndegI,
                            int nI, const Basis& bF, int gammaF, int degF, int nsizeF, int ldh,
                            const StencilTerm* st, const int32_t* st_n, int st_max, double* H,
-                           cudaStream_t s);
+                           cudaStream_t s, const int32_t* root_z = nullptr,
+                           const int32_t* slotcol = nullptr);
 HItem make_h_item(const double* Z, size_t zstride_c, int ldz, int nslotI, int ndegI, int nI,
                   const Basis& bF, int gammaF, int degF, int nsizeF, int ldh,
                   const StencilTerm* st, const int32_t* st_n, int st_max, double* H,
@@ -443,11 +497,13 @@ cudaError_t launch_half_ls_prim(const double* Z, size_t zstride_c, int ldz, cons
                                 const StencilTerm* st, const int32_t* st_n, int st_max,
                                 double* h, cudaStream_t s);
 // h from a Z held as K-split partial products Zp[p][col][c * cstride + v]
-// (Zp already offset to the first column of the wanted degenerate component).
+// (Zp already offset to the first column of the wanted degenerate component);
+// root_z / slotcol: rows and columns of Z of the default split scheme.
 cudaError_t launch_half_ls_prim_parts(const double* Zp, int nparts, size_t pstride, int ldz,
                                       int cstride, const Basis& bF, const StencilTerm* st,
                                       const int32_t* st_n, int st_max, double* h,
-                                      cudaStream_t s);
+                                      cudaStream_t s, const int32_t* root_z = nullptr,
+                                      const int32_t* slotcol = nullptr);
 
 // out[k] = exp(-(E[k] - zpe) beta) (the epilogue's initial-level factor).
 cudaError_t launch_pack_lines(const gi_line* in, gi_line_compact* out, long long n,

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -12,7 +13,7 @@
 #include <numeric>
 
 #include "engine.h"
-#include "split.h"
+#include "split8.h"
 
 namespace gi {
 
@@ -137,11 +138,10 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
   }
   b.slot_of_key.assign(2 * b.J + 2, -1);
   b.nslot = 0;
-  for (int key = 0; key < 2 * b.J + 2; key++) {
-    bool any = false;
-    for (int r = 0; r < D && !any; r++) any = b.root_key[r] == key;
-    if (any) b.slot_of_key[key] = b.nslot++;
-  }
+  std::vector<uint8_t> has_key(2 * b.J + 2, 0);
+  for (int r = 0; r < D; r++) has_key[b.root_key[r]] = 1;
+  for (int key = 0; key < 2 * b.J + 2; key++)
+    if (has_key[key]) b.slot_of_key[key] = b.nslot++;
   // ijterms (trove_functions.cpp:927-966) and Ntotal consistency
   b.ijterms.assign((size_t)b.ncase * nrep, 0);
   for (int g = 0; g < nrep; g++) {
@@ -172,6 +172,23 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
       const int s0 = b.ijterms[it + (size_t)g * b.ncase];
       const int ne = b.Nsym[g + (size_t)it * nrep];
       for (int j = 0; j < ne; j++) b.s_case[g][s0 + j] = it;
+    }
+  }
+  // most non-zero coefficients on one root, per gamma
+  b.root_ent.assign(nrep, 0);
+  for (int g = 0; g < nrep; g++) {
+    const int nt = b.Ntotal[g], dg = c->degen[g];
+    for (int r = 0; r < D; r++) {
+      const int ic = b.icontr2icase[r], s0 = b.ijterms[ic + (size_t)g * b.ncase];
+      const int ne = b.Nsym[g + (size_t)ic * nrep];
+      const double* rep = b.repres[g].data() + (size_t)b.icontr2icase[r + D] * dg * nt;
+      int n = 0;
+      for (int j = 0; j < ne; j++) {
+        bool any = false;
+        for (int d = 0; d < dg; d++) any = any || rep[s0 + j + (size_t)d * nt] != 0.0;
+        n += any;
+      }
+      b.root_ent[g] = std::max(b.root_ent[g], n);
     }
   }
   // device copies
@@ -219,12 +236,35 @@ gi_status ensure_ycsr(Ctx* c, Basis& b) {
       return fail(c, GI_ERR_ARG, "basis J=%d: iroot_correlat_j0[%d]=%d >= N=%d", b.J, r, b.iroot[r], N);
     ptr[(size_t)b.slot_of_key[b.root_key[r]] * N + b.iroot[r] + 1]++;
   }
-  for (size_t i = 0; i + 1 < ptr.size(); i++) ptr[i + 1] += ptr[i];
+  b.y_mult = 0;
+  for (size_t i = 0; i + 1 < ptr.size(); i++) {
+    b.y_mult = std::max(b.y_mult, ptr[i + 1]);
+    ptr[i + 1] += ptr[i];
+  }
   std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
   for (int r = 0; r < b.D; r++) roots[fill[(size_t)b.slot_of_key[b.root_key[r]] * N + b.iroot[r]]++] = r;
   GI_CUDA(c, b.d_yptr.upload(ptr));
   GI_CUDA(c, b.d_yroot.upload(roots));
+  b.d_ys.clear();
+  b.d_yc.clear();
   b.y_N = N;
+  return GI_OK;
+}
+
+// The basis's Y table of gamma for the default split scheme (after
+// ensure_ycsr, under the model lock).
+gi_status ensure_y_table(Ctx* c, Basis& b, int g) {
+  b.d_ys.resize(c->nrep);
+  b.d_yc.resize(c->nrep);
+  if (b.d_ys[g].p) return GI_OK;
+  const size_t n = (size_t)b.root_ent[g] * b.y_mult * b.nslot * c->N;
+  GI_CUDA(c, b.d_yc[g].alloc(c->degen[g] * n));
+  GI_CUDA(c, b.d_ys[g].alloc(n));
+  const cudaError_t e = launch_y_table(b, g, c->degen[g], c->N, b.root_ent[g] * b.y_mult,
+                                       b.d_ys[g].p, b.d_yc[g].p, cudaStreamLegacy);
+  if (e == cudaSuccess) GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
+  if (e != cudaSuccess) b.d_ys[g].reset();
+  GI_CUDA(c, e);
   return GI_OK;
 }
 
@@ -550,23 +590,54 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   // is planned and uploaded here, so the launch sequence never waits.
   const int N = c->N, Kp = c->Kp;
   const size_t ws_limit = c->budget ? c->budget / 2 : ((size_t)64 << 30);
-  const int s_digits = (P.precision == GI_PREC_SPLIT) ? split_digits(c) : 0;
+  const size_t digit_bytes = (P.precision == GI_PREC_SPLIT) ? split_digit_bytes(c) : 0;
+  // the default split scheme: the order of the vibrational functions in its
+  // digits and in Z
+  const bool s8 = P.precision == GI_PREC_SPLIT && split8_selected(c);
+  const VibPlan* vp = nullptr;
+  if (s8) {
+    gi_status s = split_prepare(c);
+    if (s != GI_OK) return s;
+    vp = vib_plan(c, &s);
+    if (!vp) return s;
+    std::lock_guard<std::mutex> lk(c->mmu());
+    for (auto& kv : c->bases)
+      if ((s = ensure_root_z(c, *kv.second, *vp)) != GI_OK) return s;
+    for (auto& pp : pairs) {
+      const Block& b = *pp.I->blk;
+      if ((s = ensure_y_table(c, *c->bases[b.J], b.gamma)) != GI_OK) return s;
+    }
+  }
+  const int ldz = s8 ? vp->ldz : Kp;
   struct Unit {
     BlockPlan* I;
     std::vector<PairPlan*> pairs;
     int nI, ncolY;
     size_t off;   // into the record/level and energy tables
     size_t ycol;  // first Y/Z column of the unit within its round
+    size_t sc;    // default split scheme: into the slot column table
+  };
+  // columns of one (unit, slot) in a band of the default split scheme's GEMM
+  struct Group8 {
+    size_t unit;
+    int slot, rows;
+    size_t col0;  // within the band
   };
   struct Round {
     std::vector<Unit> units;
     size_t ncolY = 0;
+    size_t ncolZ = 0;  // columns of Z (the bands padded to whole tiles)
+    std::vector<Band8> bands;
+    std::vector<std::vector<Group8>> groups8;  // per band
+    size_t bbytes = 0;                         // B digits
+    double flops8 = 0.0;                       // digit products of the half-ls GEMM
   };
   std::vector<Round> rounds(1);
   std::vector<int32_t> h_ivec;  // per unit: nI record ids then nI level ids
   std::vector<double> h_EI;
   // bytes per Y column: Y, 3 Z, digit planes; plus the widest H/T per column
-  const size_t per_col = (size_t)Kp * (8 * 4 + 2 * (size_t)s_digits);
+  const size_t per_col = s8 ? (size_t)ldz * 24 + (size_t)vp->nk * 32 * digit_bytes
+                            : (size_t)Kp * (8 * 4 + digit_bytes);
   size_t round_bytes = 0;
   for (auto& kv : plans) {
     BlockPlan& I = kv.second;
@@ -580,7 +651,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     for (auto* pp : mine) {
       const Block& fb = *pp->F->blk;
       per_vec += (size_t)ndegI * c->degen[fb.gamma] *
-                 (fb.ld * (8 + 2 * (size_t)s_digits) + round_up(fb.nvec, 2) * 8);
+                 (fb.ld * (8 + digit_bytes) + round_up(fb.nvec, 2) * 8);
     }
     const int chunk =
         (int)std::min<size_t>(std::max<size_t>(1, ws_limit / per_vec), I.ivec.size());
@@ -591,13 +662,74 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
         round_bytes = 0;
       }
       Round& R = rounds.back();
-      Unit u{&I, mine, nI, nI * ndegI * nslot, h_EI.size(), R.ncolY};
+      Unit u{&I, mine, nI, nI * ndegI * nslot, h_EI.size(), R.ncolY, 0};
       for (int i = 0; i < nI; i++) h_EI.push_back(I.blk->energies[I.ivec[i0 + i]]);
       for (int i = 0; i < nI; i++) h_ivec.push_back(I.ivec[i0 + i]);
       for (int i = 0; i < nI; i++) h_ivec.push_back(I.level_of_rec[I.ivec[i0 + i]]);
       R.ncolY += u.ncolY;
       round_bytes += per_vec * nI;
       R.units.push_back(std::move(u));
+    }
+  }
+  // The bands of a round's half-line-strength GEMM: the columns of every
+  // (unit, slot) whose Y is non-zero on the same classes of functions and whose
+  // Z is read on the same classes, per component.
+  std::vector<int32_t> h_slotcol;
+  for (Round& R : rounds) {
+    R.ncolZ = R.ncolY;
+    if (!s8) continue;
+    std::map<std::array<uint32_t, 4>, size_t> index;
+    for (size_t k = 0; k < R.units.size(); k++) {
+      Unit& u = R.units[k];
+      const Block& b = *u.I->blk;
+      const Basis& bI = *c->bases[b.J];
+      u.sc = h_slotcol.size();
+      h_slotcol.resize(u.sc + bI.nslot);
+      for (int slot = 0; slot < bI.nslot; slot++) {
+        std::array<uint32_t, 4> key{vib_support(*vp, bI, b.gamma, slot), 0, 0, 0};
+        if (!key[0]) key[0] = 1;  // an all-zero column: contracted over any class
+        vib_rows_needed(c, *vp, bI, igamma_pair[b.gamma], slot, key.data() + 1);
+        auto it = index.find(key);
+        if (it == index.end()) {
+          if (R.bands.size() == (size_t)kMaxProb8) {  // more kinds than a launch takes: one for the rest
+            Band8& last = R.bands.back();
+            last.kset |= key[0];
+            for (int q = 0; q < 3; q++) last.rset[q] |= key[q + 1];
+            it = index.emplace(key, R.bands.size() - 1).first;
+          } else {
+            it = index.emplace(key, R.bands.size()).first;
+            R.bands.emplace_back();
+            R.groups8.emplace_back();
+            R.bands.back().kset = key[0];
+            for (int q = 0; q < 3; q++) R.bands.back().rset[q] = key[q + 1];
+          }
+        }
+        Band8& band = R.bands[it->second];
+        const int rows = u.nI * c->degen[b.gamma];
+        R.groups8[it->second].push_back(Group8{k, slot, rows, band.ncol});
+        band.ncol += rows;
+      }
+    }
+    R.ncolZ = 0;
+    for (size_t q = 0; q < R.bands.size(); q++) {
+      Band8& band = R.bands[q];
+      band.col0 = R.ncolZ;
+      band.boff = R.bbytes;
+      R.ncolZ += (band.ncol + kCols8 - 1) / kCols8 * kCols8;
+      double nv = 0.0, nf = 0.0;
+      for (int k = 0; k < vp->ncls; k++) {
+        const double n = (double)vp->members[k].size();
+        if (band.kset >> k & 1) {
+          band.nk += vp->s0[k + 1] - vp->s0[k];
+          nv += n;
+        }
+        for (int q3 = 0; q3 < 3; q3++)
+          if (band.rset[q3] >> k & 1) nf += n;
+      }
+      R.bbytes += b_bytes8(band.ncol, band.nk);
+      R.flops8 += (double)kDigits8 * (kDigits8 + 1) / 2 * 2.0 * nv * nf * (double)band.ncol;
+      for (const Group8& g : R.groups8[q])
+        h_slotcol[R.units[g.unit].sc + g.slot] = (int32_t)(band.col0 + g.col0);
     }
   }
   // final blocks of a round and the H/T column ranges of their units
@@ -611,7 +743,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   std::vector<std::vector<Target>> targets(rounds.size());
   size_t max_y = 1, max_h = 1, max_t = 1;
   for (size_t r = 0; r < rounds.size(); r++) {
-    max_y = std::max(max_y, rounds[r].ncolY * Kp);
+    max_y = std::max(max_y, rounds[r].ncolZ * ldz);
     std::map<BlockPlan*, size_t> idx;
     for (const Unit& u : rounds[r].units)
       for (PairPlan* pp : u.pairs) {
@@ -634,7 +766,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   GI_CUDA(c, c->w_ivec.assign(h_ivec));
   GI_CUDA(c, c->w_EI.assign(h_EI));
   DevArray<double>& d_EI = c->w_EI;
-  GI_CUDA(c, c->w_y.reserve(max_y));
+  if (!s8) GI_CUDA(c, c->w_y.reserve(max_y));  // the default split scheme builds digits directly
   GI_CUDA(c, c->w_z.reserve(3 * max_y));
   c->stats = gi_stats{};
   c->timing = (flags & GI_RUN_PHASE_TIMING) != 0;
@@ -644,10 +776,12 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   const bool use_graph = (flags & GI_RUN_GRAPH) && !c->timing && !c->parent && !c->streamed();
   bool grouped_final = false, fused_y = false;
   if (P.precision == GI_PREC_SPLIT) {
-    gi_status s = split_prepare(c);
-    if (s != GI_OK) return s;
+    if (!s8) {
+      gi_status s = split_prepare(c);
+      if (s != GI_OK) return s;
+    }
     grouped_final = split_grouped_final(c);
-    fused_y = split_fused_y(c);
+    fused_y = s8 || split_fused_y(c);
   }
   // the persistent final GEMM forms the lines itself (no T round trip, no
   // epilogue launches)
@@ -659,9 +793,10 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   // per group.  A group's H and T live side by side in the workspaces.
   std::vector<std::vector<std::pair<size_t, size_t>>> groups(rounds.size());
   size_t max_gh = 1, max_gcols = 1;  // the largest group's H elements and columns
+  size_t max_b8 = 1, max_cols8 = 1;  // default split scheme: B bytes and padded columns
   max_h = max_t = 1;
   for (size_t r = 0; r < rounds.size(); r++) {
-    size_t t0 = 0, items = 0, hs = 0, ts = 0, cols = 0;
+    size_t t0 = 0, items = 0, hs = 0, ts = 0, cols = 0, b8 = 0, cols8 = 0;
     for (size_t t = 0; t < targets[r].size(); t++) {
       Target& T = targets[r][t];
       T.hoff = hs;
@@ -669,18 +804,22 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       hs += T.ncolH * T.F->blk->ld;
       ts += T.ncolH * round_up(T.F->blk->nvec, 2);
       cols += T.ncolH;
-      items += grouped_final ? split_grouped_items(T.F->blk->nvec, (int)T.ncolH) : 0;
+      b8 += b_bytes8(T.ncolH, T.F->blk->ld / 32);
+      cols8 += (T.ncolH + kCols8 - 1) / kCols8 * kCols8;
+      items += grouped_final ? split_grouped_items(c, T.F->blk->nvec, (int)T.ncolH) : 0;
       const bool close = !grouped_final || t + 1 == targets[r].size() ||
                          items >= (size_t)16 * std::max(c->nsm, 1) ||
-                         (int)(t + 1 - t0) == split_grouped_max_jobs();
+                         (int)(t + 1 - t0) == split_grouped_max_jobs(c);
       if (close) {
         groups[r].push_back({t0, t + 1});
         max_h = std::max(max_h, hs);
         max_t = std::max(max_t, ts);
         max_gh = std::max(max_gh, hs);
         max_gcols = std::max(max_gcols, cols);
+        max_b8 = std::max(max_b8, b8);
+        max_cols8 = std::max(max_cols8, cols8);
         t0 = t + 1;
-        items = hs = ts = cols = 0;
+        items = hs = ts = cols = b8 = cols8 = 0;
       }
     }
   }
@@ -698,9 +837,12 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     for (size_t r = 0; r < rounds.size(); r++) {
       max_b = std::max(max_b, rounds[r].ncolY * Kp);
       max_cols = std::max(max_cols, rounds[r].ncolY);
+      max_b8 = std::max(max_b8, rounds[r].bbytes);
+      max_cols8 = std::max(max_cols8, rounds[r].ncolZ);
       for (const Target& T : targets[r]) finals.push_back(T.F->blk);
     }
-    gi_status s = split_reserve(c, max_b, max_cols, finals);
+    gi_status s = s8 ? split8_reserve(c, max_b8, max_cols8, finals)
+                     : split_reserve(c, max_b, max_cols, finals);
     if (s != GI_OK) return s;
   }
 
@@ -784,6 +926,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     mixv(grouped_final);
     mixv(fused_y);
     if (P.precision == GI_PREC_SPLIT) mixv(split_identity(c));
+    if (s8) mixv(vp->uid);
     for (size_t r = 0; r < rounds.size(); r++) {
       mixv(rounds[r].ncolY);
       for (const Unit& u : rounds[r].units) {
@@ -926,11 +1069,11 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       one = rounds[r].units.size() == 1 && (!zblk || zblk == u.I->blk);
       zblk = u.I->blk;
       zoff[r] = ztotal;
-      ztotal += u.ncolY;
+      ztotal += rounds[r].ncolZ;
       ids.insert(ids.end(), h_ivec.begin() + 2 * u.off, h_ivec.begin() + 2 * u.off + u.nI);
     }
     if (one && zblk && ztotal) {
-      gi_status s = zcache_acquire(c, zblk, ids.data(), (int)ids.size(), 3 * ztotal * Kp, &zref);
+      gi_status s = zcache_acquire(c, zblk, ids.data(), (int)ids.size(), 3 * ztotal * ldz, &zref);
       if (s != GI_OK) return s;
     }
   }
@@ -952,13 +1095,105 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   std::vector<std::pair<int, int>> ylists(rounds.size(), {0, 0});  // Y digit items per round
   const char* bs_env = getenv("GI_BATCH_SMALL");
   const bool batch_small = !(bs_env && bs_env[0] == '0');
+  // The default split scheme's tables: slot columns, and per band its K slices,
+  // its row tiles (for every panel of the dipole) and its column groups of Y
+  struct Y8Range {
+    size_t item0 = 0, n = 0, tile0 = 0;
+    long long blocks = 0;
+  };
+  std::vector<Y8Range> y8(rounds.size());
+  std::vector<YItem8> h_y8;
+  if (s8) {
+    std::vector<uint16_t> h_kl;
+    std::vector<int32_t> h_vl, h_ytile;
+    std::vector<ATile> h_at;
+    std::map<uint32_t, std::pair<size_t, size_t>> ksets;  // offsets into h_kl, h_vl
+    const int P8 = dipole_panel_rows(c), step = P8 ? P8 : N;
+    std::vector<std::vector<VibTile>> ptiles;
+    for (int f0 = 0; f0 < N; f0 += step)
+      ptiles.push_back(split8_tiles(*vp, f0, std::min(step, N - f0)));
+    for (Round& R : rounds)
+      for (Band8& band : R.bands) {
+        if (ksets.count(band.kset)) continue;
+        ksets[band.kset] = {h_kl.size(), h_vl.size()};
+        for (int k = 0; k < vp->ncls; k++)
+          if (band.kset >> k & 1)
+            for (int q = vp->s0[k]; q < vp->s0[k + 1]; q++) {
+              h_kl.push_back((uint16_t)q);
+              h_vl.insert(h_vl.end(), vp->vk.begin() + 32 * (size_t)q,
+                          vp->vk.begin() + 32 * (size_t)(q + 1));
+            }
+      }
+    GI_CUDA(c, c->w_kl8.assign(h_kl));
+    GI_CUDA(c, c->w_vl8.assign(h_vl));
+    GI_CUDA(c, c->w_slotcol.assign(h_slotcol));
+    std::vector<std::vector<std::vector<size_t>>> at0(rounds.size());  // [round][band][panel]
+    for (size_t r = 0; r < rounds.size(); r++) {
+      Round& R = rounds[r];
+      const int64_t zc = (int64_t)(zref.z ? ztotal : R.ncolZ) * ldz;
+      at0[r].resize(R.bands.size());
+      for (size_t q = 0; q < R.bands.size(); q++) {
+        Band8& band = R.bands[q];
+        band.kl = c->w_kl8.p + ksets[band.kset].first;
+        for (const auto& tiles : ptiles) {
+          at0[r][q].push_back(h_at.size());
+          int n = 0;
+          for (size_t t = 0; t < tiles.size(); t++) {
+            const VibTile& T = tiles[t];
+            if (!(band.rset[T.comp] >> T.cls & 1)) continue;
+            h_at.push_back(ATile{(int32_t)t, T.rows, T.comp * zc + vp->z0[T.cls] + T.i0});
+            n++;
+          }
+          band.nA.push_back(n);
+        }
+      }
+      y8[r].item0 = h_y8.size();
+      y8[r].tile0 = h_ytile.size();
+      if (zref.hit) continue;
+      for (size_t q = 0; q < R.bands.size(); q++)
+        for (const Group8& g : R.groups8[q]) {
+          const Unit& u = R.units[g.unit];
+          const Block& b = *u.I->blk;
+          const Basis& bI = *c->bases[b.J];
+          YItem8 y{};
+          y.vecs = b.d_vecs.p;
+          y.ivec = c->w_ivec.p + 2 * u.off;
+          y.nent = bI.root_ent[b.gamma] * bI.y_mult;
+          y.nsv = (long long)bI.nslot * N;
+          y.ys = bI.d_ys[b.gamma].p + (size_t)g.slot * N;
+          y.yc = bI.d_yc[b.gamma].p + (size_t)g.slot * N;
+          y.vlist = c->w_vl8.p + ksets[R.bands[q].kset].second;
+          y.out = split8_b(c) + R.bands[q].boff;
+          y.e_out = split8_b_exp(c) + R.bands[q].col0;
+          y.ld = b.ld;
+          y.ndeg = c->degen[b.gamma];
+          y.nk = R.bands[q].nk;
+          y.col0 = (int)g.col0;
+          y.rows = g.rows;
+          y.blk0 = y8[r].blocks;
+          for (; (long long)(h_ytile.size() - y8[r].tile0) * 64 < y.blk0 + y.rows;)
+            h_ytile.push_back((int32_t)(h_y8.size() - y8[r].item0));
+          y8[r].blocks += g.rows;
+          h_y8.push_back(y);
+        }
+      y8[r].n = h_y8.size() - y8[r].item0;
+    }
+    GI_CUDA(c, c->w_at8.assign(h_at));
+    for (size_t r = 0; r < rounds.size(); r++)
+      for (size_t q = 0; q < rounds[r].bands.size(); q++)
+        for (size_t a : at0[r][q]) rounds[r].bands[q].at.push_back(c->w_at8.p + a);
+    GI_CUDA(c, c->w_yitems8.assign(h_y8));
+    GI_CUDA(c, c->w_ytile8.assign(h_ytile));
+    mixv(c->w_kl8.p); mixv(c->w_vl8.p); mixv(c->w_slotcol.p); mixv(c->w_at8.p);
+    mixv(c->w_yitems8.p); mixv(c->w_ytile8.p);
+  }
   if (batch_small) {
     std::vector<HItem> hitems;
     std::vector<NormItem> nitems;
     std::vector<YItem> yitems;
     for (size_t r = 0; r < rounds.size(); r++) {
       const Round& R = rounds[r];
-      if (fused_y && !zref.hit) {  // the round's Y rows, unit by unit
+      if (fused_y && !s8 && !zref.hit) {  // the round's Y rows, unit by unit
         ylists[r].first = (int)yitems.size();
         for (const Unit& u : R.units) {
           const Block& b = *u.I->blk;
@@ -984,8 +1219,8 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
         }
         ylists[r].second = (int)yitems.size() - ylists[r].first;
       }
-      double* zbase = zref.z ? zref.z + zoff[r] * Kp : c->w_z.p;
-      const size_t zc = (zref.z ? ztotal : R.ncolY) * Kp;
+      double* zbase = zref.z ? zref.z + zoff[r] * ldz : c->w_z.p;
+      const size_t zc = (zref.z ? ztotal : R.ncolZ) * ldz;
       for (const auto& grp : groups[r]) {
         GroupLists gl;
         gl.h0 = (int)hitems.size();
@@ -996,11 +1231,15 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
           for (size_t k = 0; k < T.parts.size(); k++) {
             const Unit& u = *T.parts[k].first;
             const PairPlan* pp = T.parts[k].second;
-            const HItem it = make_h_item(
-                zbase + u.ycol * Kp, zc, Kp, c->bases[u.I->blk->J]->nslot,
+            HItem it = make_h_item(
+                zbase + (s8 ? 0 : u.ycol * Kp), zc, ldz, c->bases[u.I->blk->J]->nslot,
                 c->degen[u.I->blk->gamma], u.nI, bF, fb.gamma, c->degen[fb.gamma], fb.nsize,
                 fb.ld, c->w_stencil.p + pp->st_off * 6, c->w_stencil_n.p + pp->st_off, 6,
                 c->w_h.p + T.hoff + T.hcol[k] * fb.ld, gl.hblocks);
+            if (s8) {
+              it.root_v = bF.d_root_z.p;
+              it.slotcol = c->w_slotcol.p + u.sc;
+            }
             if (it.nblk == 0) continue;
             gl.hblocks += it.nblk;
             hitems.push_back(it);
@@ -1045,8 +1284,19 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     const Round& R = rounds[r];
     if (R.units.empty()) continue;
     // Z of this round: the workspace, or its columns of the cache entry
-    double* zbase = zref.z ? zref.z + zoff[r] * Kp : c->w_z.p;
-    const size_t zc = (zref.z ? ztotal : R.ncolY) * Kp;  // stride between dipole components
+    double* zbase = zref.z ? zref.z + zoff[r] * ldz : c->w_z.p;
+    const size_t zc = (zref.z ? ztotal : R.ncolZ) * ldz;  // stride between dipole components
+    if (s8 && !zref.hit) {  // every unit's columns in one launch, or one launch per column group
+      const YItem8* it = c->w_yitems8.p + y8[r].item0;
+      gi_status s = GI_OK;
+      if (batch_small) {
+        s = split8_build_y(c, it, c->w_ytile8.p + y8[r].tile0, (int)y8[r].n, y8[r].blocks);
+      } else {
+        for (size_t k = 0; k < y8[r].n && s == GI_OK; k++)
+          s = split8_build_y(c, it + k, nullptr, 1, h_y8[y8[r].item0 + k].rows);
+      }
+      if (s != GI_OK) return s;
+    }
     if (fused_y && batch_small && ylists[r].second) {  // every unit's Y rows in one launch
       gi_status s = split_build_y_digits_items(c, c->w_yitems.p + ylists[r].first,
                                                ylists[r].second, (long long)R.ncolY, R.ncolY);
@@ -1056,7 +1306,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       if (zref.hit) break;  // Z of this round is in the cache
       const Basis& bI = *c->bases[u.I->blk->J];
       const int ndegI = c->degen[u.I->blk->gamma];
-      if (fused_y && batch_small) {
+      if (s8 || (fused_y && batch_small)) {
         // built above
       } else if (fused_y) {  // straight into the digit planes of the half-ls GEMM's B operand
         gi_status s = split_build_y_digits(c, u.I->blk->d_vecs.p, u.I->blk->ld,
@@ -1075,6 +1325,11 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     }
     if (zref.hit) {
       // computed by an earlier job
+    } else if (s8) {
+      c->stats.flops_tensor += R.flops8;
+      gi_status s = split8_gemm_dipole(c, R.bands, zbase, ldz);
+      if (s != GI_OK) return s;
+      fl_half += 2.0 * 3.0 * N * (double)N * R.ncolY;
     } else if (P.precision == GI_PREC_SPLIT) {
       gi_status s = split_gemm_dipole(c, c->w_y.p, Kp, zbase, Kp, zc, (int)R.ncolY, fused_y);
       if (s != GI_OK) return s;
@@ -1108,11 +1363,13 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
           const int ndegI = c->degen[u.I->blk->gamma];
           const int nslot = c->bases[u.I->blk->J]->nslot;
           GI_CUDA(c, timed(c, GI_PHASE_STENCIL, [&] {
-                    return launch_build_h(zbase + u.ycol * Kp, zc, Kp, nslot, ndegI, u.nI, bF,
-                                          fb.gamma, ndegF, fb.nsize, ldh,
+                    return launch_build_h(zbase + (s8 ? 0 : u.ycol * Kp), zc, ldz, nslot, ndegI,
+                                          u.nI, bF, fb.gamma, ndegF, fb.nsize, ldh,
                                           c->w_stencil.p + pp->st_off * 6,
                                           c->w_stencil_n.p + pp->st_off, 6,
-                                          c->w_h.p + T.hoff + T.hcol[k] * ldh, c->stream);
+                                          c->w_h.p + T.hoff + T.hcol[k] * ldh, c->stream,
+                                          s8 ? bF.d_root_z.p : nullptr,
+                                          s8 ? c->w_slotcol.p + u.sc : nullptr);
                   }));
         }
       }
@@ -1364,6 +1621,153 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
   *nlines_out = c->nlines;
   zrelease.ok = true;  // a Z this run filled is valid for later jobs
+  return GI_OK;
+}
+
+// gi_half_ls in the default split scheme: the slots' Y columns in bands of
+// equal classes, each band's contraction over all rows, K in parts so that
+// every SM has a tile.
+struct HlsPlan8 {
+  uint64_t sig = 0, uid = next_uid();
+  DevArray<YItem8> items;
+  DevArray<int32_t> tile_item, vl, slotcol;
+  DevArray<uint16_t> kl;
+  DevArray<ATile> at;
+  std::vector<Prob8> probs;
+  int nitems = 0, nparts = 1, ldz = 0;
+  long long blocks = 0;
+  size_t pstride = 0;
+  double flops = 0.0;
+};
+
+static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, HlsPlan8** out) {
+  gi_status s;
+  const VibPlan* vp = vib_plan(c, &s);
+  if (!vp) return s;
+  for (Basis* b : {&bI, &bF})
+    if ((s = ensure_root_z(c, *b, *vp)) != GI_OK) return s;
+  if ((s = ensure_y_table(c, bI, gammaI)) != GI_OK) return s;
+  const int ldz = vp->ldz;
+  // bands of slots with the same classes
+  std::map<uint32_t, std::vector<int>> bands;
+  for (int slot = 0; slot < bI.nslot; slot++)
+    bands[std::max(1u, vib_support(*vp, bI, gammaI, slot))].push_back(slot);
+  const auto tiles = split8_tiles(*vp, 0, c->N);
+  size_t cols = 0, bytes = 0;
+  int nk_min = vp->nk;
+  std::vector<int> nks;
+  for (auto& kv : bands) {
+    int nk = 0;
+    for (int k = 0; k < vp->ncls; k++)
+      if (kv.first >> k & 1) nk += vp->s0[k + 1] - vp->s0[k];
+    nks.push_back(nk);
+    nk_min = std::min(nk_min, nk);
+    cols += round_up((int)kv.second.size(), kCols8);
+    bytes += b_bytes8(kv.second.size(), nk);
+  }
+  // two to three waves of tiles; every band has a slice for each part
+  const int want = (int)(5 * std::max(c->nsm, 1) / (2 * std::max<size_t>(1, tiles.size() * bands.size())));
+  const int parts = std::max(1, std::min({want, 8, nk_min}));
+  const size_t pstride = cols * 3 * (size_t)ldz;
+  GI_CUDA(c, c->hls_z.reserve(parts * pstride));
+  if ((s = split8_reserve(c, bytes, cols, {})) != GI_OK) return s;
+  uint64_t sig = vp->uid;
+  for (uint64_t v : {bI.uid, bF.uid, (uint64_t)gammaI, (uint64_t)ideg,
+                     (uint64_t)(uintptr_t)c->hls_z.p, (uint64_t)(uintptr_t)c->hls_v.p,
+                     (uint64_t)(uintptr_t)c->hls_iv.p, split8_identity(c)})
+    sig = (sig ^ v) * 1099511628211ull + (sig >> 29);
+  auto& plans = c->hls_plans8;
+  for (size_t k = 0; k < plans.size(); k++)
+    if (plans[k]->sig == sig) {
+      std::rotate(plans.begin(), plans.begin() + k, plans.begin() + k + 1);
+      *out = plans[0].get();
+      return GI_OK;
+    }
+  auto hp = std::make_shared<HlsPlan8>();
+  hp->sig = sig;
+  hp->ldz = ldz;
+  hp->nparts = parts;
+  hp->pstride = pstride;
+  std::vector<uint16_t> kl;
+  std::vector<int32_t> vl, slotcol(bI.nslot), tile_item;
+  std::vector<ATile> at;
+  std::vector<YItem8> items;
+  for (size_t t = 0; t < tiles.size(); t++)
+    at.push_back(ATile{(int32_t)t, tiles[t].rows,
+                       (int64_t)tiles[t].comp * ldz + vp->z0[tiles[t].cls] + tiles[t].i0});
+  GI_CUDA(c, hp->at.assign(at));
+  size_t col0 = 0, boff = 0, nb = 0;
+  std::vector<size_t> kl0, vl0;
+  for (auto& kv : bands) {
+    kl0.push_back(kl.size());
+    vl0.push_back(vl.size());
+    for (int k = 0; k < vp->ncls; k++)
+      if (kv.first >> k & 1)
+        for (int q = vp->s0[k]; q < vp->s0[k + 1]; q++) {
+          kl.push_back((uint16_t)q);
+          vl.insert(vl.end(), vp->vk.begin() + 32 * (size_t)q, vp->vk.begin() + 32 * (size_t)(q + 1));
+        }
+  }
+  GI_CUDA(c, hp->kl.assign(kl));
+  GI_CUDA(c, hp->vl.assign(vl));
+  for (auto& kv : bands) {
+    const int nk = nks[nb];
+    for (size_t i = 0; i < kv.second.size(); i++) {
+      const int slot = kv.second[i];
+      slotcol[slot] = (int32_t)(col0 + i);
+      YItem8 y{};
+      y.vecs = c->hls_v.p;
+      y.ivec = c->hls_iv.p;
+      y.nent = bI.root_ent[gammaI] * bI.y_mult;
+      y.nsv = (long long)bI.nslot * c->N;
+      y.ys = bI.d_ys[gammaI].p + (size_t)slot * c->N;
+      y.yc = bI.d_yc[gammaI].p + (size_t)ideg * y.nent * y.nsv + (size_t)slot * c->N;
+      y.vlist = hp->vl.p + vl0[nb];
+      y.out = split8_b(c) + boff;
+      y.e_out = split8_b_exp(c) + col0;
+      y.ld = round_up(bI.Ntotal[gammaI], 64);
+      y.ndeg = 1;
+      y.nk = nk;
+      y.col0 = (int)i;
+      y.rows = 1;
+      y.blk0 = (long long)items.size();
+      if ((items.size() & 63) == 0) tile_item.push_back((int32_t)items.size());
+      items.push_back(y);
+    }
+    for (int q = 0; q < parts; q++) {
+      // every part has a slice, so that each partial product is written
+      const int k0 = (int)((long long)nk * q / parts), k1 = (int)((long long)nk * (q + 1) / parts);
+      Prob8 p{};
+      split8_dipole_operand(c, &p);
+      p.B = split8_b(c) + boff + (size_t)k0 * kBTileSlice8;
+      p.eb = split8_b_exp(c) + col0;
+      p.C = c->hls_z.p + q * pstride + col0 * 3 * (size_t)ldz;
+      p.ldc = 3 * (long long)ldz;
+      p.at = hp->at.p;
+      p.nA = (int)at.size();
+      p.kl = hp->kl.p + kl0[nb] + k0;
+      p.nkB = nk;
+      p.nk = k1 - k0;
+      p.Nc = (int)kv.second.size();
+      hp->probs.push_back(p);
+    }
+    double nv = 0.0;
+    for (int k = 0; k < vp->ncls; k++)
+      if (kv.first >> k & 1) nv += (double)vp->members[k].size();
+    hp->flops += (double)kDigits8 * (kDigits8 + 1) / 2 * 2.0 * nv * 3.0 * c->N *
+                 (double)kv.second.size();
+    col0 += round_up((int)kv.second.size(), kCols8);
+    boff += b_bytes8(kv.second.size(), nk);
+    nb++;
+  }
+  GI_CUDA(c, hp->slotcol.assign(slotcol));
+  GI_CUDA(c, hp->tile_item.assign(tile_item));
+  GI_CUDA(c, hp->items.assign(items));
+  hp->nitems = (int)items.size();
+  hp->blocks = (long long)items.size();
+  if (plans.size() >= 8) plans.pop_back();
+  plans.insert(plans.begin(), hp);
+  *out = hp.get();
   return GI_OK;
 }
 
@@ -1821,7 +2225,7 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   const int ncol = bI.nslot;
   // grow-only workspaces of the context: repeated calls allocate nothing
   GI_CUDA(c, c->hls_v.reserve(ld));
-  GI_CUDA(c, c->hls_iv.reserve(1));
+  if (!c->hls_iv.p) GI_CUDA(c, c->hls_iv.assign(std::vector<int32_t>{0}));  // the one vector's index
   GI_CUDA(c, c->hls_y.reserve((size_t)ncol * c->Kp));
   GI_CUDA(c, c->hls_h.reserve(bF.D));
   // the vector and the result pass through pinned staging of the context;
@@ -1843,17 +2247,30 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   }
   const int max_parts = 8;
   const size_t ldz_max = (size_t)3 * round_up(c->N, 128);
-  if (split_path) GI_CUDA(c, c->hls_z.reserve((size_t)max_parts * ncol * ldz_max));
+  HlsPlan8* h8 = nullptr;
+  if (split_path && split8_active(c)) {
+    s = hls_plan8(c, bI, bF, gammaI, ideg, &h8);
+    if (s != GI_OK) return s;
+  } else if (split_path) GI_CUDA(c, c->hls_z.reserve((size_t)max_parts * ncol * ldz_max));
   else GI_CUDA(c, c->hls_z.reserve((size_t)3 * ncol * c->Kp));
   // the call's device work: the vector in, Y, the dipole GEMM, the stencil,
   // the result out (all on c->stream; capturable)
   auto issue = [&]() -> gi_status {
-    GI_CUDA(c, cudaMemsetAsync(c->hls_v.p, 0, sizeof(double) * ld, c->stream));
-    GI_CUDA(c, cudaMemsetAsync(c->hls_iv.p, 0, sizeof(int32_t), c->stream));
     GI_CUDA(c, cudaMemcpyAsync(c->hls_v.p, c->hls_pin, sizeof(double) * nsize,
                                cudaMemcpyHostToDevice, c->stream));
     double* y = c->hls_y.p;
     double* hh = c->hls_h.p;
+    if (h8) {
+      gi_status q = split8_build_y(c, h8->items.p, h8->tile_item.p, h8->nitems, h8->blocks);
+      if (q != GI_OK) return q;
+      std::vector<Prob8> probs = h8->probs;
+      c->stats.flops_tensor += h8->flops;
+      q = split8_launch(c, GI_PHASE_HALFLS_GEMM, probs, nullptr, false);
+      if (q != GI_OK) return q;
+      GI_CUDA(c, launch_half_ls_prim_parts(c->hls_z.p, h8->nparts, h8->pstride, 3 * h8->ldz,
+                                           h8->ldz, bF, dst, dstn, 6, hh, c->stream,
+                                           bF.d_root_z.p, h8->slotcol.p));
+    } else {
     GI_CUDA(c, launch_build_y(c->hls_v.p, ld, c->hls_iv.p, 1, 1, bI, gammaI, ndeg, c->N, c->Kp,
                               y, c->stream, ideg));
     if (split_path) {
@@ -1870,6 +2287,7 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
       gi_status q = dipole_gemm_fp64(c, y, c->Kp, c->hls_z.p, c->Kp, zc, ncol, c->stream);
       if (q != GI_OK) return q;
       GI_CUDA(c, launch_half_ls_prim(c->hls_z.p, zc, c->Kp, bF, dst, dstn, 6, hh, c->stream));
+    }
     }
     GI_CUDA(c, cudaMemcpyAsync(c->hls_pin, hh, sizeof(double) * bF.D, cudaMemcpyDeviceToHost,
                                c->stream));
@@ -1890,6 +2308,7 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   mixv(c->hls_v.p); mixv(c->hls_iv.p); mixv(c->hls_y.p); mixv(c->hls_z.p); mixv(c->hls_h.p);
   mixv(c->hls_pin); mixv(c->hls_pin_cap);
   if (split_path) mixv(split_identity(c));
+  if (h8) mixv(h8->uid);
   std::memcpy(c->hls_pin, vsym, sizeof(double) * nsize);
   *err_word = 0;
   // graphs need a capturable stream (not the legacy or per-thread default
@@ -1938,6 +2357,7 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   GI_CUDA(c, cudaStreamSynchronize(c->stream));
   std::memcpy(half_ls, c->hls_pin, sizeof(double) * bF.D);
   if (*err_word) {
+    split8_error_seen(c);
     c->err = "split GEMM: a pipeline wait timed out (code " + std::to_string(*err_word) + ")";
     return GI_ERR_DEVICE;
   }

@@ -67,6 +67,60 @@ cudaError_t launch_build_y(const double* vecs, int ld, const int32_t* ivec, int 
   return cudaGetLastError();
 }
 
+// The CSR of k_build_y flattened: one thread per (slot, v), its (symmetrised
+// function, coefficients) entries in the same order, zero coefficients left out.
+__global__ void k_y_table(const int32_t* __restrict__ yptr, const int32_t* __restrict__ yroot,
+                          const int32_t* __restrict__ root_case,
+                          const int32_t* __restrict__ root_lam,
+                          const int32_t* __restrict__ case_iterm,
+                          const int32_t* __restrict__ case_nelem, const double* __restrict__ rep,
+                          int Ntot, int degen, long long nsv, int E, int32_t* __restrict__ ys,
+                          double* __restrict__ yc) {
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (q >= nsv) return;
+  int n = 0;
+  for (int p = yptr[q]; p < yptr[q + 1]; ++p) {
+    const int r = yroot[p];
+    const int c = root_case[r], lam = root_lam[r];
+    for (int j = 0; j < case_nelem[c]; ++j) {
+      const int s = case_iterm[c] + j;
+      bool any = false;
+      for (int d = 0; d < degen; ++d)
+        any = any || rep[s + (size_t)d * Ntot + (size_t)lam * degen * Ntot] != 0.0;
+      if (!any || n == E) continue;
+      ys[n * nsv + q] = s;
+      for (int d = 0; d < degen; ++d)
+        yc[((long long)d * E + n) * nsv + q] =
+            rep[s + (size_t)d * Ntot + (size_t)lam * degen * Ntot];
+      ++n;
+    }
+  }
+  for (; n < E; ++n) {
+    ys[n * nsv + q] = 0;
+    for (int d = 0; d < degen; ++d) yc[((long long)d * E + n) * nsv + q] = 0.0;
+  }
+}
+
+__global__ void k_root_z(const int32_t* __restrict__ root_v, const int32_t* __restrict__ zpos, int D,
+                         int32_t* __restrict__ out) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < D) out[r] = zpos[root_v[r]];
+}
+cudaError_t launch_root_z(const Basis& b, const int32_t* zpos, int32_t* out, cudaStream_t s) {
+  k_root_z<<<(b.D + 255) / 256, 256, 0, s>>>(b.d_root_v.p, zpos, b.D, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_y_table(const Basis& b, int gamma, int degen, int N, int E, int32_t* ys,
+                           double* yc, cudaStream_t s) {
+  const long long nsv = (long long)b.nslot * N;
+  if (nsv == 0 || E == 0) return cudaSuccess;
+  k_y_table<<<(unsigned)((nsv + 255) / 256), 256, 0, s>>>(
+      b.d_yptr.p, b.d_yroot.p, b.d_root_case.p, b.d_root_lam.p, b.d_case_iterm[gamma].p,
+      b.d_case_nelem[gamma].p, b.d_rep[gamma].p, b.Ntotal[gamma], degen, nsv, E, ys, yc);
+  return cudaGetLastError();
+}
+
 // ------------------------------------------------------------------ H build
 // One thread per symmetrised final function s of one initial column (i, dI);
 // writes H for every final degenerate component dF.
@@ -78,25 +132,35 @@ __device__ __forceinline__ void build_h_col(
     const int32_t* __restrict__ root_key, const int32_t* __restrict__ root_lam,
     const double* __restrict__ rep, int Ntot, const StencilTerm* __restrict__ st,
     const int32_t* __restrict__ st_n, int st_max, int nsizeF, int ldh, int s,
-    double* __restrict__ H) {
+    double* __restrict__ H, const int32_t* __restrict__ slotcol) {
   double acc[NDEGF];
 #pragma unroll
   for (int d = 0; d < NDEGF; ++d) acc[d] = 0.0;
   if (s < nsizeF) {
-    const double* zcol = Z + (size_t)colI * nslotI * ldz;
+    const double* zcol = Z + (size_t)colI * (slotcol ? 1 : nslotI) * ldz;
     const int cs = s_case[s];
     for (int p = case_ptr[cs]; p < case_ptr[cs + 1]; ++p) {
       const int r = case_roots[p];
       const int v = root_v[r], key = root_key[r], lam = root_lam[r];
+      // a root the symmetrised function has no part in is passed over: its
+      // rows of Z may not have been computed
+      double w[NDEGF];
+      bool any = false;
+#pragma unroll
+      for (int d = 0; d < NDEGF; ++d) {
+        w[d] = rep[s + (size_t)d * Ntot + (size_t)lam * NDEGF * Ntot];
+        any = any || w[d] != 0.0;
+      }
+      if (!any) continue;
       double h = 0.0;
       const int nt = st_n[key];
       for (int t = 0; t < nt; ++t) {
         const StencilTerm term = st[key * st_max + t];
-        h = fma(term.coef, zcol[(size_t)term.c * zc + (size_t)term.slotI * ldz + v], h);
+        const size_t col = slotcol ? slotcol[term.slotI] : term.slotI;
+        h = fma(term.coef, zcol[(size_t)term.c * zc + col * ldz + v], h);
       }
 #pragma unroll
-      for (int d = 0; d < NDEGF; ++d)
-        acc[d] = fma(rep[s + (size_t)d * Ntot + (size_t)lam * NDEGF * Ntot], h, acc[d]);
+      for (int d = 0; d < NDEGF; ++d) acc[d] = fma(w[d], h, acc[d]);
     }
   }
 #pragma unroll
@@ -111,12 +175,12 @@ __global__ void k_build_h(const double* __restrict__ Z, size_t zc, int ldz, int 
                           const int32_t* __restrict__ root_lam, const double* __restrict__ rep,
                           int Ntot, const StencilTerm* __restrict__ st,
                           const int32_t* __restrict__ st_n, int st_max, int nsizeF, int ldh,
-                          double* __restrict__ H) {
+                          double* __restrict__ H, const int32_t* __restrict__ slotcol) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const int colI = blockIdx.y;  // i * ndegI + dI
   if (s >= ldh) return;
   build_h_col<NDEGF>(Z, zc, ldz, nslotI, colI, s_case, case_ptr, case_roots, root_v, root_key,
-                     root_lam, rep, Ntot, st, st_n, st_max, nsizeF, ldh, s, H);
+                     root_lam, rep, Ntot, st, st_n, st_max, nsizeF, ldh, s, H, slotcol);
 }
 
 // Every H build of a group of final blocks in one launch: item k covers
@@ -139,11 +203,11 @@ __global__ void __launch_bounds__(256) k_build_h_items(const HItem* __restrict__
     if (it.ndegF == 2)
       build_h_col<2>(it.Z, it.zc, it.ldz, it.nslotI, colI, it.s_case, it.case_ptr, it.case_roots,
                      it.root_v, it.root_key, it.root_lam, it.rep, it.Ntot, it.st, it.st_n,
-                     it.st_max, it.nsizeF, it.ldh, s, it.H);
+                     it.st_max, it.nsizeF, it.ldh, s, it.H, it.slotcol);
     else
       build_h_col<1>(it.Z, it.zc, it.ldz, it.nslotI, colI, it.s_case, it.case_ptr, it.case_roots,
                      it.root_v, it.root_key, it.root_lam, it.rep, it.Ntot, it.st, it.st_n,
-                     it.st_max, it.nsizeF, it.ldh, s, it.H);
+                     it.st_max, it.nsizeF, it.ldh, s, it.H, it.slotcol);
   }
 }
 
@@ -189,19 +253,22 @@ HItem make_h_item(const double* Z, size_t zstride_c, int ldz, int nslotI, int nd
 cudaError_t launch_build_h(const double* Z, size_t zstride_c, int ldz, int nslotI, int ndegI,
                            int nI, const Basis& bF, int gammaF, int degF, int nsizeF, int ldh,
                            const StencilTerm* st, const int32_t* st_n, int st_max, double* H,
-                           cudaStream_t s) {
+                           cudaStream_t s, const int32_t* root_z, const int32_t* slotcol) {
   if (nI == 0) return cudaSuccess;
+  const int32_t* root_v = root_z ? root_z : bF.d_root_v.p;
   dim3 grid((ldh + 255) / 256, nI * ndegI);
   if (degF == 1)
     k_build_h<1><<<grid, 256, 0, s>>>(Z, zstride_c, ldz, nslotI, ndegI, bF.d_s_case[gammaF].p,
-                                      bF.d_case_ptr.p, bF.d_case_roots.p, bF.d_root_v.p,
+                                      bF.d_case_ptr.p, bF.d_case_roots.p, root_v,
                                       bF.d_root_key.p, bF.d_root_lam.p, bF.d_rep[gammaF].p,
-                                      bF.Ntotal[gammaF], st, st_n, st_max, nsizeF, ldh, H);
+                                      bF.Ntotal[gammaF], st, st_n, st_max, nsizeF, ldh, H,
+                                      slotcol);
   else if (degF == 2)
     k_build_h<2><<<grid, 256, 0, s>>>(Z, zstride_c, ldz, nslotI, ndegI, bF.d_s_case[gammaF].p,
-                                      bF.d_case_ptr.p, bF.d_case_roots.p, bF.d_root_v.p,
+                                      bF.d_case_ptr.p, bF.d_case_roots.p, root_v,
                                       bF.d_root_key.p, bF.d_root_lam.p, bF.d_rep[gammaF].p,
-                                      bF.Ntotal[gammaF], st, st_n, st_max, nsizeF, ldh, H);
+                                      bF.Ntotal[gammaF], st, st_n, st_max, nsizeF, ldh, H,
+                                      slotcol);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();
@@ -240,14 +307,16 @@ __global__ void k_half_ls_prim_parts(const double* __restrict__ Zp, int nparts, 
                                      const int32_t* __restrict__ root_key,
                                      const StencilTerm* __restrict__ st,
                                      const int32_t* __restrict__ st_n, int st_max, int D,
-                                     double* __restrict__ h) {
+                                     double* __restrict__ h,
+                                     const int32_t* __restrict__ slotcol) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= D) return;
   const int v = root_v[r], key = root_key[r];
   double acc = 0.0;
   for (int t = 0; t < st_n[key]; ++t) {
     const StencilTerm term = st[key * st_max + t];
-    const double* z = Zp + (size_t)term.slotI * ldz + (size_t)term.c * cstride + v;
+    const int col = slotcol ? slotcol[term.slotI] : term.slotI;
+    const double* z = Zp + (size_t)col * ldz + (size_t)term.c * cstride + v;
     double zs = z[0];
     for (int p = 1; p < nparts; ++p) zs += z[(size_t)p * pstride];
     acc = fma(term.coef, zs, acc);
@@ -258,10 +327,11 @@ __global__ void k_half_ls_prim_parts(const double* __restrict__ Zp, int nparts, 
 cudaError_t launch_half_ls_prim_parts(const double* Zp, int nparts, size_t pstride, int ldz,
                                       int cstride, const Basis& bF, const StencilTerm* st,
                                       const int32_t* st_n, int st_max, double* h,
-                                      cudaStream_t s) {
-  k_half_ls_prim_parts<<<(bF.D + 255) / 256, 256, 0, s>>>(Zp, nparts, pstride, ldz, cstride,
-                                                          bF.d_root_v.p, bF.d_root_key.p, st,
-                                                          st_n, st_max, bF.D, h);
+                                      cudaStream_t s, const int32_t* root_z,
+                                      const int32_t* slotcol) {
+  k_half_ls_prim_parts<<<(bF.D + 255) / 256, 256, 0, s>>>(
+      Zp, nparts, pstride, ldz, cstride, root_z ? root_z : bF.d_root_v.p, bF.d_root_key.p, st, st_n,
+      st_max, bF.D, h, slotcol);
   return cudaGetLastError();
 }
 

@@ -143,9 +143,8 @@ static size_t need_bytes(const Server* s, const Block& b, bool final_block) {
   size_t n = 0;
   if (!b.resident) n += (size_t)std::max(b.nvec, 1) * b.ld * sizeof(double);
   if (final_block && s->precision == GI_PREC_SPLIT && (!b.resident || b.digits_s == 0)) {
-    const int s_digits = split_digits(s->owner);
     const size_t vpad = (size_t)round_up(std::max(b.nvec, 1), 128);
-    n += (size_t)s_digits * vpad * b.ld * sizeof(uint16_t) + vpad * sizeof(int32_t);
+    n += split_digit_bytes(s->owner) * vpad * b.ld + vpad * sizeof(int32_t);
   }
   return n;
 }

@@ -45,9 +45,10 @@
 #include <string>
 #include <tuple>
 
-#include "split.h"
+#include "split8.h"
 #include "epilogue.cuh"
 #include "items.cuh"
+#include "tc.cuh"
 #include "../../include/gi_probe.h"
 
 namespace gi {
@@ -75,63 +76,6 @@ size_t smem_bytes(int s, int bn) {
 }
 
 // ------------------------------------------------------------------ PTX
-__device__ __forceinline__ uint32_t sptr(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* b, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(sptr(b)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(sptr(b)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ uint32_t mbar_try(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(sptr(b)), "r"(parity)
-      : "memory");
-  return ok;
-}
-__device__ __forceinline__ uint64_t gtimer() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-  return t;
-}
-// Bounded wait on an mbarrier phase.  Returns false when the CTA is aborting
-// (another warp timed out) or this wait exceeded its time limit (then it
-// raises the abort itself and records the error).
-// `sleep_ns` backs the poll off so that a waiting warp leaves the issue slots of
-// its SM sub-partition to the MMA-issuing warp.
-// CL: cluster-scope acquire (barriers that the peer CTA of a pair completes).
-__device__ __forceinline__ uint32_t mbar_try_cl(uint64_t* b, uint32_t parity);
-template <bool CL = false>
-__device__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag, int* err,
-                          int code, unsigned sleep_ns = 0) {
-  uint64_t t0 = 0;
-  for (uint32_t it = 1;; ++it) {
-    if (CL ? mbar_try_cl(b, parity) : mbar_try(b, parity)) return true;
-    if (sleep_ns) __nanosleep(sleep_ns);
-    if ((it & 63) == 0) {
-      if (*abort_flag) return false;
-      if (*reinterpret_cast<volatile int*>(err)) {  // another CTA timed out: stop waiting
-        *abort_flag = 1;
-        return false;
-      }
-      const uint64_t t = gtimer();
-      if (t0 == 0) {
-        t0 = t;
-      } else if (t - t0 > 4000000000ull) {  // 4 s: far beyond any tile's work
-        *abort_flag = 1;
-        atomicExch(err, code);
-        return false;
-      }
-    }
-  }
-}
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar,
                                             int c0, int c1, int c2) {
   asm volatile(
@@ -149,47 +93,6 @@ __device__ __forceinline__ double ld_acc(const double* p) {
   return v;
 }
 
-// v * 2^E for an integer |v| < 2^53 (so the double is exact), built from the
-// bits with integer instructions: FP64 throughput is low on this GPU and the
-// epilogues convert every output element.  Results outside the normal range
-// take ldexp.
-__device__ __forceinline__ double scaled_int_body(long long v, int E) {
-  if (v == 0) return 0.0;
-  const unsigned long long sgn = v < 0 ? (1ull << 63) : 0ull;
-  const unsigned long long a = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
-  const int msb = 63 - __clzll((long long)a);
-  const int ex = 1023 + msb + E;
-  if (msb > 52 || ex <= 0 || ex >= 2047) return ldexp((double)v, E);
-  const unsigned long long mant = (a << (52 - msb)) & ((1ull << 52) - 1);
-  return __longlong_as_double((long long)(sgn | ((unsigned long long)ex << 52) | mant));
-}
-// The epilogues call these instead of inlining the conversion: inlined into
-// the unrolled column chunks, it made the pass-1 epilogue of the half-ls GEMM
-// a long stretch of straight-line code that ran out of the instruction cache
-// once per tile (39 us of a 265 us tile, against 21 us called, measured with
-// per-tile clock stamps).
-__device__ __noinline__ double scaled_int(long long v, int E) { return scaled_int_body(v, E); }
-// a0 * 2^ea0 + b0 * 2^eb0 and the same for a second element, in one call (the
-// two parts of a two-pass tile's exact sums, added in FP64; the conversions of
-// the two elements interleave)
-__device__ __noinline__ double2 scaled_pair2(long long a0, int ea0, long long b0, int eb0,
-                                             long long a1, int ea1, long long b1, int eb1) {
-  double2 r;
-  r.x = scaled_int_body(a0, ea0) + scaled_int_body(b0, eb0);
-  r.y = scaled_int_body(a1, ea1) + scaled_int_body(b1, eb1);
-  return r;
-}
-// Shared-memory matrix descriptor of a K-major bf16 tile whose rows are 32
-// bytes (16 elements) with the 32-byte swizzle: 8-row groups 256 bytes apart.
-__device__ __forceinline__ uint64_t sdesc_sw32(uint32_t addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFF);          // start address
-  d |= (uint64_t)1 << 16;                          // leading byte offset (unused here)
-  d |= (uint64_t)((256 >> 4) & 0x3FFF) << 32;      // stride byte offset: 8 rows x 32 B
-  d |= (uint64_t)1 << 46;                          // descriptor version (tcgen05)
-  d |= (uint64_t)6 << 61;                          // SWIZZLE_32B
-  return d;
-}
 // The same for 128-byte rows with the 128-byte swizzle (8-row groups 1024
 // bytes apart).  In the grouped digit layout one such row holds the 16-element
 // K slice of four digit planes; the descriptor of plane p of a group starts
@@ -218,12 +121,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
       "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-          sptr(bar))
-      : "memory");
-}
 // ---- the 2-SM pair (cta_group::2): a cluster of two CTAs on one TPC, the
 // MMA issued by rank 0 over both CTAs' shared memory (rows 0-127 of A and the
 // first half of B's rows from rank 0, the rest from rank 1, at the same
@@ -242,18 +139,6 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::
                    : "memory");
-}
-// Try-wait with cluster-scope acquire: phases completed by the peer CTA's
-// arrivals or TMA bytes.
-__device__ __forceinline__ uint32_t mbar_try_cl(uint64_t* b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(sptr(b)), "r"(parity)
-      : "memory");
-  return ok;
 }
 __device__ __forceinline__ void mbar_arrive_cl(uint32_t bar_cluster) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar_cluster)
@@ -666,10 +551,6 @@ __device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t* r) {
         "=r"(r[7])
       : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-}
-
 // ACC: add to C (the later launches of a K-segmented GEMM); a template
 // argument, so the first launch's code carries no trace of it.
 // PAIR: the tile is 256 x BN, computed by a cluster of two CTAs with
@@ -1403,29 +1284,6 @@ __global__ void __launch_bounds__(kThreadsG, 1)
 // digits: a_p in [-2^(w-1), 2^(w-1)) for p >= 1 and the remaining top digit
 // |a_0| <= 2^(w-1), so X = sum_p a_p 2^(w(s-1-p)) exactly.
 
-// Row exponent from the largest magnitude's bit pattern: 2^(e-1) <= max < 2^e.
-__device__ __forceinline__ int row_exponent(unsigned long long maxbits) {
-  if (maxbits == 0) return 0;
-  const int eb = (int)(maxbits >> 52);
-  return eb ? eb - 1022 : -1021 - (__clzll((long long)maxbits) - 12);
-}
-
-__device__ __forceinline__ long long fixed_point(double x, int e, int ws) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int eb = (int)((b >> 52) & 0x7FF);
-  const long long mant = (long long)(b & 0xFFFFFFFFFFFFFull) | (eb ? (1ll << 52) : 0ll);
-  const int sh = (eb ? eb : 1) - 1075 - e + ws;  // x 2^(ws-e) = mant 2^sh
-  long long X;
-  if (sh >= 0) {
-    X = mant << sh;
-  } else if (sh > -54) {
-    X = (mant + (1ll << (-sh - 1))) >> (-sh);  // round half up
-  } else {
-    X = 0;
-  }
-  return (b >> 63) ? -X : X;
-}
-
 __device__ __forceinline__ uint16_t bf16_of_int(int a) {
   const __nv_bfloat16 h = __float2bfloat16_rn((float)a);  // |a| <= 256: exact
   return *reinterpret_cast<const uint16_t*>(&h);
@@ -1755,19 +1613,6 @@ bool make_map_groups(CUtensorMap* map, const void* base, int K, int rows, int nq
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// One launch configuration of the split GEMM: the kernel (one pass with all
-// diagonals in tensor memory, or two passes with wider tiles) and the L2
-// raster group (row tiles whose digit planes share about ga_mb MB of L2).
-struct GemmConfig {
-  int kind = 1;  // 0: k_split_gemm (one pass); 1, 2: k_split_gemm2 (two passes,
-                 // diagonals split at s/2 or s - s/2); these read the plain
-                 // layout.  6, 7, 8: k_split_gemm_g on the grouped layout (two
-                 // passes split at s/2 or s - s/2, or one pass); 9: its 2-SM
-                 // pair form (256-row tiles, two passes split at s/2, s = 9).
-                 // 3-5 are unused.
-  int ga_mb = 64;
-};
-
 // Two-pass geometry: diagonals [0, S/2) then [S/2, S), each pass's accumulators
 // within the 512 tensor-memory columns, at most 128 wide.
 __host__ __device__ constexpr int d1_of(int s) { return s / 2; }
@@ -2037,6 +1882,8 @@ static gi_status check(Ctx* c, cudaError_t e, const char* what) {
 }
 
 gi_status split_prepare(Ctx* c) {
+  if (split8_selected(c)) return split8_prepare(c);
+  if (c->split8) split8_deactivate(c);
   SplitState* S = state(c);
   const SplitShape sh = shape_of(c);
   if (!encode_fn()) {
@@ -2158,6 +2005,58 @@ static int col_bucket(int n) {
   return b;
 }
 
+// Runs a GEMM with its class's configuration: the table's, or (tuning on,
+// not inside a capture) the fastest of the valid candidates, timed here; else
+// the default.
+static gi_status tuned(Ctx* c, const TuneKey& key, GemmConfig cfg,
+                       const std::function<bool(const GemmConfig&)>& valid,
+                       const std::function<cudaError_t(const GemmConfig&)>& run) {
+  bool known = false;
+  Tuner& t = tuner();
+  {
+    std::lock_guard<std::mutex> lk(t.mu);
+    if (!c->tune_path.empty() && t.loaded != c->tune_path) tune_load(t, c->tune_path);
+    auto it = t.table.find(key);
+    if (it != t.table.end()) {
+      cfg = it->second.cfg;
+      known = true;
+    }
+  }
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (!known && c->tune_mode > 0 && cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess &&
+      cs == cudaStreamCaptureStatusNone) {
+    cudaEvent_t a = nullptr, b = nullptr;
+    gi_status g = check(c, cudaEventCreate(&a), "tuning event");
+    if (g == GI_OK) g = check(c, cudaEventCreate(&b), "tuning event");
+    if (g == GI_OK) g = check(c, run(cfg), "tuning warm-up");  // the first launch of a shape
+    float best = 1e30f;
+    GemmConfig best_cfg = cfg;
+    for (const GemmConfig& cand : kCandidates) {
+      if (g != GI_OK) break;
+      if (!valid(cand)) continue;
+      g = check(c, cudaEventRecord(a, c->stream), "tuning event");
+      if (g == GI_OK) g = check(c, run(cand), "tuning launch");
+      if (g == GI_OK) g = check(c, cudaEventRecord(b, c->stream), "tuning event");
+      if (g == GI_OK) g = check(c, cudaEventSynchronize(b), "tuning sync");
+      float ms = 0.f;
+      if (g == GI_OK) g = check(c, cudaEventElapsedTime(&ms, a, b), "tuning time");
+      if (g == GI_OK && ms < best) {
+        best = ms;
+        best_cfg = cand;
+      }
+    }
+    if (a) cudaEventDestroy(a);
+    if (b) cudaEventDestroy(b);
+    if (g != GI_OK) return g;
+    std::lock_guard<std::mutex> lk(t.mu);
+    t.table[key] = TuneEntry{best_cfg, best};
+    t.version++;
+    if (!c->tune_path.empty()) tune_save(t, c->tune_path);
+    cfg = best_cfg;
+  }
+  return check(c, run(cfg), "split GEMM launch");
+}
+
 static gi_status gemm(Ctx* c, const uint16_t* Aslices, int Arows_total, const int32_t* ea,
                       int Mpad, const uint16_t* Bslices, int Brows, const int32_t* eb,
                       double* C, int ldc, size_t strideC, int M, int Nc, int K, int batch) {
@@ -2204,8 +2103,7 @@ static gi_status gemm(Ctx* c, const uint16_t* Aslices, int Arows_total, const in
     return cudaSuccess;
   };
   const TuneKey key{S->s, ((M + kBM - 1) / kBM) * batch, col_bucket(Nc), K, (int)grouped};
-  GemmConfig cfg = default_config(S->s, grouped);
-  bool known = false;
+  const GemmConfig cfg = default_config(S->s, grouped);
   // GI_SPLIT_FORCE="kind:ga_mb" pins one configuration (parity tests of every kernel)
   if (const char* f = getenv("GI_SPLIT_FORCE")) {
     GemmConfig g;
@@ -2213,50 +2111,16 @@ static gi_status gemm(Ctx* c, const uint16_t* Aslices, int Arows_total, const in
         g.ga_mb > 0)
       return check(c, run(g), "split GEMM launch");
   }
-  Tuner& t = tuner();
-  {
-    std::lock_guard<std::mutex> lk(t.mu);
-    if (!c->tune_path.empty() && t.loaded != c->tune_path) tune_load(t, c->tune_path);
-    auto it = t.table.find(key);
-    if (it != t.table.end()) {
-      cfg = it->second.cfg;
-      known = true;
-    }
-  }
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (!known && c->tune_mode > 0 && cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess &&
-      cs == cudaStreamCaptureStatusNone) {
-    cudaEvent_t a = nullptr, b = nullptr;
-    gi_status g = check(c, cudaEventCreate(&a), "tuning event");
-    if (g == GI_OK) g = check(c, cudaEventCreate(&b), "tuning event");
-    if (g == GI_OK) g = check(c, run(cfg), "tuning warm-up");  // the first launch of a shape
-    float best = 1e30f;
-    GemmConfig best_cfg = cfg;
-    for (const GemmConfig& cand : kCandidates) {
-      if (g != GI_OK) break;
-      if (!kind_valid(S->s, cand.kind, grouped)) continue;
-      g = check(c, cudaEventRecord(a, c->stream), "tuning event");
-      if (g == GI_OK) g = check(c, run(cand), "tuning launch");
-      if (g == GI_OK) g = check(c, cudaEventRecord(b, c->stream), "tuning event");
-      if (g == GI_OK) g = check(c, cudaEventSynchronize(b), "tuning sync");
-      float ms = 0.f;
-      if (g == GI_OK) g = check(c, cudaEventElapsedTime(&ms, a, b), "tuning time");
-      if (g == GI_OK && ms < best) {
-        best = ms;
-        best_cfg = cand;
-      }
-    }
-    if (a) cudaEventDestroy(a);
-    if (b) cudaEventDestroy(b);
-    if (g != GI_OK) return g;
-    std::lock_guard<std::mutex> lk(t.mu);
-    t.table[key] = TuneEntry{best_cfg, best};
-    t.version++;
-    if (!c->tune_path.empty()) tune_save(t, c->tune_path);
-    cfg = best_cfg;
-  }
-  return check(c, run(cfg), "split GEMM launch");
+  return tuned(c, key, cfg, [&](const GemmConfig& g) { return kind_valid(S->s, g.kind, grouped); },
+               run);
 }
+
+gi_status split_tuned(Ctx* c, int s, int nA, int ncols, int K, int layout,
+                      const std::function<cudaError_t(const GemmConfig&)>& run) {
+  return tuned(c, TuneKey{s, nA, col_bucket(ncols), K, layout}, GemmConfig{6, 64},
+               [](const GemmConfig& g) { return g.kind == 6; }, run);
+}
+uint64_t split_tuner_version() { return tuner().version; }
 
 gi_status split_gemm_dipole(Ctx* c, const double* Y, int ldy, double* Z, int ldz, size_t zstride,
                             int ncol, bool y_digits_ready) {
@@ -2369,6 +2233,7 @@ gi_status split_reserve(Ctx* c, size_t max_elems, size_t max_cols,
 
 gi_status split_gemm_final(Ctx* c, Block& fb, const double* H, int ldh, int ncol, double* T,
                            int ldt) {
+  if (split8_active(c)) return split8_gemm_final(c, {FinalJob{&fb, H, ldh, ncol, T, ldt}}, nullptr);
   SplitState* S = state(c);
   const int K = ldh;
   const int nvec = fb.nvec;
@@ -2401,13 +2266,15 @@ gi_status split_gemm_final(Ctx* c, Block& fb, const double* H, int ldh, int ncol
 // configuration take one launch per final block); GI_SPLIT_PERSIST=0 turns it
 // off.
 bool split_grouped_final(const Ctx* c) {
-  if (!c->split || !c->split->grouped || c->split->s != 9 || getenv("GI_SPLIT_FORCE"))
+  if (!split8_active(c) &&
+      (!c->split || !c->split->grouped || c->split->s != 9 || getenv("GI_SPLIT_FORCE")))
     return false;
   const char* e = getenv("GI_SPLIT_PERSIST");
   return !(e && std::strcmp(e, "0") == 0);
 }
-int split_grouped_max_jobs() { return kGpMaxProb; }
-int split_grouped_items(int nvec, int ncol) {
+int split_grouped_max_jobs(const Ctx* c) { return split8_active(c) ? kMaxProb8 : kGpMaxProb; }
+int split_grouped_items(const Ctx* c, int nvec, int ncol) {
+  if (split8_active(c)) return (round_up(nvec, kBM) / kBM) * ((ncol + kCols8 - 1) / kCols8);
   return (round_up(nvec, kBM) / kBM) * ((ncol + bn2_of(9) - 1) / bn2_of(9));
 }
 
@@ -2419,6 +2286,7 @@ bool split_fused_epilogue(const Ctx* c) {
 
 gi_status split_gemm_final_grouped(Ctx* c, const std::vector<FinalJob>& jobs,
                                    const FusedLines* lines) {
+  if (split8_active(c)) return split8_gemm_final(c, jobs, lines);
   SplitState* S = state(c);
   constexpr int SS = 9, BN = bn2_of(SS), D1 = d1_of(SS);
   if (S->s != SS || !S->grouped || jobs.empty() || (int)jobs.size() > kGpMaxProb) {
@@ -2663,9 +2531,12 @@ gi_status split_build_y_digits(Ctx* c, const double* vecs, int ld, const int32_t
                "Y digits");
 }
 
-int split_digits(const Ctx* c) { return shape_of(c).s; }
+size_t split_digit_bytes(const Ctx* c) {
+  return split8_selected(c) ? (size_t)kDigits8 : 2 * (size_t)shape_of(c).s;
+}
 
 uint64_t split_identity(Ctx* c) {
+  if (split8_active(c)) return split8_identity(c);
   const SplitState* S = state(c);
   const SplitState* D = c->parent ? c->parent->split : S;
   uint64_t h = 1469598103934665603ull;
@@ -2678,15 +2549,18 @@ uint64_t split_identity(Ctx* c) {
 }
 
 const int* split_error_word(const Ctx* c) {
+  if (split8_active(c)) return split8_error_word(c);
   return c->split ? c->split->err.p : nullptr;
 }
 
 gi_status split_check(Ctx* c) {
-  if (!c->split || !c->split->err.p) return GI_OK;
+  const int* word = split_error_word(c);
+  if (!word) return GI_OK;
   int e = 0;
-  if (cudaMemcpy(&e, c->split->err.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
+  if (cudaMemcpy(&e, word, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
     return GI_ERR_CUDA;
   if (e) {
+    split8_error_seen(c);
     char buf[128];
     snprintf(buf, sizeof(buf), "split GEMM: a pipeline wait timed out (code %d)", e);
     c->err = buf;
@@ -2697,9 +2571,11 @@ gi_status split_check(Ctx* c) {
 
 void split_invalidate(Ctx* c) {
   if (c->split) c->split->N = -1;
+  split8_invalidate(c);
 }
 
 void split_release(Ctx* c) {
+  split8_release(c);
   delete c->split;
   c->split = nullptr;
 }
@@ -2748,6 +2624,15 @@ extern "C" gi_status gi_probe_split_gemm(int device, int slices, int M, int N, i
     ck(cudaMemcpy2D(dB.p, sizeof(double) * Kp, B, sizeof(double) * K, sizeof(double) * K, N,
                     cudaMemcpyHostToDevice));
     ck(cudaDeviceSynchronize());
+  }
+  if (g == GI_OK && split8_selected(&c)) {
+    g = split8_probe(&c, M, N, Kp, dA.p, dB.p, Kp, dC.p);
+    if (g == GI_OK) g = split_check(&c);
+    if (g == GI_OK) ck(cudaMemcpy(C, dC.p, sizeof(double) * N * M, cudaMemcpyDeviceToHost));
+    cudaStreamSynchronize(c.stream);
+    split_release(&c);
+    cudaStreamDestroy(c.stream);
+    return g;
   }
   if (g == GI_OK) {
     ck(slice(dA.p, Kp, M, Kp, Mpad, S->s, S->w, S->grouped, sa.p, xa.p, c.stream));

@@ -1,8 +1,28 @@
 // Split-precision (Ozaki-style bf16 slice) GEMMs on the tcgen05 tensor pipe.
 #pragma once
+#include <functional>
+
 #include "engine.h"
 
 namespace gi {
+// One launch configuration of the split GEMM: the kernel (one pass with all
+// diagonals in tensor memory, or two passes with wider tiles) and the L2
+// raster group (row tiles whose digit planes share about ga_mb MB of L2).
+struct GemmConfig {
+  int kind = 1;  // 0: k_split_gemm (one pass); 1, 2: k_split_gemm2 (two passes,
+                 // diagonals split at s/2 or s - s/2); these read the plain
+                 // layout.  6, 7, 8: k_split_gemm_g on the grouped layout (two
+                 // passes split at s/2 or s - s/2, or one pass); 9: its 2-SM
+                 // pair form (256-row tiles, two passes split at s/2, s = 9).
+                 // 3-5 are unused.
+  int ga_mb = 64;
+};
+
+// The autotuner for a GEMM whose launch `run` may be repeated (split.cu); the
+// candidates differ in ga_mb only.  Bumped on every table change: the version.
+gi_status split_tuned(Ctx* c, int s, int nA, int ncols, int K, int layout,
+                      const std::function<cudaError_t(const GemmConfig&)>& run);
+uint64_t split_tuner_version();
 // Z[c][n*ldz + f] = sum_v mu_c(v, f) * Y[n*ldy + v] for c = 0..2, n < ncol.
 // y_digits_ready: split_build_y_digits already wrote Y's digits (Y unused).
 gi_status split_gemm_dipole(Ctx* c, const double* Y, int ldy, double* Z, int ldz, size_t zstride,
@@ -58,8 +78,8 @@ struct FusedLines {
   long long rec_cap;
 };
 bool split_grouped_final(const Ctx* c);  // the persistent grouped launch applies
-int split_grouped_max_jobs();
-int split_grouped_items(int nvec, int ncol);  // work items of one job
+int split_grouped_max_jobs(const Ctx* c);
+int split_grouped_items(const Ctx* c, int nvec, int ncol);  // work items of one job
 // With lines != null the epilogue warps form every job's lines (S, A, I,
 // filters, thresholds) on the last K segment instead of storing T.
 gi_status split_gemm_final_grouped(Ctx* c, const std::vector<FinalJob>& jobs,
@@ -77,8 +97,8 @@ gi_status split_reserve(Ctx* c, size_t max_elems, size_t max_cols,
 // Identity of the split state a captured launch sequence depends on (its
 // workspaces, the dipole digits and the digit shape).
 uint64_t split_identity(Ctx* c);
-// Digit planes per operand the next split-precision run will use.
-int split_digits(const Ctx* c);
+// Bytes of digits per operand element in the next split-precision run.
+size_t split_digit_bytes(const Ctx* c);
 void split_invalidate(Ctx* c);  // the dipole changed: drop its cached slices
 // After a run: reads the device error word the split kernels set on a timeout.
 gi_status split_check(Ctx* c);

@@ -1,0 +1,1140 @@
+// Split-precision GEMMs on the fp8 tensor pipe (sm_103a): the default scheme.
+//
+// C[n*ldc + m] = sum_k A[m][k] B[n][k] in FP64 accuracy from e4m3 products.
+// Each row is scaled by its own power of two so |x| < 1/2 and cut into eleven
+// balanced base-32 digits,
+//   x = sum_p a_p 2^(-5(p+1)) + tail,  a_p in [-16, 16],  |tail| <= 2^-56,
+// every digit an exact e4m3 integer.  Products a_p b_q with p + q = d <= 10
+// share the weight 2^(-5d) and one fp32 accumulator, which stays an exact
+// integer while it is at most 2^24: a product is at most 2^8 and diagonal d
+// has d + 1 of them per k, so every diagonal is exact for any operands up to
+// K = 5952 (11 * 5952 * 2^8 < 2^24; the tensor pipe's fp32 sums of e4m3
+// products were checked bit for bit up to there).  Longer K runs in segments
+// whose FP64 results are added.
+//
+// Why e4m3: 66 digit products of the fp8 pipe replace 45 of the bf16 pipe
+// (nine base-64 digits) at twice the rate, and an element is 11 bytes instead
+// of 18, everywhere it is stored or moved.
+//
+// Why stacked: an MMA costs max(N/2, 32 + N/4) cycles for M = 128 (measured,
+// N = 32..256: below N = 128 it waits for its operands, 128 B/clk of shared
+// memory).  The digit planes of B lie one after the other in shared memory
+// (40 rows each), and so do the accumulators of the diagonals in tensor
+// memory, so plane p of A times planes 0..10-p of B is ONE product of width
+// 40 (11 - p) onto diagonals p..10: 16 MMAs of up to 224 columns per K slice,
+// 1376 cycles against 66 x 42 for one MMA per digit pair.
+//
+// Why blocked operands: the cuts write the digits where the MMA's
+// shared-memory image wants them (32-byte rows, 32-byte swizzle), one K slice
+// of a tile contiguous in memory, so a stage is two bulk copies (45,056 and
+// 14,080 bytes) with no tensor maps.
+#include <cuda_fp16.h>
+#include <cuda_fp8.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdlib>
+#include <cstring>
+
+#include "epilogue.cuh"
+#include "items.cuh"
+#include "split8.h"
+#include "tc.cuh"
+
+namespace gi {
+namespace {
+
+constexpr int kS = kDigits8, kW = 5, kBN = kCols8, kBM = 128;
+constexpr uint32_t kAP = kBM * 32, kBP = kBN * 32;  // bytes of a plane's K slice
+constexpr uint32_t kAS = kS * kAP, kBS = kS * kBP, kStage = kAS + kBS;
+constexpr int kST = 3;            // stages
+constexpr int kSegSlices = 186;   // K = 5952 per exact segment
+constexpr int kHi = 6;            // diagonals 0..5 in the high word of an exact sum
+constexpr int kRing = 4;          // work items in flight between the roles
+constexpr int kThreads = 320;     // warp 0 copies, warp 1 MMA, warps 2..9 epilogue
+// the earlier segments' sums of a tile (20 per epilogue thread), after the
+// stages (256 bytes the junk columns read) and the barriers
+constexpr size_t kSumOff = (size_t)kST * kStage + 256 + 512;
+constexpr size_t kSmem = kSumOff + sizeof(double) * 20 * 256 + 1024;
+static_assert(kSmem <= 227 * 1024, "shared memory");
+static_assert(kStage % 256 == 0 && kAS % 256 == 0, "swizzle periods");
+static_assert((size_t)kS * kSegSlices * 32 * 256 <= (1u << 24), "exact diagonal sums");
+static_assert(kS * kBN + 8 <= 512, "tensor memory columns");
+
+struct Params8 {
+  Prob8 p[kMaxProb8];
+  int nprob, nitems, fused;
+  int* ctr;  // [0] next item, [1] finished CTAs; both back to 0 at the end
+  gi_line* out;
+  unsigned long long* counter;
+  long long cap;
+  RefineRec* rec;
+  long long rec_cap;
+};
+static_assert(sizeof(Params8) <= 32764, "kernel parameter limit");
+
+__device__ __forceinline__ void mma_e4m3(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc,
+                                         uint32_t acc) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+// kind::f8f6f4, e4m3 x e4m3 -> f32, K-major, M = 128.
+__host__ __device__ constexpr uint32_t idesc_e4m3(int N) {
+  return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes,
+                                          uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::
+          "r"(sptr(dst)),
+      "l"(src), "r"(bytes), "r"(sptr(bar))
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(sptr(b)) : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+
+// Every digit product of one K slice: plane p of A with planes 0..10-p of B.
+// The window of j = 11 - p planes is 40 j columns, rounded up to a multiple of
+// 16: the extra 8 fall on columns 440..447, which nothing reads.  Windows past
+// 256 columns take two MMAs.  zero: the first slice of a segment overwrites.
+__device__ __forceinline__ void mma_slice(uint32_t tmem, uint64_t a0, uint64_t b0, bool zero) {
+#pragma unroll
+  for (int j = kS; j >= 1; --j) {
+    const int N = (kBN * j + 15) / 16 * 16;
+    const int N1 = N > 256 ? (N / 2 + 15) / 16 * 16 : N;
+    const uint32_t d = tmem + (uint32_t)(kS - j) * kBN;
+    const uint64_t a = a0 + (uint64_t)((kS - j) * kAP >> 4);
+    const uint32_t acc = (j == kS && zero) ? 0u : 1u;
+    mma_e4m3(d, a, b0, idesc_e4m3(N1), acc);
+    if (N > 256) mma_e4m3(d + N1, a, b0 + (uint64_t)(N1 * 32 >> 4), idesc_e4m3(N - N1), acc);
+  }
+}
+
+// The lines of one thread's four columns: groups of G = ndegI * ndegF
+// consecutive columns are the moments of one initial level.
+template <int G>
+__device__ __forceinline__ void lines_of4(const Params8& P, const Prob8& pr, int n0, int m,
+                                          bool row_ok, const double* v) {
+#pragma unroll
+  for (int g0 = 0; g0 < 4; g0 += G) {
+    const int n = n0 + g0;
+    if (n >= pr.Nc) break;  // the same for every lane of the warp
+    int q = 0;
+    while (q + 1 < pr.nparts && pr.parts[q + 1].c0 <= n) ++q;
+    const EpiPart& pt = pr.parts[q];
+    const EpiParams& ep = pt.ep;
+    const int i = (n - pt.c0) / G;
+    // column offset dI * ndegF + dF within the group -> moment index dI + 2 dF
+    double t[4] = {0.0, 0.0, 0.0, 0.0}, hnq[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int o = 0; o < G; ++o) {
+      const int dI = (G == 4) ? (o >> 1) : (G == 2 ? (ep.ndegF == 1 ? o : 0) : 0);
+      const int dF = (G == 4) ? (o & 1) : (G == 2 ? (ep.ndegF == 1 ? 0 : o) : 0);
+      if (ep.combo_mask & (1 << (dI + 2 * dF))) {
+        t[dI + 2 * dF] = v[g0 + o];
+        hnq[dI + 2 * dF] = pt.hn[i * G + o];
+      }
+    }
+    const bool ok_f = row_ok && pr.upper[m];
+    LineEval r;
+    eval_line(ep, t, hnq, pt.EI[i], ok_f ? pr.EF[m] : 0.0, pt.BI[i], ok_f, pt.lvI[i],
+              ok_f ? pr.lvF[m] : -1, r);
+    append_line(r, ep.part, i, m, P.out, P.counter, P.cap, P.rec, P.rec_cap);
+  }
+}
+
+// One persistent CTA per SM; work items are 128 x 40 tiles of the launch's
+// problems, dealt out by an atomic counter (tiles differ in K).  Bound: the
+// tensor pipe; a tile's epilogue holds the tensor memory only while it folds
+// the diagonals into exact integers, the conversion to FP64 and the stores (or
+// the lines) overlap the next tile's MMAs.
+__global__ void __launch_bounds__(kThreads, 1)
+    k_split8(const __grid_constant__ Params8 P, int* err) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + (size_t)kST * kStage + 256);
+  uint64_t* empty = full + kST;
+  uint64_t* itemf = empty + kST;   // a work item has been published
+  uint64_t* iteme = itemf + kRing; // ... and taken by every epilogue warp
+  uint64_t* accf = iteme + kRing;  // a segment's sums are final
+  uint64_t* tfree = accf + 1;      // ... and have been read
+  uint64_t* drain = tfree + 1;
+  int* items = reinterpret_cast<int*>(drain + 1);
+  int* meta = items + kRing;       // per stage: bit 0 first, 1 last of a segment, 2 of a tile, 3 quit
+  int* seg_last = meta + kST;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(seg_last + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kST; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < kRing; ++i) {
+      mbar_init(&itemf[i], 1);
+      mbar_init(&iteme[i], 8);
+    }
+    mbar_init(accf, 2);  // the MMAs' commit and the issuer's own arrival
+    mbar_init(tfree, 8);
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(
+                     sptr(tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  // item -> problem, row tile, column tile (GA row tiles stay in L2 while the
+  // column tiles stream past them)
+  auto decode = [&](int item, int& pi, int& ai, int& ct) {
+    pi = 0;
+    while (pi + 1 < P.nprob && P.p[pi + 1].first <= item) ++pi;
+    const Prob8& pr = P.p[pi];
+    const int local = item - pr.first;
+    const int grp = local / (pr.GA * pr.nB);
+    const int r = local - grp * pr.GA * pr.nB;
+    const int gsz = min(pr.GA, pr.nA - grp * pr.GA);
+    ai = grp * pr.GA + r % gsz;
+    ct = r / gsz;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {  // scheduler and copies
+      int it = 0, ic = 0;
+      bool ok = true;
+      int item = atomicAdd(P.ctr, 1);
+      for (; ok; ++ic) {
+        const int slot = ic % kRing;
+        if (ic >= kRing) ok = mbar_wait(&iteme[slot], ((ic / kRing) - 1) & 1, abort_flag, err, 41);
+        if (!ok) break;
+        const bool quit = item >= P.nitems;
+        items[slot] = quit ? -1 : item;
+        mbar_arrive(&itemf[slot]);
+        if (quit) break;
+        const int next = atomicAdd(P.ctr, 1);  // used after this tile's copies
+        int pi, ai, ct;
+        decode(item, pi, ai, ct);
+        const Prob8& pr = P.p[pi];
+        const int tile = pr.at ? pr.at[ai].tile : ai;
+        const uint8_t* Ab = pr.A + (size_t)tile * pr.nkA * kAS;
+        const uint8_t* Bb = pr.B + (size_t)ct * pr.nkB * kBS;
+        int ks_next = pr.kl ? pr.kl[0] : 0;
+        for (int k = 0; k < pr.nk; ++k, ++it) {
+          const int st = it % kST, ks = ks_next;
+          if (k + 1 < pr.nk) ks_next = pr.kl ? pr.kl[k + 1] : k + 1;  // ahead of the wait
+          if (it >= kST && !mbar_wait(&empty[st], ((it / kST) - 1) & 1, abort_flag, err, 42)) {
+            ok = false;
+            break;
+          }
+          unsigned char* sa = smem + (size_t)st * kStage;
+          const int in_seg = k % kSegSlices;
+          const bool last = k + 1 == pr.nk;
+          meta[st] = (in_seg == 0 ? 1 : 0) | ((last || in_seg == kSegSlices - 1) ? 2 : 0) |
+                     (last ? 4 : 0);
+          mbar_expect_tx(&full[st], kStage);
+          bulk_load(sa, Ab + (size_t)ks * kAS, kAS, &full[st]);
+          bulk_load(sa + kAS, Bb + (size_t)k * kBS, kBS, &full[st]);
+        }
+        item = next;
+      }
+      if (ok) {  // the MMA issuer leaves on a stage without copies
+        const int st = it % kST;
+        if (it < kST || mbar_wait(&empty[st], ((it / kST) - 1) & 1, abort_flag, err, 43)) {
+          meta[st] = 8;
+          mbar_arrive(&full[st]);
+        }
+      }
+      if (*abort_flag) {  // copies in flight land before the shared memory goes away
+        for (int j = (it > kST ? it - kST : 0); j < it; ++j) {
+          const uint64_t t0 = gtimer();
+          while (!mbar_try(&full[j % kST], (j / kST) & 1) && gtimer() - t0 < 1000000000ull) {
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // MMA issuer
+      int it = 0, seg = 0;
+      bool ok = true;
+      for (;; ++it) {
+        const int st = it % kST;
+        ok = mbar_wait(&full[st], (it / kST) & 1, abort_flag, err, 44);
+        if (!ok) break;
+        const int mt = meta[st];
+        if (mt & 8) break;
+        if ((mt & 1) && seg > 0) {  // the epilogue has read the previous segment
+          ok = mbar_wait(tfree, (seg - 1) & 1, abort_flag, err, 45);
+          if (!ok) break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const uint32_t sa = sptr(smem + (size_t)st * kStage);
+        mma_slice(tmem, sdesc_sw32(sa), sdesc_sw32(sa + kAS), (mt & 1) != 0);
+        mma_commit(&empty[st]);
+        if (mt & 2) {
+          *seg_last = (mt & 4) ? 1 : 0;
+          mma_commit(accf);
+          mbar_arrive(accf);
+          ++seg;
+        }
+      }
+      // every MMA issued has completed before the tensor memory is freed
+      mma_commit(drain);
+      const uint64_t t0 = gtimer();
+      while (!mbar_try(drain, 0) && gtimer() - t0 < 1000000000ull) {
+      }
+    }
+  } else {
+    // warps 2..9: tensor-memory lane quadrant (warp % 4), 20 of the 40 columns
+    const int q4 = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t lanes = (uint32_t)(q4 * 32) << 16;
+    const int r = q4 * 32 + lane;  // row within the tile
+    double* prev = reinterpret_cast<double*>(smem + kSumOff) + (threadIdx.x - 64);
+    int seg = 0;
+    bool ok = true;
+    for (int ic = 0; ok; ++ic) {
+      const int slot = ic % kRing;
+      ok = mbar_wait(&itemf[slot], (ic / kRing) & 1, abort_flag, err, 46, 64);
+      if (!ok) break;
+      const int item = items[slot];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&iteme[slot]);
+      if (item < 0) break;
+      int pi, ai, ct;
+      decode(item, pi, ai, ct);
+      const Prob8& pr = P.p[pi];
+      ATile at;
+      if (pr.at) {
+        at = pr.at[ai];
+      } else {
+        at.tile = ai;
+        at.rows = min(kBM, pr.M - ai * kBM);
+        at.coff = (int64_t)ai * kBM;
+      }
+      const bool row_ok = r < at.rows;
+      const int er = pr.ea[at.tile * kBM + r] - 2 * kW;
+      const int n0 = ct * kBN + half * 20;
+      double sum[20];
+      for (bool last = false, first = true; !last; first = false, ++seg) {
+        ok = mbar_wait(accf, seg & 1, abort_flag, err, 47, 128);
+        if (!ok) break;
+        last = *seg_last != 0;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        // exact sums, hi = diagonals 0..5 and lo = 6..10 (below 2^53 each)
+        long long hi[20], lo[20];
+#pragma unroll
+        for (int ch = 0; ch < 5; ++ch) {
+          uint32_t f[kS][4];
+#pragma unroll
+          for (int d = 0; d < kS; ++d)
+            tmem_ld4(tmem + lanes + d * kBN + half * 20 + ch * 4, f[d]);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            // pairs of diagonals fit 32 bits (|sum| <= 2^24): 2^29 + 2^24
+            auto pair = [&](int d) {
+              return __float2int_rn(__uint_as_float(f[d][j])) * 32 +
+                     __float2int_rn(__uint_as_float(f[d + 1][j]));
+            };
+            long long h = pair(0);
+            h = h * 1024 + pair(2);
+            h = h * 1024 + pair(4);
+            long long l = pair(6);
+            l = l * 1024 + pair(8);
+            l = l * 32 + __float2int_rn(__uint_as_float(f[10][j]));
+            hi[ch * 4 + j] = h;
+            lo[ch * 4 + j] = l;
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(tfree);
+        const int32_t* eb = pr.eb + n0;
+#pragma unroll
+        for (int j = 0; j < 20; j += 2) {
+          const int e0 = er + eb[j], e1 = er + eb[j + 1];
+          const double2 o =
+              scaled_pair2(hi[j], e0 - kW * (kHi - 1), lo[j], e0 - kW * (kS - 1), hi[j + 1],
+                           e1 - kW * (kHi - 1), lo[j + 1], e1 - kW * (kS - 1));
+          sum[j] = o.x;
+          sum[j + 1] = o.y;
+        }
+        if (!first) {
+#pragma unroll
+          for (int j = 0; j < 20; ++j) sum[j] += prev[j * 256];
+        }
+        if (!last) {
+#pragma unroll
+          for (int j = 0; j < 20; ++j) prev[j * 256] = sum[j];
+        }
+      }
+      if (!ok) break;
+      if (P.fused) {
+        const int G = pr.parts[0].grp, m = ai * kBM + r;
+#pragma unroll
+        for (int ch = 0; ch < 5; ++ch) {
+          if (n0 + ch * 4 >= pr.Nc) break;  // the same for every lane
+          if (G == 4)
+            lines_of4<4>(P, pr, n0 + ch * 4, m, row_ok, sum + ch * 4);
+          else if (G == 2)
+            lines_of4<2>(P, pr, n0 + ch * 4, m, row_ok, sum + ch * 4);
+          else
+            lines_of4<1>(P, pr, n0 + ch * 4, m, row_ok, sum + ch * 4);
+        }
+      } else if (row_ok) {
+        double* dst = pr.C + at.coff + r;
+#pragma unroll
+        for (int j = 0; j < 20; ++j)
+          if (n0 + j < pr.Nc) dst[(long long)(n0 + j) * pr.ldc] = sum[j];
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem));
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(P.ctr + 1, 1) == (int)gridDim.x - 1) {  // the last CTA: ready for the next launch
+      P.ctr[0] = 0;
+      P.ctr[1] = 0;
+    }
+  }
+}
+
+// ------------------------------------------------------------------ digits
+// X = round(x 2^(55 - e)), |X| <= 2^54; adding 16 in every base-32 place makes
+// the balanced digits plain 5-bit fields (minus 16), with no carry chain.  The
+// top field is not masked: it reaches 32 (the digit 16).
+constexpr unsigned long long bias_of(int n) {
+  return n == 0 ? 0ull : bias_of(n - 1) | (16ull << (kW * (n - 1)));
+}
+constexpr unsigned long long kBias = bias_of(kS);
+// e4m3 of two digits u - 16, u = 0..32: 0x6400 | u is the half 1024 + u.
+__device__ __forceinline__ uint32_t e4m3x2(uint32_t u0, uint32_t u1) {
+  const uint32_t h = (u0 | 0x6400u) | ((u1 | 0x6400u) << 16);
+  const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&h), __float2half2_rn(1040.0f));
+  return (uint32_t)__nv_cvt_halfraw2_to_fp8x2(static_cast<__half2_raw>(d), __NV_SATFINITE,
+                                              __NV_E4M3);
+}
+// The digits of four consecutive elements k..k+3 of a row: one word per plane,
+// planes `ps` bytes apart.
+__device__ __forceinline__ void cut4(const double* x, int e, uint8_t* dst, uint32_t ps) {
+  unsigned long long b[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) b[i] = (unsigned long long)fixed_point(x[i], e, kW * kS) + kBias;
+#pragma unroll
+  for (int p = 0; p < kS; ++p) {
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u[i] = (uint32_t)(b[i] >> (kW * (kS - 1 - p)));
+      if (p > 0) u[i] &= 31u;
+    }
+    *reinterpret_cast<uint32_t*>(dst + p * ps) = e4m3x2(u[0], u[1]) | (e4m3x2(u[2], u[3]) << 16);
+  }
+}
+// Byte of element k (a multiple of 4) of row r within a tile's slices of
+// `ss` bytes: 32-byte rows, 16-byte halves swapped in every other group of
+// four rows (the 32-byte swizzle).
+__device__ __forceinline__ size_t row_byte(int r, int k, uint32_t ss) {
+  return (size_t)(k >> 5) * ss + r * 32 + ((((k >> 4) ^ (r >> 2)) & 1) << 4) + (k & 15);
+}
+
+__device__ __forceinline__ int block_exponent(unsigned long long mx) {
+  __shared__ unsigned long long wmax[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = wmax[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) mx = max(mx, wmax[i]);
+  return row_exponent(mx) + 1;  // |x| < 2^(e-1): every digit within 16
+}
+__device__ __forceinline__ unsigned long long magnitude(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+}
+
+// One row of K = 4 K4 doubles (null: zeros) into row r of a tile; vk gathers
+// its elements (-1: zero).  Memory bound: 8 B read (twice, the second time
+// from L2) and 11 B written per element.
+__device__ __forceinline__ void cut_row(const double* __restrict__ x, const int32_t* __restrict__ vk,
+                                        int K, uint8_t* tile, uint32_t ps, uint32_t ss, int r,
+                                        int32_t* e_out) {
+  auto get = [&](int k, double* v) {
+    if (!x) {
+      v[0] = v[1] = v[2] = v[3] = 0.0;
+    } else if (vk) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int s = vk[k + i];
+        v[i] = s >= 0 ? x[s] : 0.0;
+      }
+    } else {
+      const double2 a = *reinterpret_cast<const double2*>(x + k);
+      const double2 b = *reinterpret_cast<const double2*>(x + k + 2);
+      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    }
+  };
+  unsigned long long mx = 0;
+  for (int k = threadIdx.x * 4; k < K; k += 1024) {
+    double v[4];
+    get(k, v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mx = max(mx, magnitude(v[i]));
+  }
+  const int e = block_exponent(mx);
+  if (threadIdx.x == 0) *e_out = e;
+  for (int k = threadIdx.x * 4; k < K; k += 1024) {
+    double v[4];
+    get(k, v);
+    cut4(v, e, tile + row_byte(r, k, ss), ps);
+  }
+}
+
+// Rows of an A operand: block b is row b % 128 of tile b / 128.  rowsrc: source
+// row of each (-1: zeros); null: row b of `rows`.
+__global__ void __launch_bounds__(256) k_cut8_a(const double* __restrict__ X, size_t ldx, int rows,
+                                                int K, const int32_t* __restrict__ rowsrc,
+                                                const int32_t* __restrict__ vk,
+                                                uint8_t* __restrict__ out,
+                                                int32_t* __restrict__ e_out) {
+  const int b = blockIdx.x, src = rowsrc ? rowsrc[b] : (b < rows ? b : -1);
+  cut_row(src >= 0 ? X + (size_t)src * ldx : nullptr, vk, K,
+          out + (size_t)(b >> 7) * (K >> 5) * kAS, kAP, kAS, b & 127, e_out + b);
+}
+
+// Rows of several B operands in one launch: operand j has rows
+// [row0[j], row0[j + 1]) of the grid.
+constexpr int kMaxOps8 = kMaxProb8;
+struct CutOps8 {
+  int n;
+  int row0[kMaxOps8 + 1];
+  int K[kMaxOps8];
+  int ldx[kMaxOps8];
+  const double* X[kMaxOps8];
+  uint8_t* out[kMaxOps8];
+  int32_t* e[kMaxOps8];
+};
+__global__ void __launch_bounds__(256) k_cut8_b(const __grid_constant__ CutOps8 ops) {
+  const int b = blockIdx.x;
+  int j = 0;
+  while (j + 1 < ops.n && ops.row0[j + 1] <= b) ++j;
+  const int n = b - ops.row0[j], t = n / kBN;
+  cut_row(ops.X[j] + (size_t)n * ops.ldx[j], nullptr, ops.K[j],
+          ops.out[j] + (size_t)t * (ops.K[j] >> 5) * kBS, kBP, kBS, n - t * kBN, ops.e[j] + n);
+}
+
+// Columns of Y straight into digits: block = one column (i, d) of a (unit,
+// slot) group.  The value at each K position is the symmetrised -> primitive
+// transform of the roots of that (slot, function) (k_build_y's arithmetic, from
+// the basis's table), held in shared memory between the exponent and the cut
+// (recomputed when the row does not fit).
+__global__ void __launch_bounds__(256) k_build_y8(const YItem8* __restrict__ items,
+                                                  const int32_t* __restrict__ tile_item, int n,
+                                                  int cached) {
+  extern __shared__ __align__(16) double ys[];
+  const long long b = blockIdx.x;
+  int q = tile_item ? tile_item[b >> 6] : 0;
+  while (q + 1 < n && items[q + 1].blk0 <= b) ++q;
+  const YItem8& it = items[q];
+  const int j = (int)(b - (tile_item ? it.blk0 : 0));  // i * ndeg + d
+  const int i = j / it.ndeg, d = j - i * it.ndeg;
+  const int K = it.nk * 32;
+  const double* vs = it.vecs + (size_t)it.ivec[i] * it.ld;
+  const double* yc = it.yc + (size_t)d * it.nent * it.nsv;
+  // four consecutive positions: their loads are independent (a position's are
+  // a chain of three)
+  auto values = [&](int k, double* x) {
+    const int4 v4 = *reinterpret_cast<const int4*>(it.vlist + k);
+    const int v[4] = {v4.x, v4.y, v4.z, v4.w};
+    x[0] = x[1] = x[2] = x[3] = 0.0;
+    for (int n = 0; n < it.nent; ++n) {
+      int s[4];
+      double c[4];
+#pragma unroll
+      for (int q4 = 0; q4 < 4; ++q4) {
+        s[q4] = v[q4] >= 0 ? it.ys[n * it.nsv + v[q4]] : 0;
+        c[q4] = v[q4] >= 0 ? yc[n * it.nsv + v[q4]] : 0.0;
+      }
+#pragma unroll
+      for (int q4 = 0; q4 < 4; ++q4)
+        if (c[q4] != 0.0) x[q4] = fma(vs[s[q4]], c[q4], x[q4]);
+    }
+  };
+  unsigned long long mx = 0;
+  for (int k = threadIdx.x * 4; k < K; k += 1024) {
+    double x[4];
+    values(k, x);
+#pragma unroll
+    for (int q4 = 0; q4 < 4; ++q4) mx = max(mx, magnitude(x[q4]));
+    if (cached) {
+      *reinterpret_cast<double2*>(ys + k) = make_double2(x[0], x[1]);
+      *reinterpret_cast<double2*>(ys + k + 2) = make_double2(x[2], x[3]);
+    }
+  }
+  const int e = block_exponent(mx);  // its barrier: every value of the row is in shared memory
+  const int col = it.col0 + j, t = col / kBN, r = col - t * kBN;
+  if (threadIdx.x == 0) it.e_out[col] = e;
+  uint8_t* tile = it.out + (size_t)t * it.nk * kBS;
+  for (int k = threadIdx.x * 4; k < K; k += 1024) {
+    double v[4];
+    if (cached) {
+      const double2 a = *reinterpret_cast<const double2*>(ys + k);
+      const double2 c = *reinterpret_cast<const double2*>(ys + k + 2);
+      v[0] = a.x; v[1] = a.y; v[2] = c.x; v[3] = c.y;
+    } else {
+      values(k, v);
+    }
+    cut4(v, e, tile + row_byte(r, k, kBS), kBP);
+  }
+}
+constexpr int kYSmem = 200 * 1024;  // longest cached row: 25,600 functions
+
+cudaError_t attributes8() {
+  static std::once_flag once;
+  static cudaError_t status = cudaSuccess;
+  std::call_once(once, [] {
+    status = cudaFuncSetAttribute(k_split8, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)kSmem);
+    if (status == cudaSuccess)
+      status = cudaFuncSetAttribute(k_build_y8, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kYSmem);
+  });
+  return status;
+}
+
+}  // namespace
+
+// ------------------------------------------------------------------ host
+struct Split8 {
+  bool on = false;
+  std::unique_ptr<VibPlan> plan;    // (null in a serving worker)
+  // the dipole's digits: made for `mu_uid`'s order of functions
+  uint64_t mu_uid = 0;
+  bool mu_valid = false;
+  int panel = 0;
+  DevArray<uint8_t> mu;
+  DevArray<int32_t> mu_exp, rowsrc, vk, zpos;
+  std::vector<size_t> panel_tile;   // first row-source tile of each panel, and the end
+  DevArray<uint8_t> b;              // B operand workspace
+  DevArray<int32_t> b_exp;
+  DevArray<int> ctr, err;
+  bool err_clean = false;           // the error word is 0
+};
+
+static Split8* st8(Ctx* c) {
+  if (!c->split8) c->split8 = new Split8();
+  return c->split8;
+}
+static gi_status check8(Ctx* c, cudaError_t e, const char* what) {
+  if (e == cudaSuccess) return GI_OK;
+  c->err = std::string("split precision: ") + what + ": " + cudaGetErrorString(e);
+  return e == cudaErrorMemoryAllocation ? GI_ERR_NOMEM : GI_ERR_CUDA;
+}
+
+bool split8_selected(const Ctx* c) {
+  if (c->params.split_slices > 0 || getenv("GI_SPLIT_FORCE")) return false;
+  const char* l = getenv("GI_SPLIT_LAYOUT");
+  return !(l && std::strcmp(l, "plain") == 0);
+}
+bool split8_active(const Ctx* c) { return c->split8 && c->split8->on; }
+
+static uint64_t mix64(uint64_t h, uint64_t v) {
+  h ^= v + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
+  h *= 0xFF51AFD7ED558CCDull;
+  return h ^ (h >> 32);
+}
+
+const VibPlan* vib_plan(Ctx* c, gi_status* st) {
+  *st = GI_OK;
+  Ctx* o = c->parent ? c->parent : c;
+  Split8* S = st8(o);
+  uint64_t key = mix64(14695981039346656037ull, (uint64_t)o->N);
+  for (auto& kv : o->bases) key = mix64(key, kv.second->uid);
+  if (S->plan && S->plan->key == key) return S->plan.get();
+  if (c->parent) {  // bases cannot change while serving
+    *st = fail(c, GI_ERR_STATE, "split precision: the serving context is not prepared");
+    return nullptr;
+  }
+  auto vp = std::make_unique<VibPlan>();
+  const int N = o->N;
+  vp->key = key;
+  vp->N = N;
+  std::vector<int> cls(N, 0);
+  vp->ncls = 1;
+  vp->members.assign(vp->ncls, {});
+  for (int v = 0; v < N; v++)
+    if (cls[v] >= 0) vp->members[cls[v]].push_back(v);
+  vp->zpos.assign(N, -1);
+  int z = 0, s = 0;
+  for (int k = 0; k < vp->ncls; k++) {
+    const int n = (int)vp->members[k].size();
+    vp->z0.push_back(z);
+    vp->s0.push_back(s);
+    for (int i = 0; i < n; i++) vp->zpos[vp->members[k][i]] = z + i;
+    vp->vk.insert(vp->vk.end(), vp->members[k].begin(), vp->members[k].end());
+    vp->vk.resize((size_t)round_up((int)vp->vk.size(), 32), -1);
+    z += round_up(n, 16);
+    s = (int)(vp->vk.size() / 32);
+  }
+  vp->s0.push_back(s);
+  vp->nk = s;
+  vp->ldz = std::max(round_up(z, 64), 64);
+  for (auto& kv : o->bases)
+    vp->support[kv.second->uid].assign((size_t)o->nrep * kv.second->nslot, vp->all());
+  S->plan = std::move(vp);
+  return S->plan.get();
+}
+
+std::vector<VibTile> split8_tiles(const VibPlan& vp, int f0, int rows) {
+  std::vector<VibTile> t;
+  for (int comp = 0; comp < 3; comp++)
+    for (int k = 0; k < vp.ncls; k++) {
+      const auto& m = vp.members[k];
+      const int a = (int)(std::lower_bound(m.begin(), m.end(), f0) - m.begin());
+      const int b = (int)(std::lower_bound(m.begin(), m.end(), f0 + rows) - m.begin());
+      for (int i = a; i < b; i += kBM) t.push_back(VibTile{comp, k, i, std::min(kBM, b - i)});
+    }
+  return t;
+}
+
+gi_status ensure_root_z(Ctx* c, Basis& b, const VibPlan& vp) {
+  if (b.z_uid == vp.uid) return GI_OK;
+  const Split8* S = (c->parent ? c->parent : c)->split8;
+  GI_CUDA(c, b.d_root_z.reserve(std::max(b.D, 1)));
+  GI_CUDA(c, launch_root_z(b, S->zpos.p, b.d_root_z.p, cudaStreamLegacy));
+  GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
+  b.z_uid = vp.uid;
+  return GI_OK;
+}
+
+uint32_t vib_support(const VibPlan& vp, const Basis& b, int gamma, int slot) {
+  auto it = vp.support.find(b.uid);
+  return it == vp.support.end() ? vp.all() : it->second[(size_t)gamma * b.nslot + slot];
+}
+
+void vib_rows_needed(const Ctx* c, const VibPlan& vp, const Basis& bI, int gF, int slot,
+                     uint32_t rset[3]) {
+  const Ctx* o = c->parent ? c->parent : c;
+  int key = 0;
+  while (bI.slot_of_key[key] != slot) key++;
+  const int kI = key >> 1, tauI = key & 1;
+  for (int jF = bI.J - 1; jF <= bI.J + 1; jF++) {
+    auto it = o->bases.find(jF);
+    if (it == o->bases.end()) continue;
+    const Basis& bF = *it->second;
+    for (int kF = std::max(kI - 1, 0); kF <= std::min(kI + 1, jF); kF++)
+      for (int tauF = 0; tauF < 2; tauF++) {
+        const int sF = bF.slot_of_key[2 * kF + tauF];
+        if (sF < 0 || (kF == kI && tauF == tauI)) continue;
+        // the component of the two keys (stencil_fill)
+        rset[kF == kI ? 2 : tauF != tauI ? 0 : 1] |= vib_support(vp, bF, gF, sF);
+      }
+  }
+}
+
+static cudaError_t cut_dipole(Ctx* c, Split8* S, const VibPlan& vp, const double* mu, int p) {
+  const size_t t0 = S->panel_tile[p], nt = S->panel_tile[p + 1] - t0;
+  if (nt == 0) return cudaSuccess;
+  k_cut8_a<<<(unsigned)(nt * kBM), 256, 0, c->stream>>>(mu, (size_t)c->Kp, 0, vp.nk * 32,
+                                                        S->rowsrc.p + t0 * kBM, S->vk.p, S->mu.p,
+                                                        S->mu_exp.p);
+  return cudaGetLastError();
+}
+
+gi_status split8_prepare(Ctx* c) {
+  Split8* S = st8(c);
+  S->on = true;
+  gi_status g;
+  const VibPlan* vp = vib_plan(c, &g);
+  if (!vp) return g;
+  if (!S->err.p) {
+    if ((g = check8(c, S->err.reserve(1), "error word")) != GI_OK) return g;
+    if ((g = check8(c, S->ctr.reserve(2), "work counter")) != GI_OK) return g;
+    if ((g = check8(c, cudaMemsetAsync(S->ctr.p, 0, 2 * sizeof(int), c->stream), "work counter")) !=
+        GI_OK)
+      return g;
+  }
+  if (!S->err_clean) {
+    if ((g = check8(c, cudaMemsetAsync(S->err.p, 0, sizeof(int), c->stream), "error word")) !=
+        GI_OK)
+      return g;
+    S->err_clean = true;
+  }
+  if ((g = check8(c, attributes8(), "kernel attributes")) != GI_OK) return g;
+  if (c->parent) {
+    const Split8* P = c->parent->split8;
+    if (!P || !P->mu_valid || P->mu_uid != vp->uid)
+      return fail(c, GI_ERR_STATE,
+                  "split precision: the dipole digits of the serving context are not prepared");
+    return GI_OK;
+  }
+  const int P = dipole_panel_rows(c);  // 0: the dipole is resident
+  if (S->mu_valid && S->mu_uid == vp->uid && S->panel == P) return GI_OK;
+  S->mu_valid = false;
+  const int N = c->N, step = P ? P : N;
+  std::vector<int32_t> src;
+  S->panel_tile.assign(1, 0);
+  size_t most = 0;
+  for (int f0 = 0; f0 < N; f0 += step) {
+    const auto tiles = split8_tiles(*vp, f0, std::min(step, N - f0));
+    for (const VibTile& t : tiles)
+      for (int r = 0; r < kBM; r++)
+        src.push_back(r < t.rows ? t.comp * step + vp->members[t.cls][t.i0 + r] - f0 : -1);
+    S->panel_tile.push_back(S->panel_tile.back() + tiles.size());
+    most = std::max(most, tiles.size());
+  }
+  if ((g = check8(c, S->rowsrc.assign(src), "dipole rows")) != GI_OK) return g;
+  if ((g = check8(c, S->vk.assign(vp->vk), "dipole columns")) != GI_OK) return g;
+  if ((g = check8(c, S->zpos.assign(vp->zpos), "rows of Z")) != GI_OK) return g;
+  if ((g = check8(c, S->mu.reserve(a_bytes8(most, vp->nk)), "dipole digits")) != GI_OK) return g;
+  if ((g = check8(c, S->mu_exp.reserve(most * kBM), "dipole exponents")) != GI_OK) return g;
+  S->panel = P;
+  S->mu_uid = vp->uid;
+  if (!P) {
+    if ((g = check8(c, cut_dipole(c, S, *vp, c->d_mu.p, 0), "dipole digits")) != GI_OK) return g;
+    if ((g = check8(c, cudaStreamSynchronize(c->stream), "dipole digits")) != GI_OK) return g;
+  }
+  S->mu_valid = true;
+  return GI_OK;
+}
+
+// A final block's digits, cut once and kept with the block until its vectors
+// change (serving workers share blocks: the cut happens under the model lock
+// and the others wait on its event).
+static gi_status block_digits8(Ctx* c, Block& fb, bool wait) {
+  const int vpad = round_up(fb.nvec, kBM);
+  gi_status g;
+  std::lock_guard<std::mutex> lk(c->mmu());
+  if (fb.digits_s != kS || fb.digits_w != kW || fb.digits_layout != 2) {
+    const size_t nd = a_bytes8(vpad / kBM, fb.ld / 32) / sizeof(uint16_t);
+    if (fb.d_digits.n != std::max<size_t>(nd, 1)) {
+      g = check8(c, fb.d_digits.alloc(nd), "V digits");
+      if (g != GI_OK) return g;
+    }
+    if (fb.d_digit_exp.n != (size_t)std::max(vpad, 1)) {
+      g = check8(c, fb.d_digit_exp.alloc(vpad), "V exponents");
+      if (g != GI_OK) return g;
+    }
+    if (vpad) {
+      g = check8(c, timed(c, GI_PHASE_SLICE, [&] {
+                   k_cut8_a<<<vpad, 256, 0, c->stream>>>(
+                       fb.d_vecs.p, (size_t)fb.ld, fb.nvec, fb.ld, nullptr, nullptr,
+                       reinterpret_cast<uint8_t*>(fb.d_digits.p), fb.d_digit_exp.p);
+                   return cudaGetLastError();
+                 }),
+                 "V digits");
+      if (g != GI_OK) return g;
+    }
+    if (!fb.digits_ev) {
+      g = check8(c, cudaEventCreateWithFlags(&fb.digits_ev, cudaEventDisableTiming), "event");
+      if (g != GI_OK) return g;
+    }
+    g = check8(c, cudaEventRecord(fb.digits_ev, c->stream), "event");
+    if (g != GI_OK) return g;
+    fb.digits_s = kS;
+    fb.digits_w = kW;
+    fb.digits_layout = 2;
+  }
+  if (wait && fb.digits_ev) {
+    // inside a graph capture the cut precedes the capture on this stream
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    g = check8(c, cudaStreamIsCapturing(c->stream, &cs), "capture status");
+    if (g != GI_OK) return g;
+    if (cs == cudaStreamCaptureStatusNone) {
+      g = check8(c, cudaStreamWaitEvent(c->stream, fb.digits_ev, 0), "event wait");
+      if (g != GI_OK) return g;
+    }
+  }
+  return GI_OK;
+}
+
+gi_status split8_reserve(Ctx* c, size_t b_bytes, size_t cols, const std::vector<Block*>& finals) {
+  Split8* S = st8(c);
+  gi_status g = check8(c, S->b.reserve(std::max<size_t>(b_bytes, 1)), "B digits");
+  if (g != GI_OK) return g;
+  // a tile's epilogue reads the exponents of all its columns
+  g = check8(c, S->b_exp.reserve(cols + kCols8), "B exponents");
+  if (g != GI_OK) return g;
+  for (Block* b : finals) {
+    g = block_digits8(c, *b, false);
+    if (g != GI_OK) return g;
+  }
+  return GI_OK;
+}
+void split8_dipole_operand(Ctx* c, Prob8* p) {
+  const Split8* D = (c->parent ? c->parent : c)->split8;
+  p->A = D->mu.p;
+  p->ea = D->mu_exp.p;
+  p->nkA = (c->parent ? c->parent : c)->split8->plan->nk;
+}
+uint8_t* split8_b(Ctx* c) { return st8(c)->b.p; }
+int32_t* split8_b_exp(Ctx* c) { return st8(c)->b_exp.p; }
+
+gi_status split8_build_y(Ctx* c, const YItem8* items, const int32_t* tile_item, int n,
+                         long long blocks) {
+  if (n <= 0 || blocks <= 0) return GI_OK;
+  if (blocks > 0x7FFFFFFFll) return check8(c, cudaErrorInvalidValue, "Y digits");
+  gi_status g;
+  const VibPlan* vp = vib_plan(c, &g);
+  if (!vp) return g;
+  const size_t row = (size_t)vp->nk * 32 * sizeof(double);
+  const int cached = row <= (size_t)kYSmem;
+  return check8(c, timed(c, GI_PHASE_CORRELATE, [&] {
+                  k_build_y8<<<(unsigned)blocks, 256, cached ? row : 0, c->stream>>>(
+                      items, tile_item, n, cached);
+                  return cudaGetLastError();
+                }),
+                "Y digits");
+}
+
+// Launches the problems as one work list, longest contractions first.  tune:
+// the launch only stores C, so the autotuner may repeat it.
+gi_status split8_launch(Ctx* c, int phase, std::vector<Prob8>& probs, const FusedLines* lines,
+                        bool tune) {
+  Split8* S = st8(c);
+  std::vector<Prob8> live;
+  for (const Prob8& p : probs)
+    if (p.nA > 0 && p.Nc > 0 && p.nk > 0) live.push_back(p);
+  if (live.empty()) return GI_OK;
+  if (live.size() > (size_t)kMaxProb8) return check8(c, cudaErrorInvalidValue, "problem count");
+  std::stable_sort(live.begin(), live.end(),
+                   [](const Prob8& a, const Prob8& b) { return a.nk > b.nk; });
+  Params8* P = new Params8();  // 16 KB: not on the host stack
+  P->nprob = (int)live.size();
+  P->fused = lines ? 1 : 0;
+  P->ctr = S->ctr.p;
+  if (lines) {
+    P->out = lines->out;
+    P->counter = lines->counter;
+    P->cap = lines->cap;
+    P->rec = lines->rec;
+    P->rec_cap = lines->rec_cap;
+  }
+  long long total_a = 0, total_n = 0, max_k = 0;
+  for (const Prob8& p : live) {
+    total_a = std::max<long long>(total_a, p.nA);
+    total_n += p.Nc;
+    max_k = std::max<long long>(max_k, p.nk);
+  }
+  auto run = [&](const GemmConfig& cfg) -> cudaError_t {
+    long long items = 0;
+    for (int q = 0; q < P->nprob; q++) {
+      Prob8& p = P->p[q];
+      p = live[q];
+      p.nB = (p.Nc + kBN - 1) / kBN;
+      // row tiles whose digits share ga_mb MB of L2
+      p.GA = (int)std::max<size_t>(1, std::min<size_t>(p.nA, ((size_t)cfg.ga_mb << 20) /
+                                                                 ((size_t)p.nk * kAS)));
+      p.first = (int)items;
+      items += (long long)p.nA * p.nB;
+    }
+    if (items > 0x7FFF0000ll) return cudaErrorInvalidValue;
+    P->nitems = (int)items;
+    const int grid = (int)std::min<long long>(items, std::max(c->nsm, 1));
+    k_split8<<<grid, kThreads, kSmem, c->stream>>>(*P, S->err.p);
+    return cudaGetLastError();
+  };
+  gi_status g = GI_OK;
+  timed(c, phase, [&] {
+    if (tune)
+      g = split_tuned(c, kS, (int)total_a, (int)total_n, (int)(max_k * 32), 2, run);
+    else
+      g = check8(c, run(GemmConfig{6, 64}), "GEMM launch");
+    return cudaSuccess;
+  });
+  delete P;
+  return g;
+}
+
+gi_status split8_gemm_dipole(Ctx* c, const std::vector<Band8>& bands, double* Z, int ldz) {
+  Split8* S = st8(c);
+  gi_status g;
+  const VibPlan* vp = vib_plan(c, &g);
+  if (!vp) return g;
+  auto launch = [&](int panel) {
+    std::vector<Prob8> probs;
+    for (const Band8& b : bands) {
+      Prob8 p{};
+      split8_dipole_operand(c, &p);
+      p.B = S->b.p + b.boff;
+      p.eb = S->b_exp.p + b.col0;
+      p.C = Z + b.col0 * (size_t)ldz;
+      p.ldc = ldz;
+      p.at = b.at[panel];
+      p.nA = b.nA[panel];
+      p.kl = b.kl;
+      p.nkB = p.nk = b.nk;
+      p.Nc = (int)b.ncol;
+      probs.push_back(p);
+    }
+    return split8_launch(c, GI_PHASE_HALFLS_GEMM, probs, nullptr, true);
+  };
+  if (!S->panel || c->parent) return launch(0);
+  int p = 0;
+  return for_each_dipole_panel(c, c->stream, [&](const double* mu, size_t, int, int) -> gi_status {
+    gi_status q = check8(c, timed(c, GI_PHASE_SLICE, [&] { return cut_dipole(c, S, *vp, mu, p); }),
+                         "dipole panel digits");
+    return q != GI_OK ? q : launch(p++);
+  });
+}
+
+gi_status split8_gemm_final(Ctx* c, const std::vector<FinalJob>& jobs, const FusedLines* lines) {
+  Split8* S = st8(c);
+  if (jobs.empty() || (int)jobs.size() > kMaxOps8)
+    return fail(c, GI_ERR_STATE, "split precision: final GEMM problem count");
+  gi_status g;
+  const char* bs_env = getenv("GI_BATCH_SMALL");
+  const bool batch = !(bs_env && bs_env[0] == '0');  // off: one cut per problem
+  std::vector<Prob8> probs;
+  CutOps8* ops = new CutOps8();
+  size_t boff = 0, eoff = 0;
+  g = GI_OK;
+  auto cut = [&] {
+    if (ops->n == 0) return GI_OK;
+    const gi_status q = check8(c, timed(c, GI_PHASE_SLICE, [&] {
+                                 k_cut8_b<<<ops->row0[ops->n], 256, 0, c->stream>>>(*ops);
+                                 return cudaGetLastError();
+                               }),
+                               "H digits");
+    ops->n = 0;
+    return q;
+  };
+  for (const FinalJob& j : jobs) {
+    Block& fb = *j.fb;
+    if ((g = block_digits8(c, fb, /*wait=*/true)) != GI_OK) break;
+    if (j.ncol <= 0) continue;
+    Prob8 p{};
+    p.A = reinterpret_cast<const uint8_t*>(fb.d_digits.p);
+    p.ea = fb.d_digit_exp.p;
+    p.B = S->b.p + boff;
+    p.eb = S->b_exp.p + eoff;
+    p.C = j.T;
+    p.ldc = j.ldt;
+    p.nkA = p.nkB = p.nk = j.ldh / 32;
+    p.M = fb.nvec;
+    p.nA = (fb.nvec + kBM - 1) / kBM;
+    p.Nc = j.ncol;
+    p.parts = j.parts;
+    p.nparts = j.nparts;
+    p.EF = j.EF;
+    p.upper = j.upper;
+    p.lvF = j.lvF;
+    if (boff + b_bytes8(j.ncol, p.nk) > S->b.n || eoff + j.ncol + kCols8 > S->b_exp.n ||
+        (lines && (!j.parts || j.nparts <= 0))) {
+      g = fail(c, GI_ERR_STATE, "split precision: final GEMM workspace not prepared");
+      break;
+    }
+    probs.push_back(p);
+    const int o = ops->n++;
+    if (o == 0) ops->row0[0] = 0;
+    ops->K[o] = j.ldh;
+    ops->ldx[o] = j.ldh;
+    ops->X[o] = j.H;
+    ops->out[o] = S->b.p + boff;
+    ops->e[o] = S->b_exp.p + eoff;
+    ops->row0[o + 1] = ops->row0[o] + j.ncol;
+    boff += b_bytes8(j.ncol, p.nk);
+    eoff += round_up(j.ncol, kCols8);  // whole tiles: aligned exponents
+    c->stats.flops_tensor +=
+        (double)kS * (kS + 1) / 2 * 2.0 * fb.nvec * (double)j.ncol * fb.nsize;
+    if (!batch && (g = cut()) != GI_OK) break;
+  }
+  if (g == GI_OK) g = cut();
+  delete ops;
+  if (g != GI_OK) return g;
+  return split8_launch(c, GI_PHASE_FINAL_GEMM, probs, lines, !lines && jobs.size() == 1);
+}
+
+uint64_t split8_identity(Ctx* c) {
+  Split8* S = st8(c);
+  const Split8* D = c->parent ? c->parent->split8 : S;
+  uint64_t h = 0;
+  for (uint64_t v : {(uint64_t)(uintptr_t)S->b.p, (uint64_t)(uintptr_t)S->b_exp.p,
+                     (uint64_t)(uintptr_t)S->ctr.p, (uint64_t)(uintptr_t)S->err.p,
+                     (uint64_t)(uintptr_t)D->mu.p, (uint64_t)(uintptr_t)D->mu_exp.p, D->mu_uid,
+                     split_tuner_version()})
+    h = mix64(h, v);
+  return h;
+}
+void split8_error_seen(Ctx* c) {
+  if (c->split8) c->split8->err_clean = false;
+}
+const int* split8_error_word(const Ctx* c) { return c->split8 ? c->split8->err.p : nullptr; }
+void split8_deactivate(Ctx* c) { c->split8->on = false; }
+void split8_invalidate(Ctx* c) {
+  if (c->split8) c->split8->mu_valid = false;
+}
+void split8_release(Ctx* c) {
+  delete c->split8;
+  c->split8 = nullptr;
+}
+
+gi_status split8_probe(Ctx* c, int M, int N, int K, const double* dA, const double* dB, int ld,
+                       double* dC) {
+  Split8* S = st8(c);
+  S->on = true;
+  const int vpad = round_up(M, kBM), nk = ld / 32;
+  DevArray<uint8_t> a, b;
+  DevArray<int32_t> ea, eb;
+  gi_status g = check8(c, S->err.reserve(1), "error word");
+  if (g == GI_OK) g = check8(c, S->ctr.reserve(2), "work counter");
+  if (g == GI_OK) g = check8(c, cudaMemset(S->err.p, 0, sizeof(int)), "error word");
+  if (g == GI_OK) g = check8(c, cudaMemset(S->ctr.p, 0, 2 * sizeof(int)), "work counter");
+  if (g == GI_OK) g = check8(c, attributes8(), "kernel attributes");
+  if (g == GI_OK) g = check8(c, a.alloc(a_bytes8(vpad / kBM, nk)), "A digits");
+  if (g == GI_OK) g = check8(c, b.alloc(b_bytes8(N, nk)), "B digits");
+  if (g == GI_OK) g = check8(c, ea.alloc(vpad), "A exponents");
+  if (g == GI_OK) g = check8(c, eb.alloc(N + kCols8), "B exponents");
+  if (g == GI_OK) g = check8(c, cudaDeviceSynchronize(), "operands");
+  if (g != GI_OK) return g;
+  k_cut8_a<<<vpad, 256, 0, c->stream>>>(dA, (size_t)ld, M, ld, nullptr, nullptr, a.p, ea.p);
+  if ((g = check8(c, cudaGetLastError(), "A digits")) != GI_OK) return g;
+  CutOps8* ops = new CutOps8();
+  ops->n = 1;
+  ops->row0[0] = 0;
+  ops->row0[1] = N;
+  ops->K[0] = ops->ldx[0] = ld;
+  ops->X[0] = dB;
+  ops->out[0] = b.p;
+  ops->e[0] = eb.p;
+  k_cut8_b<<<N, 256, 0, c->stream>>>(*ops);
+  delete ops;
+  if ((g = check8(c, cudaGetLastError(), "B digits")) != GI_OK) return g;
+  Prob8 p{};
+  p.A = a.p;
+  p.ea = ea.p;
+  p.B = b.p;
+  p.eb = eb.p;
+  p.C = dC;
+  p.ldc = M;
+  p.nkA = p.nkB = p.nk = nk;
+  p.M = M;
+  p.nA = vpad / kBM;
+  p.Nc = N;
+  std::vector<Prob8> probs{p};
+  g = split8_launch(c, GI_PHASE_FINAL_GEMM, probs, nullptr, true);
+  if (g == GI_OK) g = check8(c, cudaStreamSynchronize(c->stream), "probe");
+  return g;
+}
+
+}  // namespace gi

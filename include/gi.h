@@ -84,7 +84,8 @@ typedef struct {
   int32_t quanta_upper[2][GI_MAX_MODES];
   int32_t reduced;         /* SYMMETRY REDUCED */
   int32_t precision;       /* gi_precision */
-  int32_t split_slices;    /* bf16 slices per FP64 operand in GI_PREC_SPLIT (0: default) */
+  int32_t split_slices;    /* GI_PREC_SPLIT: bf16 digits per FP64 operand (2..10); 0: the
+                              default scheme, eleven e4m3 digits */
   int32_t reserved;
   double thresh_linestrength; /* keep lines with S >= this (Debye^2) */
   double thresh_intensity;    /* keep lines with I >= this (cm/molecule) */
@@ -140,8 +141,8 @@ typedef struct {
   double seconds_gpu;      /* device time of the last gi_run (CUDA events) */
   double flops_halfls;     /* algorithmic FP64 flops of the half line strength */
   double flops_final;      /* algorithmic FP64 flops of the final contraction */
-  double flops_tensor;     /* bf16 tensor flops of the split-precision GEMMs: digit-pair
-                              products x 2 x the true (unpadded) M, N and K */
+  double flops_tensor;     /* tensor flops (bf16 or e4m3 digits) of the split-precision GEMMs:
+                              digit-pair products x 2 x the true (unpadded) M, N and K */
   double bytes_correlate;  /* algorithmic HBM bytes of the correlate phase */
   double seconds_phase[GI_NPHASE]; /* device time per phase (GI_RUN_PHASE_TIMING) */
   int32_t launches_phase[GI_NPHASE];

@@ -1,0 +1,39 @@
+"""The default split-precision GEMM (e4m3 digits on the fp8 tensor pipe) alone,
+at the edges of its 128 x 40 tiles, 32-wide K slices and 5952-wide exact
+segments, through gi_probe_split_gemm.
+
+Bound: each operand is rounded to 2^-56 of a power of two at most four times
+its row's largest element, and the dropped digit products (diagonals 11 and up,
+55 pairs of at most 2^8 with weights from 2^-65) add at most 2^-53 of the two
+powers' product per k: together below 2^-48 K max|a| max|b|.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (127, 39, 31), (128, 40, 32), (129, 41, 33),
+                                   (257, 80, 95), (384, 121, 64), (130, 83, 5952),
+                                   (129, 44, 5953), (140, 41, 11969)])
+def test_tile_and_segment_edges(pkg, M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    A = rng.standard_normal((M, K)) * np.exp(rng.uniform(-20.0, 20.0, (M, 1)))
+    B = rng.standard_normal((N, K)) * np.exp(rng.uniform(-20.0, 20.0, (N, 1)))
+    got = pkg.split_gemm(A, B)
+    err = np.abs(got - A @ B.T)
+    bound = np.abs(A).max(axis=1)[:, None] * np.abs(B).max(axis=1)[None, :]
+    assert (err <= (2.0 ** -48 + 2.0 ** -52) * K * bound).all()
+
+
+@pytest.mark.parametrize("value", [0.5 - 2.0 ** -54, 16.0 / 31.0, -1.0, 1.0 / 3.0])
+@pytest.mark.parametrize("K", [5952, 6000])
+def test_constant_rows_stay_exact(pkg, value, K):
+    """Every digit of a plane the same sign and size along K: the largest
+    diagonal sums a segment can reach, where an inexact one would show at
+    2^-24 of the result."""
+    A = np.full((130, K), value)
+    B = np.full((42, K), value)
+    got = pkg.split_gemm(A, B)
+    want = K * value * value
+    assert np.abs(got - want).max() <= 1e-15 * abs(want)
