@@ -184,6 +184,13 @@ struct Basis {
   // (slot, v) -> roots CSR; depends on the dipole size N
   int y_N = -1;
   DevArray<int32_t> d_yptr, d_yroot;
+  // Kinds of J=0 functions: two functions are of one kind when the same
+  // symmetries have a non-zero coefficient on their roots, key by key.  v_kind:
+  // kind of a function (-1: no root); kind_mask: symmetries (bit gamma) of
+  // [kind * nslot + slot].
+  std::vector<int32_t> v_kind;
+  std::vector<uint8_t> kind_mask;
+  int nkind = 0;
   // most symmetrised functions with a non-zero coefficient on one root, per
   // gamma, and most roots on one (slot, v)
   std::vector<int32_t> root_ent;
@@ -445,8 +452,9 @@ struct ZRef {
   double* z = nullptr;
   bool hit = false;
 };
+// gF: the final symmetry whose rows of Z the run computes (-1: every row).
 gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, size_t elems,
-                         ZRef* out);
+                         int gF, ZRef* out);
 void zcache_release(Ctx* w, ZRef& r, bool ok);
 // Stops the serving loop of c (if any): fails queued jobs, joins the workers.
 gi_status server_stop(Ctx* c);
@@ -476,6 +484,10 @@ int dipole_panel_rows(const Ctx* c);
 cudaError_t launch_build_y(const double* vecs, int ld, const int32_t* ivec, int nI, int ndeg,
                            const Basis& b, int gamma, int degen, int N, int Kp, double* Y,
                            cudaStream_t s, int d0 = 0);
+// The symmetries (bit gamma) with a non-zero coefficient on each root, and
+// (ent, zeroed by the caller) the most functions with one on a root, per gamma.
+cudaError_t launch_root_masks(const Basis& b, const std::vector<int32_t>& degen, uint8_t* mask,
+                              int32_t* ent, cudaStream_t s);
 // out[r] = zpos[root_v[r]].
 cudaError_t launch_root_z(const Basis& b, const int32_t* zpos, int32_t* out, cudaStream_t s);
 // Basis::d_ys / d_yc of gamma (E entries per position) from its CSR.

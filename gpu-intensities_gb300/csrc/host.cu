@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <numeric>
+#include <string>
 
 #include "engine.h"
 #include "split8.h"
@@ -174,23 +175,6 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
       for (int j = 0; j < ne; j++) b.s_case[g][s0 + j] = it;
     }
   }
-  // most non-zero coefficients on one root, per gamma
-  b.root_ent.assign(nrep, 0);
-  for (int g = 0; g < nrep; g++) {
-    const int nt = b.Ntotal[g], dg = c->degen[g];
-    for (int r = 0; r < D; r++) {
-      const int ic = b.icontr2icase[r], s0 = b.ijterms[ic + (size_t)g * b.ncase];
-      const int ne = b.Nsym[g + (size_t)ic * nrep];
-      const double* rep = b.repres[g].data() + (size_t)b.icontr2icase[r + D] * dg * nt;
-      int n = 0;
-      for (int j = 0; j < ne; j++) {
-        bool any = false;
-        for (int d = 0; d < dg; d++) any = any || rep[s0 + j + (size_t)d * nt] != 0.0;
-        n += any;
-      }
-      b.root_ent[g] = std::max(b.root_ent[g], n);
-    }
-  }
   // device copies
   std::vector<int32_t> root_lam(D), root_case(D);
   for (int r = 0; r < D; r++) {
@@ -223,6 +207,32 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
     GI_CUDA(c, b.d_rep.back().upload(b.repres[g]));
   }
   b.y_N = -1;
+  // the kinds of functions and the most coefficients on a root
+  DevArray<uint8_t> d_mask;
+  GI_CUDA(c, d_mask.alloc((size_t)D + 4 * (GI_MAX_REP + 1)));
+  int32_t* d_ent = reinterpret_cast<int32_t*>(d_mask.p);
+  GI_CUDA(c, cudaMemsetAsync(d_ent, 0, 4 * GI_MAX_REP, cudaStreamLegacy));
+  GI_CUDA(c, launch_root_masks(b, c->degen, d_mask.p + 4 * GI_MAX_REP, d_ent, cudaStreamLegacy));
+  std::vector<uint8_t> h((size_t)D + 4 * GI_MAX_REP);
+  GI_CUDA(c, cudaMemcpy(h.data(), d_mask.p, h.size(), cudaMemcpyDeviceToHost));
+  const int32_t* ent = reinterpret_cast<const int32_t*>(h.data());
+  b.root_ent.assign(ent, ent + nrep);
+  const uint8_t* mask = h.data() + 4 * GI_MAX_REP;
+  std::vector<uint8_t> use((size_t)(b.iroot_max + 1) * b.nslot, 0);
+  b.v_kind.assign((size_t)b.iroot_max + 1, -1);
+  for (int r = 0; r < D; r++) {
+    use[(size_t)b.iroot[r] * b.nslot + b.slot_of_key[b.root_key[r]]] |= mask[r];
+    b.v_kind[b.iroot[r]] = 0;
+  }
+  std::map<std::string, int> kinds;
+  for (size_t v = 0; v < b.v_kind.size(); v++) {
+    if (b.v_kind[v] < 0) continue;
+    const std::string key(reinterpret_cast<const char*>(&use[v * b.nslot]), b.nslot);
+    const auto it = kinds.emplace(key, (int)kinds.size());
+    b.v_kind[v] = it.first->second;
+    if (it.second) b.kind_mask.insert(b.kind_mask.end(), key.begin(), key.end());
+  }
+  b.nkind = (int)kinds.size();
   return GI_OK;
 }
 
@@ -1073,7 +1083,8 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       ids.insert(ids.end(), h_ivec.begin() + 2 * u.off, h_ivec.begin() + 2 * u.off + u.nI);
     }
     if (one && zblk && ztotal) {
-      gi_status s = zcache_acquire(c, zblk, ids.data(), (int)ids.size(), 3 * ztotal * ldz, &zref);
+      gi_status s = zcache_acquire(c, zblk, ids.data(), (int)ids.size(), 3 * ztotal * ldz,
+                                   s8 ? c->job.gF : -1, &zref);
       if (s != GI_OK) return s;
     }
   }
@@ -1629,10 +1640,9 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
 // every SM has a tile.
 struct HlsPlan8 {
   uint64_t sig = 0, uid = next_uid();
-  DevArray<YItem8> items;
-  DevArray<int32_t> tile_item, vl, slotcol;
-  DevArray<uint16_t> kl;
-  DevArray<ATile> at;
+  DevArray<uint8_t> blob;  // every table below
+  const YItem8* items = nullptr;
+  const int32_t *tile_item = nullptr, *slotcol = nullptr;
   std::vector<Prob8> probs;
   int nitems = 0, nparts = 1, ldz = 0;
   long long blocks = 0;
@@ -1695,7 +1705,6 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
   for (size_t t = 0; t < tiles.size(); t++)
     at.push_back(ATile{(int32_t)t, tiles[t].rows,
                        (int64_t)tiles[t].comp * ldz + vp->z0[tiles[t].cls] + tiles[t].i0});
-  GI_CUDA(c, hp->at.assign(at));
   size_t col0 = 0, boff = 0, nb = 0;
   std::vector<size_t> kl0, vl0;
   for (auto& kv : bands) {
@@ -1708,8 +1717,24 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
           vl.insert(vl.end(), vp->vk.begin() + 32 * (size_t)q, vp->vk.begin() + 32 * (size_t)(q + 1));
         }
   }
-  GI_CUDA(c, hp->kl.assign(kl));
-  GI_CUDA(c, hp->vl.assign(vl));
+  // one allocation and one copy for all tables, each from a 256-byte boundary
+  const size_t nitem = bI.nslot, ntile = (nitem + 63) / 64;
+  size_t at_off = 0, total = 0;
+  auto place = [&](size_t bytes) {
+    const size_t o = total;
+    total += (bytes + 255) / 256 * 256;
+    return o;
+  };
+  at_off = place(at.size() * sizeof(ATile));
+  const size_t kl_off = place(kl.size() * sizeof(uint16_t));
+  const size_t vl_off = place(vl.size() * sizeof(int32_t));
+  const size_t it_off = place(nitem * sizeof(YItem8));
+  const size_t ti_off = place(ntile * sizeof(int32_t));
+  const size_t sc_off = place(nitem * sizeof(int32_t));
+  GI_CUDA(c, hp->blob.alloc(total));
+  const ATile* d_at = reinterpret_cast<const ATile*>(hp->blob.p + at_off);
+  const uint16_t* d_kl = reinterpret_cast<const uint16_t*>(hp->blob.p + kl_off);
+  const int32_t* d_vl = reinterpret_cast<const int32_t*>(hp->blob.p + vl_off);
   for (auto& kv : bands) {
     const int nk = nks[nb];
     for (size_t i = 0; i < kv.second.size(); i++) {
@@ -1722,7 +1747,7 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
       y.nsv = (long long)bI.nslot * c->N;
       y.ys = bI.d_ys[gammaI].p + (size_t)slot * c->N;
       y.yc = bI.d_yc[gammaI].p + (size_t)ideg * y.nent * y.nsv + (size_t)slot * c->N;
-      y.vlist = hp->vl.p + vl0[nb];
+      y.vlist = d_vl + vl0[nb];
       y.out = split8_b(c) + boff;
       y.e_out = split8_b_exp(c) + col0;
       y.ld = round_up(bI.Ntotal[gammaI], 64);
@@ -1743,9 +1768,9 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
       p.eb = split8_b_exp(c) + col0;
       p.C = c->hls_z.p + q * pstride + col0 * 3 * (size_t)ldz;
       p.ldc = 3 * (long long)ldz;
-      p.at = hp->at.p;
+      p.at = d_at;
       p.nA = (int)at.size();
-      p.kl = hp->kl.p + kl0[nb] + k0;
+      p.kl = d_kl + kl0[nb] + k0;
       p.nkB = nk;
       p.nk = k1 - k0;
       p.Nc = (int)kv.second.size();
@@ -1754,15 +1779,26 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
     double nv = 0.0;
     for (int k = 0; k < vp->ncls; k++)
       if (kv.first >> k & 1) nv += (double)vp->members[k].size();
-    hp->flops += (double)kDigits8 * (kDigits8 + 1) / 2 * 2.0 * nv * 3.0 * c->N *
+    double rows = 0.0;
+    for (const VibTile& t : tiles) rows += t.rows;
+    hp->flops += (double)kDigits8 * (kDigits8 + 1) / 2 * 2.0 * nv * rows *
                  (double)kv.second.size();
     col0 += round_up((int)kv.second.size(), kCols8);
     boff += b_bytes8(kv.second.size(), nk);
     nb++;
   }
-  GI_CUDA(c, hp->slotcol.assign(slotcol));
-  GI_CUDA(c, hp->tile_item.assign(tile_item));
-  GI_CUDA(c, hp->items.assign(items));
+  std::vector<uint8_t> blob(total, 0);
+  std::memcpy(blob.data() + at_off, at.data(), at.size() * sizeof(ATile));
+  std::memcpy(blob.data() + kl_off, kl.data(), kl.size() * sizeof(uint16_t));
+  std::memcpy(blob.data() + vl_off, vl.data(), vl.size() * sizeof(int32_t));
+  std::memcpy(blob.data() + it_off, items.data(), items.size() * sizeof(YItem8));
+  std::memcpy(blob.data() + ti_off, tile_item.data(), tile_item.size() * sizeof(int32_t));
+  std::memcpy(blob.data() + sc_off, slotcol.data(), slotcol.size() * sizeof(int32_t));
+  GI_CUDA(c, cudaMemcpy(hp->blob.p, blob.data(), total, cudaMemcpyHostToDevice));
+  GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
+  hp->items = reinterpret_cast<const YItem8*>(hp->blob.p + it_off);
+  hp->tile_item = reinterpret_cast<const int32_t*>(hp->blob.p + ti_off);
+  hp->slotcol = reinterpret_cast<const int32_t*>(hp->blob.p + sc_off);
   hp->nitems = (int)items.size();
   hp->blocks = (long long)items.size();
   if (plans.size() >= 8) plans.pop_back();
@@ -2261,7 +2297,7 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
     double* y = c->hls_y.p;
     double* hh = c->hls_h.p;
     if (h8) {
-      gi_status q = split8_build_y(c, h8->items.p, h8->tile_item.p, h8->nitems, h8->blocks);
+      gi_status q = split8_build_y(c, h8->items, h8->tile_item, h8->nitems, h8->blocks);
       if (q != GI_OK) return q;
       std::vector<Prob8> probs = h8->probs;
       c->stats.flops_tensor += h8->flops;
@@ -2269,7 +2305,7 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
       if (q != GI_OK) return q;
       GI_CUDA(c, launch_half_ls_prim_parts(c->hls_z.p, h8->nparts, h8->pstride, 3 * h8->ldz,
                                            h8->ldz, bF, dst, dstn, 6, hh, c->stream,
-                                           bF.d_root_z.p, h8->slotcol.p));
+                                           bF.d_root_z.p, h8->slotcol));
     } else {
     GI_CUDA(c, launch_build_y(c->hls_v.p, ld, c->hls_iv.p, 1, 1, bI, gammaI, ndeg, c->N, c->Kp,
                               y, c->stream, ideg));

@@ -101,6 +101,48 @@ __global__ void k_y_table(const int32_t* __restrict__ yptr, const int32_t* __res
   }
 }
 
+struct RootMaskArgs {
+  const int32_t *iterm[GI_MAX_REP], *nelem[GI_MAX_REP];
+  const double* rep[GI_MAX_REP];
+  int ntot[GI_MAX_REP], degen[GI_MAX_REP], nrep;
+};
+__global__ void k_root_masks(const __grid_constant__ RootMaskArgs a,
+                             const int32_t* __restrict__ root_case,
+                             const int32_t* __restrict__ root_lam, int D,
+                             uint8_t* __restrict__ mask, int32_t* __restrict__ ent) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= D) return;
+  const int c = root_case[r], lam = root_lam[r];
+  unsigned m = 0;
+  for (int g = 0; g < a.nrep; ++g) {
+    const double* rr = a.rep[g] + a.iterm[g][c] + (size_t)lam * a.degen[g] * a.ntot[g];
+    int n = 0;
+    for (int j = 0; j < a.nelem[g][c]; ++j) {
+      bool any = false;
+      for (int d = 0; d < a.degen[g]; ++d) any = any || rr[j + (size_t)d * a.ntot[g]] != 0.0;
+      n += any;
+    }
+    if (n) m |= 1u << g;
+    if (n > ent[g]) atomicMax(ent + g, n);
+  }
+  mask[r] = (uint8_t)m;
+}
+cudaError_t launch_root_masks(const Basis& b, const std::vector<int32_t>& degen, uint8_t* mask,
+                              int32_t* ent, cudaStream_t s) {
+  RootMaskArgs a{};
+  a.nrep = (int)degen.size();
+  for (int g = 0; g < a.nrep; ++g) {
+    a.iterm[g] = b.d_case_iterm[g].p;
+    a.nelem[g] = b.d_case_nelem[g].p;
+    a.rep[g] = b.d_rep[g].p;
+    a.ntot[g] = b.Ntotal[g];
+    a.degen[g] = degen[g];
+  }
+  k_root_masks<<<(b.D + 255) / 256, 256, 0, s>>>(a, b.d_root_case.p, b.d_root_lam.p, b.D, mask,
+                                                 ent);
+  return cudaGetLastError();
+}
+
 __global__ void k_root_z(const int32_t* __restrict__ root_v, const int32_t* __restrict__ zpos, int D,
                          int32_t* __restrict__ out) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;

@@ -53,6 +53,7 @@ struct JobRec {
 struct ZEntry {
   uint64_t blk_uid = 0, blk_version = 0;
   int precision = 0, slices = 0;
+  int gF = -1;                // the final symmetry it serves (-1: any)
   std::vector<int32_t> ivec;  // the initial records its columns hold
   DevArray<double> z;
   bool valid = false;         // written by a finished run
@@ -187,7 +188,7 @@ gi_status server_make_room(Ctx* c, size_t bytes, Block* keep) {
 
 // ------------------------------------------------------------------ Z cache
 gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, size_t elems,
-                         ZRef* out) {
+                         int gF, ZRef* out) {
   *out = ZRef{};
   Ctx* c = w->parent;
   Server* s = c ? c->server : nullptr;
@@ -197,7 +198,7 @@ gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, 
   for (auto& ep : s->zcache) {
     ZEntry& e = *ep;
     if (e.blk_uid != blk->uid || e.blk_version != blk->version || e.precision != prec ||
-        e.slices != sl || (int)e.ivec.size() != nI ||
+        e.slices != sl || e.gF != gF || (int)e.ivec.size() != nI ||
         !std::equal(e.ivec.begin(), e.ivec.end(), ivec))
       continue;
     if (!e.valid) {  // another job is filling it: compute without the cache
@@ -225,6 +226,7 @@ gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, 
   e->blk_version = blk->version;
   e->precision = prec;
   e->slices = sl;
+  e->gF = gF;
   e->ivec.assign(ivec, ivec + nI);
   if (e->z.alloc(elems) != cudaSuccess) {
     cudaGetLastError();

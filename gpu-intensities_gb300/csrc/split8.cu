@@ -633,7 +633,8 @@ struct Split8 {
   bool mu_valid = false;
   int panel = 0;
   DevArray<uint8_t> mu;
-  DevArray<int32_t> mu_exp, rowsrc, vk, zpos;
+  DevArray<int32_t> mu_exp, tables;  // tables: rowsrc, vk and zpos in one allocation
+  const int32_t *rowsrc = nullptr, *vk = nullptr, *zpos = nullptr;
   std::vector<size_t> panel_tile;   // first row-source tile of each panel, and the end
   DevArray<uint8_t> b;              // B operand workspace
   DevArray<int32_t> b_exp;
@@ -658,18 +659,12 @@ bool split8_selected(const Ctx* c) {
 }
 bool split8_active(const Ctx* c) { return c->split8 && c->split8->on; }
 
-static uint64_t mix64(uint64_t h, uint64_t v) {
-  h ^= v + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
-  h *= 0xFF51AFD7ED558CCDull;
-  return h ^ (h >> 32);
-}
-
 const VibPlan* vib_plan(Ctx* c, gi_status* st) {
   *st = GI_OK;
   Ctx* o = c->parent ? c->parent : c;
   Split8* S = st8(o);
-  uint64_t key = mix64(14695981039346656037ull, (uint64_t)o->N);
-  for (auto& kv : o->bases) key = mix64(key, kv.second->uid);
+  uint64_t key = 14695981039346656037ull ^ (uint64_t)o->N;
+  for (auto& kv : o->bases) key = (key ^ kv.second->uid) * 1099511628211ull;
   if (S->plan && S->plan->key == key) return S->plan.get();
   if (c->parent) {  // bases cannot change while serving
     *st = fail(c, GI_ERR_STATE, "split precision: the serving context is not prepared");
@@ -679,8 +674,38 @@ const VibPlan* vib_plan(Ctx* c, gi_status* st) {
   const int N = o->N;
   vp->key = key;
   vp->N = N;
+  // classes (-1: used by no basis): the common refinement of the bases' kinds
   std::vector<int> cls(N, 0);
+  std::vector<uint8_t> used(N, 0);
   vp->ncls = 1;
+  for (auto& kv : o->bases) {
+    const Basis& b = *kv.second;
+    std::vector<int> id((size_t)vp->ncls * (b.nkind + 1), -1);
+    int n = 0;
+    for (int v = 0; v < N; v++) {
+      const int kind = v < (int)b.v_kind.size() ? b.v_kind[v] : -1;
+      used[v] |= kind >= 0;
+      int& x = id[(size_t)cls[v] * (b.nkind + 1) + kind + 1];
+      if (x < 0) x = n++;
+      cls[v] = x;
+    }
+    vp->ncls = n;
+    if (n > 1024) break;  // far too many to tell apart below
+  }
+  {  // without the unused ones, in order of appearance
+    std::map<int, int> id;
+    for (int v = 0; v < N; v++)
+      cls[v] = used[v] ? id.emplace(cls[v], (int)id.size()).first->second : -1;
+    vp->ncls = std::max<int>(1, (int)id.size());
+  }
+  const bool one = vp->ncls > 32;  // masks of classes are 32 bits: too many kinds, one class
+  if (one) {
+    vp->ncls = 1;
+    for (auto& kv : o->bases)
+      for (size_t v = 0; v < std::min<size_t>(N, kv.second->v_kind.size()); v++)
+        used[v] |= kv.second->v_kind[v] >= 0;
+    for (int v = 0; v < N; v++) cls[v] = used[v] ? 0 : -1;
+  }
   vp->members.assign(vp->ncls, {});
   for (int v = 0; v < N; v++)
     if (cls[v] >= 0) vp->members[cls[v]].push_back(v);
@@ -699,8 +724,21 @@ const VibPlan* vib_plan(Ctx* c, gi_status* st) {
   vp->s0.push_back(s);
   vp->nk = s;
   vp->ldz = std::max(round_up(z, 64), 64);
-  for (auto& kv : o->bases)
-    vp->support[kv.second->uid].assign((size_t)o->nrep * kv.second->nslot, vp->all());
+  for (auto& kv : o->bases) {
+    const Basis& b = *kv.second;
+    auto& sup = vp->support[b.uid];
+    sup.assign((size_t)o->nrep * b.nslot, 0);
+    for (int k = 0; k < vp->ncls; k++) {
+      if (vp->members[k].empty()) continue;
+      // a class is of one kind; with all functions in one class, every kind
+      const size_t v = vp->members[k][0];
+      const int kind = v < b.v_kind.size() ? b.v_kind[v] : -1;
+      for (int q = one ? 0 : kind; q >= 0 && q < (one ? b.nkind : kind + 1); q++)
+        for (int slot = 0; slot < b.nslot; slot++)
+          for (unsigned m = b.kind_mask[(size_t)q * b.nslot + slot]; m; m &= m - 1)
+            sup[(size_t)__builtin_ctz(m) * b.nslot + slot] |= 1u << k;
+    }
+  }
   S->plan = std::move(vp);
   return S->plan.get();
 }
@@ -721,7 +759,7 @@ gi_status ensure_root_z(Ctx* c, Basis& b, const VibPlan& vp) {
   if (b.z_uid == vp.uid) return GI_OK;
   const Split8* S = (c->parent ? c->parent : c)->split8;
   GI_CUDA(c, b.d_root_z.reserve(std::max(b.D, 1)));
-  GI_CUDA(c, launch_root_z(b, S->zpos.p, b.d_root_z.p, cudaStreamLegacy));
+  GI_CUDA(c, launch_root_z(b, S->zpos, b.d_root_z.p, cudaStreamLegacy));
   GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
   b.z_uid = vp.uid;
   return GI_OK;
@@ -756,7 +794,7 @@ static cudaError_t cut_dipole(Ctx* c, Split8* S, const VibPlan& vp, const double
   const size_t t0 = S->panel_tile[p], nt = S->panel_tile[p + 1] - t0;
   if (nt == 0) return cudaSuccess;
   k_cut8_a<<<(unsigned)(nt * kBM), 256, 0, c->stream>>>(mu, (size_t)c->Kp, 0, vp.nk * 32,
-                                                        S->rowsrc.p + t0 * kBM, S->vk.p, S->mu.p,
+                                                        S->rowsrc + t0 * kBM, S->vk, S->mu.p,
                                                         S->mu_exp.p);
   return cudaGetLastError();
 }
@@ -803,9 +841,13 @@ gi_status split8_prepare(Ctx* c) {
     S->panel_tile.push_back(S->panel_tile.back() + tiles.size());
     most = std::max(most, tiles.size());
   }
-  if ((g = check8(c, S->rowsrc.assign(src), "dipole rows")) != GI_OK) return g;
-  if ((g = check8(c, S->vk.assign(vp->vk), "dipole columns")) != GI_OK) return g;
-  if ((g = check8(c, S->zpos.assign(vp->zpos), "rows of Z")) != GI_OK) return g;
+  const size_t nsrc = src.size(), nvk = vp->vk.size();
+  src.insert(src.end(), vp->vk.begin(), vp->vk.end());
+  src.insert(src.end(), vp->zpos.begin(), vp->zpos.end());
+  if ((g = check8(c, S->tables.assign(src), "dipole order")) != GI_OK) return g;
+  S->rowsrc = S->tables.p;
+  S->vk = S->rowsrc + nsrc;
+  S->zpos = S->vk + nvk;
   if ((g = check8(c, S->mu.reserve(a_bytes8(most, vp->nk)), "dipole digits")) != GI_OK) return g;
   if ((g = check8(c, S->mu_exp.reserve(most * kBM), "dipole exponents")) != GI_OK) return g;
   S->panel = P;
@@ -1068,12 +1110,12 @@ gi_status split8_gemm_final(Ctx* c, const std::vector<FinalJob>& jobs, const Fus
 uint64_t split8_identity(Ctx* c) {
   Split8* S = st8(c);
   const Split8* D = c->parent ? c->parent->split8 : S;
-  uint64_t h = 0;
+  uint64_t h = 14695981039346656037ull;
   for (uint64_t v : {(uint64_t)(uintptr_t)S->b.p, (uint64_t)(uintptr_t)S->b_exp.p,
                      (uint64_t)(uintptr_t)S->ctr.p, (uint64_t)(uintptr_t)S->err.p,
                      (uint64_t)(uintptr_t)D->mu.p, (uint64_t)(uintptr_t)D->mu_exp.p, D->mu_uid,
                      split_tuner_version()})
-    h = mix64(h, v);
+    h = (h ^ v) * 1099511628211ull;
   return h;
 }
 void split8_error_seen(Ctx* c) {

@@ -37,3 +37,43 @@ def test_constant_rows_stay_exact(pkg, value, K):
     got = pkg.split_gemm(A, B)
     want = K * value * value
     assert np.abs(got - want).max() <= 1e-15 * abs(want)
+
+
+@pytest.mark.parametrize("case", ["unused", "few_kinds", "many_kinds", "empty_columns"])
+def test_classes_of_functions(pkg, synth, case):
+    """The half-line-strength GEMM skips what the symmetries rule out, by
+    classes of functions that every basis uses alike: functions no basis uses,
+    coefficients missing from some functions (a few classes, or more than the
+    32 a launch tells apart), and keys whose columns are empty for a symmetry.
+    The same lines as the FP64 path, which contracts everything."""
+    rng = np.random.default_rng(3)
+    if case == "unused":
+        prob = synth.make_c2v(61, 90, [1, 2], nvec_max=12, nsize_scale=0.4)
+    else:
+        prob = synth.make_c3v(62, 70, [0, 1, 2, 3], nvec_max=12)
+        kinds = {"few_kinds": 3, "many_kinds": 64, "empty_columns": 1}[case]
+        lost = rng.integers(0, kinds, 70)  # the kind of each function
+        for J, b in prob.bases.items():
+            D = b.Maxcontracts
+            gone = rng.random((kinds, J + 1, 3)) < 0.3
+            for g in range(3):
+                nt, dg = int(b.Ntotal[g]), prob.degen[g]
+                rep = b.repres[g][:nt * dg * b.mat_size].reshape(b.mat_size, dg, nt)
+                nsym = b.Nsym.reshape(-1, 3)[:, g]
+                s0 = np.cumsum(nsym) - nsym
+                for r in range(D):
+                    ic, lam = b.icontr2icase[r], b.icontr2icase[r + D]
+                    k = b.k[r]
+                    if gone[lost[b.iroot_correlat_j0[r]], k, g]:
+                        rep[lam, :, s0[ic]:s0[ic] + nsym[ic]] = 0.0
+    out = []
+    for precision in (pkg.GI_PREC_FP64, pkg.GI_PREC_SPLIT):
+        with pkg.Engine(0) as eng:
+            eng.load(prob, precision=precision)
+            eng.set_refine(1 << 20)
+            eng.run()
+            out.append(np.sort(eng.lines(), order=["level_i", "level_f"]))
+    a, b = out
+    assert len(a) > 300 and np.array_equal(a[["level_i", "level_f"]], b[["level_i", "level_f"]])
+    scale = np.abs(a["t"]).max()
+    assert np.abs(a["t"] - b["t"]).max() <= 1e-12 * scale
