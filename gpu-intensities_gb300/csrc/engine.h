@@ -51,6 +51,12 @@ struct DevArray {
     return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
   }
   cudaError_t upload(const std::vector<T>& v) { return upload(v.data(), v.size()); }
+  // upload without the final wait: one of several, the last of which waits
+  cudaError_t put(const std::vector<T>& v) {
+    const cudaError_t e = alloc(v.size());
+    if (e != cudaSuccess || v.empty()) return e;
+    return cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+  }
   // Like upload, but keeps the allocation (and so the address) when it is
   // large enough: tables a captured CUDA graph reads stay where they were.
   cudaError_t assign(const std::vector<T>& v) {
@@ -320,6 +326,11 @@ struct Ctx {
   gi_line_compact* h_compact = nullptr;
   size_t h_compact_cap = 0;
   int64_t nlines = 0;
+  // gi_sort_lines: ordered copy and tables (kept up to kSortKeep bytes)
+  static constexpr size_t kSortKeep = (size_t)256 << 20;
+  DevArray<uint8_t> w_mask;  // set_basis: symmetries of the roots
+  DevArray<gi_line> w_sorted;
+  DevArray<int32_t> w_sort;
   gi_stats stats{};
 
   // per-phase device timing (GI_RUN_PHASE_TIMING)
@@ -484,6 +495,12 @@ int dipole_panel_rows(const Ctx* c);
 cudaError_t launch_build_y(const double* vecs, int ld, const int32_t* ivec, int nI, int ndeg,
                            const Basis& b, int gamma, int degen, int N, int Kp, double* Y,
                            cudaStream_t s, int d0 = 0);
+// in[0, n) ordered by (level_i, level_f) into out; no two lines of one pair of
+// levels, level ids below nlev <= kSortMaxLevels.  ws: sort_lines_bytes(n, nlev).
+constexpr int kSortMaxLevels = 800000;  // 200 KB of shared memory
+inline size_t sort_lines_bytes(size_t n, int nlev) { return (2 * (size_t)nlev + 1 + 2 * n) * 4; }
+cudaError_t launch_sort_lines(const gi_line* in, gi_line* out, long long n, int nlev, int32_t* ws,
+                              cudaStream_t s);
 // The symmetries (bit gamma) with a non-zero coefficient on each root, and
 // (ent, zeroed by the caller) the most functions with one on a root, per gamma.
 cudaError_t launch_root_masks(const Basis& b, const std::vector<int32_t>& degen, uint8_t* mask,

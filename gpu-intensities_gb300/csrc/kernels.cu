@@ -440,6 +440,130 @@ cudaError_t launch_pack_lines(const gi_line* in, gi_line_compact* out, long long
   return cudaGetLastError();
 }
 
+// ------------------------------------------------------------------ line order
+// Lines ordered by (level_i, level_f).  A pair of levels has at most one line,
+// so within one initial level a line's place is the number of smaller final
+// levels present: counted directly for short lists, else from a bitmap of the
+// final levels.  Three passes over 4-8 B per line and one over the records:
+// bound by the records' 80 B read and written.
+__global__ void k_sort_count(const gi_line* __restrict__ in, long long n, int32_t* __restrict__ cnt) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x)
+    atomicAdd(cnt + in[k].level_i, 1);
+}
+// first[i] = lines of levels below i (first[nlev] = all), cur = a copy (over cnt).
+__global__ void __launch_bounds__(1024) k_sort_scan(int32_t* __restrict__ cur,
+                                                    int32_t* __restrict__ first, int nlev) {
+  __shared__ int part[1024];
+  const int per = (nlev + 1023) / 1024, a = threadIdx.x * per, b = min(a + per, nlev);
+  int s = 0;
+  for (int i = a; i < b; ++i) s += cur[i];
+  part[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 1; o < 1024; o <<= 1) {
+    const int v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
+    __syncthreads();
+    part[threadIdx.x] += v;
+    __syncthreads();
+  }
+  s = threadIdx.x ? part[threadIdx.x - 1] : 0;
+  for (int i = a; i < b; ++i) {
+    const int c = cur[i];
+    first[i] = s;
+    cur[i] = s;
+    s += c;
+  }
+  if (threadIdx.x == 1023) first[nlev] = part[1023];
+}
+__global__ void k_sort_deal(const gi_line* __restrict__ in, long long n, int32_t* __restrict__ cur,
+                            int2* __restrict__ lst) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x) {
+    const int2 l = *reinterpret_cast<const int2*>(in + k);  // level_i, level_f
+    lst[atomicAdd(cur + l.x, 1)] = make_int2(l.y, (int)k);
+  }
+}
+constexpr int kSortDirect = 512;
+__global__ void __launch_bounds__(256) k_sort_place(const gi_line* __restrict__ in,
+                                                    const int2* __restrict__ lst,
+                                                    const int32_t* __restrict__ first, int nlev,
+                                                    gi_line* __restrict__ out) {
+  extern __shared__ unsigned sm[];  // bitmap of the final levels, then its prefix counts
+  const int f0 = first[blockIdx.x], n = first[blockIdx.x + 1] - f0;
+  if (n == 0) return;
+  auto copy = [&](int k, int rank) {
+    const uint4* src = reinterpret_cast<const uint4*>(in + lst[f0 + k].y);
+    uint4* dst = reinterpret_cast<uint4*>(out + f0 + rank);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) dst[q] = src[q];
+  };
+  static_assert(sizeof(gi_line) == 80, "five 16-byte words");
+  if (n <= kSortDirect) {
+    for (int k = threadIdx.x; k < n; k += 256) sm[k] = (unsigned)lst[f0 + k].x;
+    __syncthreads();
+    for (int k = threadIdx.x; k < n; k += 256) {
+      const unsigned f = sm[k];
+      int rank = 0;
+      for (int j = 0; j < n; ++j) rank += sm[j] < f;
+      copy(k, rank);
+    }
+    return;
+  }
+  const int nw = (nlev + 31) >> 5;
+  unsigned* pre = sm + nw;
+  for (int w = threadIdx.x; w < nw; w += 256) sm[w] = 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k < n; k += 256) {
+    const int f = lst[f0 + k].x;
+    atomicOr(sm + (f >> 5), 1u << (f & 31));
+  }
+  __syncthreads();
+  __shared__ unsigned part[256];
+  const int per = (nw + 255) / 256, a = min((int)threadIdx.x * per, nw), b = min(a + per, nw);
+  unsigned s = 0;
+  for (int w = a; w < b; ++w) s += __popc(sm[w]);
+  part[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 1; o < 256; o <<= 1) {
+    const unsigned v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
+    __syncthreads();
+    part[threadIdx.x] += v;
+    __syncthreads();
+  }
+  s = threadIdx.x ? part[threadIdx.x - 1] : 0;
+  for (int w = a; w < b; ++w) {
+    pre[w] = s;
+    s += __popc(sm[w]);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < n; k += 256) {
+    const int f = lst[f0 + k].x;
+    copy(k, (int)(pre[f >> 5] + __popc(sm[f >> 5] & ((1u << (f & 31)) - 1u))));
+  }
+}
+
+cudaError_t launch_sort_lines(const gi_line* in, gi_line* out, long long n, int nlev, int32_t* ws,
+                              cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  if (nlev <= 0 || nlev > kSortMaxLevels || n > 0x7FFFFFFFll) return cudaErrorInvalidValue;
+  const size_t sm = std::max<size_t>(8 * (size_t)((nlev + 31) / 32), 4 * kSortDirect);
+  cudaError_t e = cudaSuccess;
+  if (sm > 48 * 1024)
+    e = cudaFuncSetAttribute(k_sort_place, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  // lists first: 8-byte aligned; then the cursors and the offsets
+  int2* lst = reinterpret_cast<int2*>(ws);
+  int32_t* cur = ws + 2 * n;
+  int32_t* first = cur + nlev;
+  if (e == cudaSuccess) e = cudaMemsetAsync(cur, 0, sizeof(int32_t) * nlev, st);
+  if (e != cudaSuccess) return e;
+  const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 152 * 16);
+  k_sort_count<<<blocks, 256, 0, st>>>(in, n, cur);
+  k_sort_scan<<<1, 1024, 0, st>>>(cur, first, nlev);
+  k_sort_deal<<<blocks, 256, 0, st>>>(in, n, cur, lst);
+  k_sort_place<<<nlev, 256, sm, st>>>(in, lst, first, nlev, out);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_boltz(const double* E, int n, double zpe, double beta, double* out,
                          cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
