@@ -193,17 +193,20 @@ gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, 
   Ctx* c = w->parent;
   Server* s = c ? c->server : nullptr;
   if (!s || !s->zcache_on || nI <= 0) return GI_OK;
-  std::lock_guard<std::mutex> lk(c->model_mu);
+  std::unique_lock<std::mutex> lk(c->model_mu);
   const int prec = w->params.precision, sl = w->params.split_slices;
-  for (auto& ep : s->zcache) {
-    ZEntry& e = *ep;
+  for (size_t k = 0; k < s->zcache.size(); k++) {
+    ZEntry& e = *s->zcache[k];
     if (e.blk_uid != blk->uid || e.blk_version != blk->version || e.precision != prec ||
         e.slices != sl || e.gF != gF || (int)e.ivec.size() != nI ||
         !std::equal(e.ivec.begin(), e.ivec.end(), ivec))
       continue;
-    if (!e.valid) {  // another job is filling it: compute without the cache
-      s->z_misses++;
-      return GI_OK;
+    if (!e.valid) {
+      // another job is computing it: its end (or its failure, which drops the
+      // entry) comes before this job could have computed it beside
+      s->cv_done.wait(lk);
+      k = (size_t)-1;  // the list may have changed: look again
+      continue;
     }
     e.pins++;
     e.last_use = ++s->clock;
@@ -258,6 +261,7 @@ void zcache_release(Ctx* w, ZRef& r, bool ok) {
     }
     break;
   }
+  if (!r.hit) s->cv_done.notify_all();
   r = ZRef{};
 }
 
