@@ -388,7 +388,7 @@ struct Ctx {
   std::vector<HlsGraph> hls_graphs;  // most recently used first
   uint64_t hls_last_sig = 0;         // the last call run eagerly
   std::vector<std::shared_ptr<HlsPlan8>> hls_plans8;  // most recently used first, at most 8
-  DevArray<int32_t> hls_iv;
+  DevArray<int32_t> hls_iv, hls_cnt;
   DevArray<double> w_y, w_z, w_h, w_t, w_EI;
   DevArray<unsigned long long> w_counter;
   DevArray<int32_t> w_ivec, w_int;
@@ -522,6 +522,13 @@ HItem make_h_item(const double* Z, size_t zstride_c, int ldz, int nslotI, int nd
 // Every item of a device table in one launch (nblocks = the items' blocks).
 cudaError_t launch_build_h_items(const HItem* items, const long long* firsts, int nitems,
                                  long long nblocks, cudaStream_t st);
+// One vector's half line strength in FP64 (fp64.cu): the columns of Y
+// ([nslot][Kp]) packed in place to their non-zero values, and rows [0, rows) of
+// three dipole components times them: Z[c * zc + slot * ldz + row].
+cudaError_t launch_pack_y(double* Y, int nslot, int N, int Kp, int32_t* count, cudaStream_t s);
+cudaError_t launch_dipole_rows(const double* mu, size_t mstride, int Kp, int rows, const double* Y,
+                               const int32_t* count, int nslot, int N, double* Z, size_t zc,
+                               int ldz, cudaStream_t s);
 cudaError_t launch_half_ls_prim(const double* Z, size_t zstride_c, int ldz, const Basis& bF,
                                 const StencilTerm* st, const int32_t* st_n, int st_max,
                                 double* h, cudaStream_t s);

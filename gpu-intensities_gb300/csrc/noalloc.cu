@@ -11,15 +11,16 @@
 // and the scratch lives in one file-scope device array of fixed size
 // (kScratchBytes), which every GPU that loads the library holds until exit.
 //
-// Scratch use per call: Y (ndeg * nslot * Kp doubles, zeroed at the start of
-// every call because the scatter accumulates into it) and Z (3x that, fully
-// written by the GEMM before it is read).  The 3j/K-tau term tables and the
+// Scratch use per call: Y of the requested component (nslot * Kp doubles, zeroed
+// at the start of every call because the scatter accumulates into it, then
+// packed in place) and Z (3x that, fully written before it is read); the size
+// limit counts every component.  A second array holds the packed rows' counts.  The 3j/K-tau term tables and the
 // key -> slot map are device tables of the initial basis, built when the basis
 // or the 3j table is set, so a call copies nothing from the host: it checks
 // its arguments against sizes the setters recorded and enqueues device work.
-// The array keeps the last call's contents; calls whose work overlaps on the
-// GPU share the array and race, so a caller must order them (one stream, or
-// events).
+// The array keeps the last call's contents.  Calls on different streams of one
+// device are ordered by an event recorded after each call, which the next one
+// waits for; inside a stream capture that is left to the caller.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,20 +37,24 @@ constexpr size_t kMaxElems = size_t(1) << 19;                     // ndeg * nslo
 constexpr size_t kScratchBytes = 4 * kMaxElems * sizeof(double);  // Y + 3 Z = 16 MiB
 static_assert(kScratchBytes == GI_NOALLOC_SCRATCH_BYTES, "scratch size stated in gi.h");
 
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
+// the counts of the packed rows of Y (a row has at least 64 places) go with it
+constexpr size_t kMaxRows = kMaxElems / 64;
+static __device__ __align__(256) unsigned char
+    g_noalloc_scratch[kScratchBytes + kMaxRows * sizeof(int32_t)];
 
-std::mutex g_mutex;
+std::mutex g_mutex;  // also held while a call is issued
 void* g_scratch_dev[kMaxDevices] = {};
+cudaEvent_t g_done[kMaxDevices] = {};  // the last call's work (made with the first call)
 
 // Device address of the scratch array on `device`, looked up once per device
 // with that device current.  In host code the array's name is only a
 // host-side stand-in, so kernels must be given this address.
 cudaError_t scratch_address(int device, unsigned char** out) {
   if (device < 0 || device >= kMaxDevices) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lock(g_mutex);
   if (!g_scratch_dev[device]) {
     void* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+    cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g_done[device], cudaEventDisableTiming);
     if (e != cudaSuccess) return e;
     g_scratch_dev[device] = p;
   }
@@ -58,7 +63,7 @@ cudaError_t scratch_address(int device, unsigned char** out) {
 }
 
 // Symmetrised -> primitive transform of one initial vector (the arithmetic of
-// k_build_y, dipole_kernals.cu:38-71), scattered onto Y[d][slot][v] with an
+// k_build_y, dipole_kernals.cu:38-71), component d, scattered onto Y[slot][v] with an
 // atomic add so that no (slot, v) index table is needed.
 __global__ void k_scatter_y(const double* __restrict__ vsym, const int32_t* __restrict__ root_v,
                             const int32_t* __restrict__ root_key,
@@ -67,10 +72,9 @@ __global__ void k_scatter_y(const double* __restrict__ vsym, const int32_t* __re
                             const int32_t* __restrict__ case_iterm,
                             const int32_t* __restrict__ case_nelem,
                             const double* __restrict__ rep, int Ntot, int degen,
-                            const int32_t* __restrict__ slot_of_key, int D, int nslot, int Kp,
+                            const int32_t* __restrict__ slot_of_key, int D, int d, int Kp,
                             double* __restrict__ Y) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  const int d = blockIdx.y;
   if (r >= D) return;
   const int c = root_case[r], lam = root_lam[r];
   const int it = case_iterm[c], ne = case_nelem[c];
@@ -78,7 +82,7 @@ __global__ void k_scatter_y(const double* __restrict__ vsym, const int32_t* __re
   double acc = 0.0;
   for (int j = 0; j < ne; ++j) acc = fma(vsym[it + j], rr[it + j], acc);
   const int slot = slot_of_key[root_key[r]];
-  atomicAdd(&Y[((size_t)d * nslot + slot) * Kp + root_v[r]], acc);
+  atomicAdd(&Y[(size_t)slot * Kp + root_v[r]], acc);
 }
 
 }  // namespace
@@ -123,37 +127,41 @@ extern "C" gi_status gi_half_ls_noalloc(gi_ctx* h, int jI, int gammaI, int ideg,
     return say(GI_ERR_STATE, "gi_half_ls_noalloc: the basis has no term tables");
   if (cudaSetDevice(c->device) != cudaSuccess)
     return say(GI_ERR_CUDA, "gi_half_ls_noalloc: cudaSetDevice failed");
+  std::lock_guard<std::mutex> lock(g_mutex);
   unsigned char* base = nullptr;
   if (scratch_address(c->device, &base) != cudaSuccess)
     return say(GI_ERR_CUDA, "gi_half_ls_noalloc: cudaGetSymbolAddress of the scratch failed");
   double* Y = reinterpret_cast<double*>(base);
-  double* Z = Y + elems;
+  const size_t zc = (size_t)bI.nslot * c->Kp;
+  double* Z = Y + zc;
+  int32_t* count = reinterpret_cast<int32_t*>(base + kScratchBytes);
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->stream;
 
-  cudaError_t e = cudaMemsetAsync(Y, 0, sizeof(double) * elems, s);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &cs);
+  const bool order = cs == cudaStreamCaptureStatusNone;
+  if (e == cudaSuccess && order) e = cudaStreamWaitEvent(s, g_done[c->device], 0);
+  if (e == cudaSuccess) e = cudaMemsetAsync(Y, 0, sizeof(double) * zc, s);
   if (e == cudaSuccess) {
-    dim3 grid((bI.D + 255) / 256, ndeg);
-    k_scatter_y<<<grid, 256, 0, s>>>(vsym_dev, bI.d_root_v.p, bI.d_root_key.p, bI.d_root_case.p,
-                                     bI.d_root_lam.p, bI.d_case_iterm[gammaI].p,
-                                     bI.d_case_nelem[gammaI].p, bI.d_rep[gammaI].p,
-                                     bI.Ntotal[gammaI], ndeg, bI.d_slot_of_key.p, bI.D, bI.nslot,
-                                     c->Kp, Y);
+    k_scatter_y<<<(bI.D + 255) / 256, 256, 0, s>>>(
+        vsym_dev, bI.d_root_v.p, bI.d_root_key.p, bI.d_root_case.p, bI.d_root_lam.p,
+        bI.d_case_iterm[gammaI].p, bI.d_case_nelem[gammaI].p, bI.d_rep[gammaI].p,
+        bI.Ntotal[gammaI], ndeg, bI.d_slot_of_key.p, bI.D, ideg, c->Kp, Y);
     e = cudaGetLastError();
   }
-  const int ncol = ndeg * bI.nslot;
-  const size_t zc = (size_t)ncol * c->Kp;
+  if (e == cudaSuccess) e = launch_pack_y(Y, bI.nslot, c->N, c->Kp, count, s);
   if (e == cudaSuccess) {
     // a streamed dipole passes through its preallocated staging panels
     const gi_status g = for_each_dipole_panel(c, s, [&](const double* mu, size_t ms, int rows,
                                                          int f0) {
-      e = gemm_fp64_nt(mu, c->Kp, ms, Y, c->Kp, Z + f0, c->Kp, zc, rows, ncol, c->Kp, 3, s);
+      e = launch_dipole_rows(mu, ms, c->Kp, rows, Y, count, bI.nslot, c->N, Z + f0, zc, c->Kp, s);
       return e == cudaSuccess ? GI_OK : GI_ERR_CUDA;
     });
     if (g != GI_OK && e == cudaSuccess) return g;  // a stream/event call failed (c->err set)
   }
   if (e == cudaSuccess)
-    e = launch_half_ls_prim(Z + (size_t)ideg * bI.nslot * c->Kp, zc, c->Kp, bF, d_st.p, d_stn.p,
-                            6, half_ls_dev, s);
+    e = launch_half_ls_prim(Z, zc, c->Kp, bF, d_st.p, d_stn.p, 6, half_ls_dev, s);
+  if (e == cudaSuccess && order) e = cudaEventRecord(g_done[c->device], s);
   if (e != cudaSuccess) {
     c->err = std::string("gi_half_ls_noalloc: ") + cudaGetErrorString(e);
     return GI_ERR_CUDA;

@@ -299,15 +299,17 @@ gi_status gi_half_ls(gi_ctx* ctx, int jI, int gammaI, int ideg, int jF, const do
    device-wide synchronisation of cudaMalloc/cudaFree.  The call allocates
    nothing: vsym_dev (nsize doubles of block (jI, gammaI)) and half_ls_dev
    (D_F doubles) are device buffers the caller owns, and the scratch is one
-   fixed device array of GI_NOALLOC_SCRATCH_BYTES inside the library, held by
+   fixed device array of GI_NOALLOC_SCRATCH_BYTES (and 32 KiB of counts)
+   inside the library, held by
    every GPU that loads it until the process exits.  Limit: degen(gammaI) *
    (number of (k, tau) slots of J=jI) * round_up(N, 64) <= 2^19; larger sizes
    return GI_ERR_ARG (use gi_half_ls).  The rotational term tables it reads
    are built by gi_set_basis / gi_set_threej, so the call copies nothing from
    the host: the work is enqueued on `stream` (a cudaStream_t; NULL = the
    context's stream) and the call returns without waiting.  All calls share
-   the scratch array, which keeps the last call's contents: calls whose work
-   overlaps on the GPU race, so order them (one stream, or events).  The first
+   the scratch array, which keeps the last call's contents: each call's work
+   waits for the last one's, whichever stream it is on.  Calls captured into
+   graphs are not ordered that way: order their launches (one stream, or events).  The first
    call on a device looks up the array's device address once
    (cudaGetSymbolAddress) with that device current; make that first call
    before any stream capture. */
