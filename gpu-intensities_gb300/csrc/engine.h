@@ -168,6 +168,17 @@ struct EpiPart {
   EpiParams ep;
 };
 
+// One part of a batched stand-alone epilogue: it has blocks [blk0, blk0 +
+// nI ceil(nF / 128)) of the grid.
+struct EpiItem {
+  const double* T;
+  const double *EI, *EF, *hn;
+  const int32_t *lvI, *lvF;
+  const uint8_t* upper;
+  int ldt, nI, nF, pad;
+  EpiParams ep;
+  long long blk0;
+};
 // Process-wide serial numbers: a captured launch sequence is tied to the
 // exact basis objects it read.
 uint64_t next_uid();
@@ -408,6 +419,7 @@ struct Ctx {
   DevArray<int32_t> w_ytile8, w_vl8, w_slotcol;
   DevArray<uint16_t> w_kl8;
   DevArray<ATile> w_at8;
+  DevArray<EpiItem> w_epiitems;  // FP64: the epilogue's parts of every group
   DevArray<RefineRec> w_rec;   // lines handed to the exact re-evaluation
   int64_t refine_max = 0;      // doubtful lines re-evaluated per run (gi_set_refine)
   DevArray<int32_t> w_stencil_n, w_levelI, w_levelF;
@@ -479,9 +491,6 @@ void ctx_release(Ctx* c);
 // doubles are on the device.  A resident dipole is one panel of N rows.
 using PanelFn = std::function<gi_status(const double*, size_t, int, int)>;
 gi_status for_each_dipole_panel(Ctx* c, cudaStream_t st, const PanelFn& fn);
-// Z_c = mu_c^T Y in FP64 (rows f of Z at ldz, components zc apart).
-gi_status dipole_gemm_fp64(Ctx* c, const double* Y, int ldy, double* Z, int ldz, size_t zc,
-                           int ncol, cudaStream_t st);
 // Makes `pinned` (cudaMallocHost, [3][N][N] record order) the context's
 // streamed dipole; the context frees it.
 gi_status dipole_stream_adopt(Ctx* c, int N, double* pinned, int panel_rows);
@@ -522,6 +531,21 @@ HItem make_h_item(const double* Z, size_t zstride_c, int ldz, int nslotI, int nd
 // Every item of a device table in one launch (nblocks = the items' blocks).
 cudaError_t launch_build_h_items(const HItem* items, const long long* firsts, int nitems,
                                  long long nblocks, cudaStream_t st);
+// A GEMM of an FP64 launch (fp64.cu): C[coff + n ldc + r] over row tiles of A
+// (at: 128-row tiles whose rows rowsrc names, nM = 4 per tile; else rows of M, nM
+// = ceil(M / 32)), A's elements gathered by vl (-1: zero) when given.
+struct ProbF {
+  const double* A;
+  const double* B;
+  double* C;
+  long long lda, ldc;
+  const ATile* at;
+  const int32_t* rowsrc;
+  const int32_t* vl;
+  int ldb, K, M, nM, Nc, first;
+};
+constexpr int kMaxProbF = 96;
+cudaError_t launch_gemm_f64(std::vector<ProbF> probs, cudaStream_t s);
 // One vector's half line strength in FP64 (fp64.cu): the columns of Y
 // ([nslot][Kp]) packed in place to their non-zero values, and rows [0, rows) of
 // three dipole components times them: Z[c * zc + slot * ldz + row].
@@ -576,17 +600,16 @@ cudaError_t launch_epilogue(const double* T, int ldt, int nI, int nF, const int3
                             const uint8_t* upper_ok, const double* hn, const EpiParams& p,
                             gi_line* out, unsigned long long* counter, long long cap,
                             RefineRec* rec, long long rec_cap, cudaStream_t s);
+// The same for several parts in one launch.
+cudaError_t launch_epilogue_items(const EpiItem* items, int nitems, long long blocks, gi_line* out,
+                                  unsigned long long* counter, long long cap, RefineRec* rec,
+                                  long long rec_cap, cudaStream_t s);
 // out[col] = || H[col * ldh + 0 .. n) ||_2 for col < ncol.
 cudaError_t launch_col_norms(const double* H, int ldh, int n, int ncol, double* out,
                              cudaStream_t s);
 // The same for the H of several final blocks in one launch (NormItem).
 cudaError_t launch_col_norms_items(const NormItem* items, int nitems, long long ncol,
                                    cudaStream_t s);
-// C[z][n*ldc + m] = sum_k A[z][m*lda + k] * B[n*ldb + k]; K multiple of 16.
-cudaError_t gemm_fp64_nt(const double* A, int lda, size_t strideA, const double* B, int ldb,
-                         double* C, int ldc, size_t strideC, int M, int Nc, int K, int batch,
-                         cudaStream_t s);
-
 // ------------------------------------------------------------------ host math
 double three_j(int j1, int j2, int j3, int k1, int k2, int k3);
 void precompute_threej(int jmax, std::vector<double>& out);

@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <vector>
 
 #include "engine.h"
 
@@ -115,6 +116,121 @@ __global__ void __launch_bounds__(128)
     const int i = (up ? 2 : 0) + (odd ? 1 : 0);
     if ((lane & 7) == 0 && i < nr) Z[blockIdx.y * zc + (size_t)slot * ldz + f0 + i] = s;
   }
+}
+
+// ------------------------------------------------------------------ GEMMs
+// C[coff(row tile) + n ldc + r] = sum_k A[row][vl[k]] B[n][k] for a list of
+// problems in one launch (DMMA m8n8k4).  A block is a 32 x 32 tile, a warp 16 x
+// 16 of it, operands straight from L1 and L2: a step of 16 k keeps a
+// sub-partition's FP64 pipe busy for 9500 clocks, so nothing else shows, and
+// small tiles fill the GPU at small sizes and waste little at ragged ones
+// (64 x 64 tiles, one launch per final block: 27 tiles of 300 us for a 187 x 561
+// problem; C2v N = 200, J <= 2: 4.6 ms of GEMMs, 0.6 ms this way).
+struct ParamsF {
+  ProbF p[kMaxProbF];
+  int nprob;
+};
+__global__ void __launch_bounds__(128) k_gemm_f64(const __grid_constant__ ParamsF P) {
+  int q = 0;
+  while (q + 1 < P.nprob && P.p[q + 1].first <= (int)blockIdx.x) ++q;
+  const ProbF& pr = P.p[q];
+  const int local = blockIdx.x - pr.first;
+  // row tiles fastest: the blocks in flight share columns of B
+  const int rt = local % pr.nM, n0 = (local / pr.nM) * 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  // rows of the tile: at/rowsrc (128-row tiles, four blocks each) or plain rows
+  int tile = 0, r0 = rt * 32, rows = pr.M;
+  int64_t coff = 0;
+  if (pr.at) {
+    const ATile a = pr.at[rt >> 2];
+    tile = a.tile * 128;
+    r0 = (rt & 3) * 32;
+    rows = a.rows;
+    coff = a.coff;
+  }
+  if (r0 >= rows) return;
+  const int wr = r0 + (warp >> 1) * 16, wc = n0 + (warp & 1) * 16;
+  if (wr >= rows || wc >= pr.Nc) return;
+  const double *a[2], *b[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = min(wr + i * 8 + g, rows - 1), n = min(wc + i * 8 + g, pr.Nc - 1);
+    a[i] = pr.A + (size_t)(pr.at ? pr.rowsrc[tile + r] : r) * pr.lda;
+    b[i] = pr.B + (size_t)n * pr.ldb + t;
+  }
+  double acc[2][2][2] = {};
+  double av[2][4], bv[2][4];
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const int v = pr.vl ? pr.vl[k + kk * 4 + t] : k + kk * 4 + t;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        av[i][kk] = v >= 0 ? a[i][v] : 0.0;
+        bv[i][kk] = b[i][k + kk * 4];
+      }
+    }
+  };
+  fetch(0);
+  for (int k = 0; k < pr.K; k += 16) {
+    double ac[2][4], bc[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        ac[i][kk] = av[i][kk];
+        bc[i][kk] = bv[i][kk];
+      }
+    if (k + 16 < pr.K) fetch(k + 16);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          asm volatile(
+              "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+              : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+              : "d"(ac[i][kk]), "d"(bc[j][kk]));
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = wr + i * 8 + g, n = wc + j * 8 + t * 2 + e;
+        if (r < rows && n < pr.Nc) pr.C[coff + (long long)n * pr.ldc + r] = acc[i][j][e];
+      }
+}
+
+cudaError_t launch_gemm_f64(std::vector<ProbF> probs, cudaStream_t s) {
+  probs.erase(std::remove_if(probs.begin(), probs.end(),
+                             [](const ProbF& p) { return p.nM <= 0 || p.Nc <= 0 || p.K <= 0; }),
+              probs.end());
+  if (probs.empty()) return cudaSuccess;
+  if (probs.size() > (size_t)kMaxProbF) return cudaErrorInvalidValue;
+  // longest contractions first
+  std::stable_sort(probs.begin(), probs.end(),
+                   [](const ProbF& a, const ProbF& b) { return a.K > b.K; });
+  ParamsF* P = new ParamsF();
+  P->nprob = (int)probs.size();
+  long long blocks = 0;
+  cudaError_t e = cudaSuccess;
+  for (int q = 0; q < P->nprob; q++) {
+    if (probs[q].K & 15) e = cudaErrorInvalidValue;
+    P->p[q] = probs[q];
+    P->p[q].first = (int)blocks;
+    blocks += (long long)probs[q].nM * ((probs[q].Nc + 31) / 32);
+    if (blocks > 0x7FFF0000ll) e = cudaErrorInvalidValue;
+  }
+  if (e == cudaSuccess) {
+    k_gemm_f64<<<(unsigned)blocks, 128, 0, s>>>(*P);
+    e = cudaGetLastError();
+  }
+  delete P;
+  return e;
 }
 
 static cudaError_t attributes() {

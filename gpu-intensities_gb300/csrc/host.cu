@@ -602,15 +602,16 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   const int N = c->N, Kp = c->Kp;
   const size_t ws_limit = c->budget ? c->budget / 2 : ((size_t)64 << 30);
   const size_t digit_bytes = (P.precision == GI_PREC_SPLIT) ? split_digit_bytes(c) : 0;
-  // the default split scheme: the order of the vibrational functions in its
-  // digits and in Z
+  // FP64 and the default split scheme: the order of the vibrational functions in
+  // Y (its digits) and in Z
   const bool s8 = P.precision == GI_PREC_SPLIT && split8_selected(c);
+  const bool fp = P.precision == GI_PREC_FP64;  // the same order, Y in FP64
+  const bool vib = s8 || fp;
   const VibPlan* vp = nullptr;
-  if (s8) {
-    gi_status s = split_prepare(c);
+  if (vib) {
+    gi_status s = s8 ? split_prepare(c) : GI_OK;
+    if (s == GI_OK) s = vib_prepare(c, &vp);
     if (s != GI_OK) return s;
-    vp = vib_plan(c, &s);
-    if (!vp) return s;
     std::lock_guard<std::mutex> lk(c->mmu());
     for (auto& kv : c->bases)
       if ((s = ensure_root_z(c, *kv.second, *vp)) != GI_OK) return s;
@@ -619,16 +620,16 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       if ((s = ensure_y_table(c, *c->bases[b.J], b.gamma)) != GI_OK) return s;
     }
   }
-  const int ldz = s8 ? vp->ldz : Kp;
+  const int ldz = vib ? vp->ldz : Kp;
   struct Unit {
     BlockPlan* I;
     std::vector<PairPlan*> pairs;
     int nI, ncolY;
     size_t off;   // into the record/level and energy tables
     size_t ycol;  // first Y/Z column of the unit within its round
-    size_t sc;    // default split scheme: into the slot column table
+    size_t sc;    // into the slot column table (FP64, default split scheme)
   };
-  // columns of one (unit, slot) in a band of the default split scheme's GEMM
+  // columns of one (unit, slot) in a band of the half-line-strength GEMM
   struct Group8 {
     size_t unit;
     int slot, rows;
@@ -640,15 +641,15 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     size_t ncolZ = 0;  // columns of Z (the bands padded to whole tiles)
     std::vector<Band8> bands;
     std::vector<std::vector<Group8>> groups8;  // per band
-    size_t bbytes = 0;                         // B digits
+    size_t bbytes = 0;                         // B digits, or Y in FP64
     double flops8 = 0.0;                       // digit products of the half-ls GEMM
   };
   std::vector<Round> rounds(1);
   std::vector<int32_t> h_ivec;  // per unit: nI record ids then nI level ids
   std::vector<double> h_EI;
   // bytes per Y column: Y, 3 Z, digit planes; plus the widest H/T per column
-  const size_t per_col = s8 ? (size_t)ldz * 24 + (size_t)vp->nk * 32 * digit_bytes
-                            : (size_t)Kp * (8 * 4 + digit_bytes);
+  const size_t per_col = vib ? (size_t)ldz * 24 + (size_t)vp->nk * 32 * (s8 ? digit_bytes : 8)
+                             : (size_t)Kp * (8 * 4 + digit_bytes);
   size_t round_bytes = 0;
   for (auto& kv : plans) {
     BlockPlan& I = kv.second;
@@ -688,7 +689,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   std::vector<int32_t> h_slotcol;
   for (Round& R : rounds) {
     R.ncolZ = R.ncolY;
-    if (!s8) continue;
+    if (!vib) continue;
     std::map<std::array<uint32_t, 4>, size_t> index;
     for (size_t k = 0; k < R.units.size(); k++) {
       Unit& u = R.units[k];
@@ -737,7 +738,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
         for (int q3 = 0; q3 < 3; q3++)
           if (band.rset[q3] >> k & 1) nf += n;
       }
-      R.bbytes += b_bytes8(band.ncol, band.nk);
+      R.bbytes += s8 ? b_bytes8(band.ncol, band.nk) : band.ncol * band.nk * 32 * sizeof(double);
       R.flops8 += (double)kDigits8 * (kDigits8 + 1) / 2 * 2.0 * nv * nf * (double)band.ncol;
       for (const Group8& g : R.groups8[q])
         h_slotcol[R.units[g.unit].sc + g.slot] = (int32_t)(band.col0 + g.col0);
@@ -752,9 +753,10 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     size_t hoff = 0, toff = 0;  // H and T of this block within its group's workspace
   };
   std::vector<std::vector<Target>> targets(rounds.size());
-  size_t max_y = 1, max_h = 1, max_t = 1;
+  size_t max_y = 1, max_h = 1, max_t = 1, max_yf = 1;
   for (size_t r = 0; r < rounds.size(); r++) {
     max_y = std::max(max_y, rounds[r].ncolZ * ldz);
+    max_yf = std::max(max_yf, rounds[r].bbytes / sizeof(double));
     std::map<BlockPlan*, size_t> idx;
     for (const Unit& u : rounds[r].units)
       for (PairPlan* pp : u.pairs) {
@@ -777,7 +779,8 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   GI_CUDA(c, c->w_ivec.assign(h_ivec));
   GI_CUDA(c, c->w_EI.assign(h_EI));
   DevArray<double>& d_EI = c->w_EI;
-  if (!s8) GI_CUDA(c, c->w_y.reserve(max_y));  // the default split scheme builds digits directly
+  // (the default split scheme builds digits directly)
+  if (!s8) GI_CUDA(c, c->w_y.reserve(fp ? max_yf : max_y));
   GI_CUDA(c, c->w_z.reserve(3 * max_y));
   c->stats = gi_stats{};
   c->timing = (flags & GI_RUN_PHASE_TIMING) != 0;
@@ -794,6 +797,10 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     grouped_final = split_grouped_final(c);
     fused_y = s8 || split_fused_y(c);
   }
+  const char* bs_env = getenv("GI_BATCH_SMALL");
+  const bool batch_small = !(bs_env && bs_env[0] == '0');
+  const bool fp_group = fp && batch_small;  // FP64: one launch per group of final blocks too
+  const bool grouped = grouped_final || fp_group;
   // the persistent final GEMM forms the lines itself (no T round trip, no
   // epilogue launches)
   const bool fused_epi = grouped_final && split_fused_epilogue(c);
@@ -817,10 +824,12 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       cols += T.ncolH;
       b8 += b_bytes8(T.ncolH, T.F->blk->ld / 32);
       cols8 += (T.ncolH + kCols8 - 1) / kCols8 * kCols8;
-      items += grouped_final ? split_grouped_items(c, T.F->blk->nvec, (int)T.ncolH) : 0;
-      const bool close = !grouped_final || t + 1 == targets[r].size() ||
+      items += grouped_final ? split_grouped_items(c, T.F->blk->nvec, (int)T.ncolH)
+               : fp_group    ? (T.F->blk->nvec + 31) / 32 * ((T.ncolH + 31) / 32)
+                             : 0;
+      const bool close = !grouped || t + 1 == targets[r].size() ||
                          items >= (size_t)16 * std::max(c->nsm, 1) ||
-                         (int)(t + 1 - t0) == split_grouped_max_jobs(c);
+                         (int)(t + 1 - t0) == (fp ? kMaxProbF : split_grouped_max_jobs(c));
       if (close) {
         groups[r].push_back({t0, t + 1});
         max_h = std::max(max_h, hs);
@@ -863,7 +872,8 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   // capacity bound would pin more than 16 GiB: then the copy follows the run)
   size_t nck = 0;
   for (size_t r = 0; r < rounds.size(); r++)
-    if (!rounds[r].units.empty()) nck += fused_epi ? groups[r].size() : targets[r].size();
+    if (!rounds[r].units.empty())
+      nck += fused_epi || fp_group ? groups[r].size() : targets[r].size();
   if (c->ck_cap < nck) {
     if (c->ck_count) cudaFreeHost(c->ck_count);
     c->ck_count = nullptr;
@@ -937,7 +947,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     mixv(grouped_final);
     mixv(fused_y);
     if (P.precision == GI_PREC_SPLIT) mixv(split_identity(c));
-    if (s8) mixv(vp->uid);
+    if (vib) mixv(vp->uid);
     for (size_t r = 0; r < rounds.size(); r++) {
       mixv(rounds[r].ncolY);
       for (const Unit& u : rounds[r].units) {
@@ -1085,7 +1095,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     }
     if (one && zblk && ztotal) {
       gi_status s = zcache_acquire(c, zblk, ids.data(), (int)ids.size(), 3 * ztotal * ldz,
-                                   s8 ? c->job.gF : -1, &zref);
+                                   vib ? c->job.gF : -1, &zref);
       if (s != GI_OK) return s;
     }
   }
@@ -1100,14 +1110,12 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   // one launch each per group (GI_BATCH_SMALL=0: one launch per item); the
   // lists are uploaded before any capture, at addresses the plan keeps
   struct GroupLists {
-    int h0 = 0, hn = 0, n0 = 0, nn = 0;
-    long long hblocks = 0, ncols = 0;
+    int h0 = 0, hn = 0, n0 = 0, nn = 0, e0 = 0, en = 0;
+    long long hblocks = 0, ncols = 0, eblocks = 0;
   };
   std::vector<std::vector<GroupLists>> glists(rounds.size());
   std::vector<std::pair<int, int>> ylists(rounds.size(), {0, 0});  // Y digit items per round
-  const char* bs_env = getenv("GI_BATCH_SMALL");
-  const bool batch_small = !(bs_env && bs_env[0] == '0');
-  // The default split scheme's tables: slot columns, and per band its K slices,
+  // The tables of the bands: slot columns, and per band its K slices,
   // its row tiles (for every panel of the dipole) and its column groups of Y
   struct Y8Range {
     size_t item0 = 0, n = 0, tile0 = 0;
@@ -1115,7 +1123,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   };
   std::vector<Y8Range> y8(rounds.size());
   std::vector<YItem8> h_y8;
-  if (s8) {
+  if (vib) {
     std::vector<uint16_t> h_kl;
     std::vector<int32_t> h_vl, h_ytile;
     std::vector<ATile> h_at;
@@ -1147,6 +1155,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       for (size_t q = 0; q < R.bands.size(); q++) {
         Band8& band = R.bands[q];
         band.kl = c->w_kl8.p + ksets[band.kset].first;
+        band.vl = c->w_vl8.p + ksets[band.kset].second;
         for (const auto& tiles : ptiles) {
           at0[r][q].push_back(h_at.size());
           int n = 0;
@@ -1175,8 +1184,8 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
           y.ys = bI.d_ys[b.gamma].p + (size_t)g.slot * N;
           y.yc = bI.d_yc[b.gamma].p + (size_t)g.slot * N;
           y.vlist = c->w_vl8.p + ksets[R.bands[q].kset].second;
-          y.out = split8_b(c) + R.bands[q].boff;
-          y.e_out = split8_b_exp(c) + R.bands[q].col0;
+          y.out = (s8 ? split8_b(c) : reinterpret_cast<uint8_t*>(c->w_y.p)) + R.bands[q].boff;
+          y.e_out = s8 ? split8_b_exp(c) + R.bands[q].col0 : nullptr;
           y.ld = b.ld;
           y.ndeg = c->degen[b.gamma];
           y.nk = R.bands[q].nk;
@@ -1203,6 +1212,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     std::vector<HItem> hitems;
     std::vector<NormItem> nitems;
     std::vector<YItem> yitems;
+    std::vector<EpiItem> eitems;
     for (size_t r = 0; r < rounds.size(); r++) {
       const Round& R = rounds[r];
       if (fused_y && !s8 && !zref.hit) {  // the round's Y rows, unit by unit
@@ -1244,11 +1254,11 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
             const Unit& u = *T.parts[k].first;
             const PairPlan* pp = T.parts[k].second;
             HItem it = make_h_item(
-                zbase + (s8 ? 0 : u.ycol * Kp), zc, ldz, c->bases[u.I->blk->J]->nslot,
+                zbase + (vib ? 0 : u.ycol * Kp), zc, ldz, c->bases[u.I->blk->J]->nslot,
                 c->degen[u.I->blk->gamma], u.nI, bF, fb.gamma, c->degen[fb.gamma], fb.nsize,
                 fb.ld, c->w_stencil.p + pp->st_off * 6, c->w_stencil_n.p + pp->st_off, 6,
                 c->w_h.p + T.hoff + T.hcol[k] * fb.ld, gl.hblocks);
-            if (s8) {
+            if (vib) {
               it.root_v = bF.d_root_z.p;
               it.slotcol = c->w_slotcol.p + u.sc;
             }
@@ -1268,6 +1278,34 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
           gl.ncols += (long long)T.ncolH;
         }
         gl.nn = (int)nitems.size() - gl.n0;
+        gl.e0 = (int)eitems.size();
+        size_t hn_off = 0;
+        for (size_t t = grp.first; t < grp.second && fp_group; t++) {
+          const Target& T = targets[r][t];
+          const Block& fb = *T.F->blk;
+          const auto off = farr[T.F];
+          for (size_t k = 0; k < T.parts.size(); k++) {
+            const Unit& u = *T.parts[k].first;
+            if (u.nI == 0 || fb.nvec == 0) continue;
+            EpiItem e{};
+            e.ldt = round_up(fb.nvec, 2);
+            e.T = c->w_t.p + T.toff + T.hcol[k] * e.ldt;
+            e.EI = c->w_EI.p + u.off;
+            e.EF = fb.d_energies.p;
+            e.hn = c->w_hn.p + hn_off + T.hcol[k];
+            e.lvI = c->w_ivec.p + 2 * u.off + u.nI;
+            e.lvF = c->w_int.p + off.first;
+            e.upper = c->w_upper.p + off.second;
+            e.nI = u.nI;
+            e.nF = fb.nvec;
+            e.ep = rparts[part_of[r][t][k]].ep;
+            e.blk0 = gl.eblocks;
+            gl.eblocks += (long long)u.nI * ((fb.nvec + 127) / 128);
+            eitems.push_back(e);
+          }
+          hn_off += T.ncolH;
+        }
+        gl.en = (int)eitems.size() - gl.e0;
         glists[r].push_back(gl);
       }
     }
@@ -1278,6 +1316,8 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     mixv(c->w_hfirst.p);
     GI_CUDA(c, c->w_nitems.assign(nitems));
     GI_CUDA(c, c->w_yitems.assign(yitems));
+    GI_CUDA(c, c->w_epiitems.assign(eitems));
+    mixv(c->w_epiitems.p);
     mixv(c->w_hitems.p);
     mixv(c->w_nitems.p);
     mixv(c->w_yitems.p);
@@ -1298,14 +1338,14 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     // Z of this round: the workspace, or its columns of the cache entry
     double* zbase = zref.z ? zref.z + zoff[r] * ldz : c->w_z.p;
     const size_t zc = (zref.z ? ztotal : R.ncolZ) * ldz;  // stride between dipole components
-    if (s8 && !zref.hit) {  // every unit's columns in one launch, or one launch per column group
+    if (vib && !zref.hit) {  // every unit's columns in one launch, or one launch per column group
       const YItem8* it = c->w_yitems8.p + y8[r].item0;
       gi_status s = GI_OK;
       if (batch_small) {
-        s = split8_build_y(c, it, c->w_ytile8.p + y8[r].tile0, (int)y8[r].n, y8[r].blocks);
+        s = split8_build_y(c, it, c->w_ytile8.p + y8[r].tile0, (int)y8[r].n, y8[r].blocks, s8);
       } else {
         for (size_t k = 0; k < y8[r].n && s == GI_OK; k++)
-          s = split8_build_y(c, it + k, nullptr, 1, h_y8[y8[r].item0 + k].rows);
+          s = split8_build_y(c, it + k, nullptr, 1, h_y8[y8[r].item0 + k].rows, s8);
       }
       if (s != GI_OK) return s;
     }
@@ -1318,7 +1358,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       if (zref.hit) break;  // Z of this round is in the cache
       const Basis& bI = *c->bases[u.I->blk->J];
       const int ndegI = c->degen[u.I->blk->gamma];
-      if (s8 || (fused_y && batch_small)) {
+      if (vib || (fused_y && batch_small)) {
         // built above
       } else if (fused_y) {  // straight into the digit planes of the half-ls GEMM's B operand
         gi_status s = split_build_y_digits(c, u.I->blk->d_vecs.p, u.I->blk->ld,
@@ -1347,7 +1387,29 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       if (s != GI_OK) return s;
       fl_half += 2.0 * 3.0 * N * (double)N * R.ncolY;
     } else {
-      gi_status s = dipole_gemm_fp64(c, c->w_y.p, Kp, zbase, Kp, zc, (int)R.ncolY, c->stream);
+      int panel = 0;
+      gi_status s = for_each_dipole_panel(c, c->stream, [&](const double* mu, size_t, int, int)
+                                                            -> gi_status {
+        std::vector<ProbF> probs;
+        for (const Band8& b : R.bands) {
+          ProbF p{};
+          p.A = mu;
+          p.lda = Kp;
+          p.B = c->w_y.p + b.boff / sizeof(double);
+          p.C = zbase + b.col0 * (size_t)ldz;
+          p.ldc = ldz;
+          p.at = b.at[panel];
+          p.rowsrc = vib_rowsrc(c, panel);
+          p.vl = b.vl;
+          p.ldb = p.K = b.nk * 32;
+          p.nM = 4 * b.nA[panel];
+          p.Nc = (int)b.ncol;
+          probs.push_back(p);
+        }
+        panel++;
+        GI_CUDA(c, timed(c, GI_PHASE_HALFLS_GEMM, [&] { return launch_gemm_f64(probs, c->stream); }));
+        return GI_OK;
+      });
       if (s != GI_OK) return s;
       fl_half += 2.0 * 3.0 * N * (double)N * R.ncolY;
     }
@@ -1375,13 +1437,13 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
           const int ndegI = c->degen[u.I->blk->gamma];
           const int nslot = c->bases[u.I->blk->J]->nslot;
           GI_CUDA(c, timed(c, GI_PHASE_STENCIL, [&] {
-                    return launch_build_h(zbase + (s8 ? 0 : u.ycol * Kp), zc, ldz, nslot, ndegI,
+                    return launch_build_h(zbase + (vib ? 0 : u.ycol * Kp), zc, ldz, nslot, ndegI,
                                           u.nI, bF, fb.gamma, ndegF, fb.nsize, ldh,
                                           c->w_stencil.p + pp->st_off * 6,
                                           c->w_stencil_n.p + pp->st_off, 6,
                                           c->w_h.p + T.hoff + T.hcol[k] * ldh, c->stream,
-                                          s8 ? bF.d_root_z.p : nullptr,
-                                          s8 ? c->w_slotcol.p + u.sc : nullptr);
+                                          vib ? bF.d_root_z.p : nullptr,
+                                          vib ? c->w_slotcol.p + u.sc : nullptr);
                   }));
         }
       }
@@ -1429,23 +1491,41 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
                             rec_cap};
         gi_status s = split_gemm_final_grouped(c, jobs, fused_epi ? &fl : nullptr);
         if (s != GI_OK) return s;
+      } else if (fp) {
+        std::vector<ProbF> probs;
+        for (size_t t = grp.first; t < grp.second; t++) {
+          const Target& T = targets[r][t];
+          const Block& fb = *T.F->blk;
+          ProbF p{};
+          p.A = fb.d_vecs.p;
+          p.lda = fb.ld;
+          p.B = c->w_h.p + T.hoff;
+          p.C = c->w_t.p + T.toff;
+          p.ldc = round_up(fb.nvec, 2);
+          p.ldb = p.K = fb.ld;
+          p.M = fb.nvec;
+          p.nM = (fb.nvec + 31) / 32;
+          p.Nc = (int)T.ncolH;
+          probs.push_back(p);
+        }
+        GI_CUDA(c, timed(c, GI_PHASE_FINAL_GEMM, [&] { return launch_gemm_f64(probs, c->stream); }));
       } else {
         for (size_t t = grp.first; t < grp.second; t++) {
           const Target& T = targets[r][t];
           const Block& fb = *T.F->blk;
-          const int ldh = fb.ld, ldt = round_up(fb.nvec, 2);
-          double* H = c->w_h.p + T.hoff;
-          double* Tm = c->w_t.p + T.toff;
-          if (P.precision == GI_PREC_SPLIT) {
-            gi_status s = split_gemm_final(c, *T.F->blk, H, ldh, (int)T.ncolH, Tm, ldt);
-            if (s != GI_OK) return s;
-          } else {
-            GI_CUDA(c, timed(c, GI_PHASE_FINAL_GEMM, [&] {
-                      return gemm_fp64_nt(fb.d_vecs.p, fb.ld, 0, H, ldh, Tm, ldt, 0, fb.nvec,
-                                          (int)T.ncolH, ldh, 1, c->stream);
-                    }));
-          }
+          gi_status s = split_gemm_final(c, *T.F->blk, c->w_h.p + T.hoff, fb.ld, (int)T.ncolH,
+                                         c->w_t.p + T.toff, round_up(fb.nvec, 2));
+          if (s != GI_OK) return s;
         }
+      }
+      if (fp_group) {
+        const GroupLists& gl = glists[r][gi];
+        GI_CUDA(c, timed(c, GI_PHASE_EPILOGUE, [&] {
+                  return launch_epilogue_items(c->w_epiitems.p + gl.e0, gl.en, gl.eblocks,
+                                               c->d_lines.p, c->w_counter.p,
+                                               (long long)c->d_lines.n, c->w_rec.p, rec_cap,
+                                               c->stream);
+                }));
       }
       // epilogues, and a line-count checkpoint after each block's
       for (size_t t = grp.first; t < grp.second; t++) {
@@ -1458,7 +1538,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
         for (size_t k = 0; k < T.parts.size(); k++) {
           const Unit& u = *T.parts[k].first;
           npairs_checked += (int64_t)u.nI * Fp.nupper;
-          if (fused_epi) continue;  // formed by the final GEMM's epilogue warps
+          if (fused_epi || fp_group) continue;  // formed by the final GEMM's epilogue warps, or above
           const EpiParams ep = rparts[part_of[r][t][k]].ep;
           const int32_t* d_lvI = c->w_ivec.p + 2 * u.off + u.nI;
           const double* hn = c->w_hn.p + hn_at[t - grp.first] + T.hcol[k];
@@ -1471,7 +1551,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
                                            rec_cap, c->stream);
                   }));
         }
-        if (fused_epi && t + 1 < grp.second) continue;  // one checkpoint per group
+        if ((fused_epi || fp_group) && t + 1 < grp.second) continue;  // one checkpoint per group
         // checkpoint: every line of this final block is written once this fires
         GI_CUDA(c, cudaMemcpyAsync(c->ck_count + ck, c->w_counter.p, sizeof(unsigned long long),
                                    cudaMemcpyDeviceToHost, c->stream));

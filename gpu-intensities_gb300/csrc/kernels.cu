@@ -1,5 +1,5 @@
-// Gather/scatter, stencil, epilogue and FP64 DMMA GEMM kernels of the
-// line-intensity engine (sm_103a).
+// Gather/scatter, stencil, epilogue and line order kernels of the line-intensity
+// engine (sm_103a).
 //
 // Factorisation of the reference's half line strength
 // (dipole_kernals.cu:162-227).  With keyI = 2kI+tauI, the reference sums
@@ -380,15 +380,14 @@ cudaError_t launch_half_ls_prim_parts(const double* Zp, int nparts, size_t pstri
 // ------------------------------------------------------------------ epilogue
 // One thread per (initial level i, final level f) of a part: the per-line
 // epilogue of epilogue.cuh on the moments of T.
-__global__ void k_epilogue(const double* __restrict__ T, int ldt, int nI, int nF,
-                           const int32_t* __restrict__ levelI, const double* __restrict__ EI,
-                           const int32_t* __restrict__ levelF, const double* __restrict__ EF,
-                           const uint8_t* __restrict__ upper_ok,
-                           const double* __restrict__ hn, EpiParams p,
-                           gi_line* __restrict__ out, unsigned long long* counter,
-                           long long cap, RefineRec* __restrict__ rec, long long rec_cap) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
+__device__ __forceinline__ void epilogue_block(
+    int fb, int i, const double* __restrict__ T, int ldt, int nF,
+    const int32_t* __restrict__ levelI, const double* __restrict__ EI,
+    const int32_t* __restrict__ levelF, const double* __restrict__ EF,
+    const uint8_t* __restrict__ upper_ok, const double* __restrict__ hn, const EpiParams& p,
+    gi_line* __restrict__ out, unsigned long long* counter, long long cap,
+    RefineRec* __restrict__ rec, long long rec_cap) {
+  const int f = fb * 128 + threadIdx.x;
   // the initial level's Boltzmann factor, once per block (FP64 exp is scarce)
   __shared__ double boltz_i;
   if (threadIdx.x == 0) boltz_i = exp(-(EI[i] - p.zpe) * p.beta);
@@ -407,6 +406,36 @@ __global__ void k_epilogue(const double* __restrict__ T, int ldt, int nI, int nF
   eval_line(p, t, hnq, EI[i], ok_f ? EF[f] : 0.0, boltz_i, ok_f, levelI[i],
             ok_f ? levelF[f] : -1, r);
   append_line(r, p.part, i, f, out, counter, cap, rec, rec_cap);
+}
+
+__global__ void __launch_bounds__(128)
+    k_epilogue(const double* __restrict__ T, int ldt, int nF, const int32_t* __restrict__ levelI,
+               const double* __restrict__ EI, const int32_t* __restrict__ levelF,
+               const double* __restrict__ EF, const uint8_t* __restrict__ upper_ok,
+               const double* __restrict__ hn, EpiParams p, gi_line* __restrict__ out,
+               unsigned long long* counter, long long cap, RefineRec* __restrict__ rec,
+               long long rec_cap) {
+  epilogue_block(blockIdx.x, blockIdx.y, T, ldt, nF, levelI, EI, levelF, EF, upper_ok, hn, p, out,
+                 counter, cap, rec, rec_cap);
+}
+// Every part of a group of final blocks in one launch.
+__global__ void __launch_bounds__(128)
+    k_epilogue_items(const EpiItem* __restrict__ items, int nitems, gi_line* __restrict__ out,
+                     unsigned long long* counter, long long cap, RefineRec* __restrict__ rec,
+                     long long rec_cap) {
+  const long long b = blockIdx.x;
+  const EpiItem& it = items[find_item(nitems, b, [&](int k) { return items[k].blk0; })];
+  const int nfb = (it.nF + 127) >> 7, rel = (int)(b - it.blk0);
+  epilogue_block(rel % nfb, rel / nfb, it.T, it.ldt, it.nF, it.lvI, it.EI, it.lvF, it.EF, it.upper,
+                 it.hn, it.ep, out, counter, cap, rec, rec_cap);
+}
+cudaError_t launch_epilogue_items(const EpiItem* items, int nitems, long long blocks, gi_line* out,
+                                  unsigned long long* counter, long long cap, RefineRec* rec,
+                                  long long rec_cap, cudaStream_t s) {
+  if (nitems <= 0 || blocks <= 0) return cudaSuccess;
+  if (blocks > 0x7FFFFFFFll) return cudaErrorInvalidValue;
+  k_epilogue_items<<<(unsigned)blocks, 128, 0, s>>>(items, nitems, out, counter, cap, rec, rec_cap);
+  return cudaGetLastError();
 }
 
 __global__ void k_boltz(const double* __restrict__ E, int n, double zpe, double beta,
@@ -629,111 +658,8 @@ cudaError_t launch_epilogue(const double* T, int ldt, int nI, int nF, const int3
                             RefineRec* rec, long long rec_cap, cudaStream_t s) {
   if (nI == 0 || nF == 0) return cudaSuccess;
   dim3 grid((nF + 127) / 128, nI);
-  k_epilogue<<<grid, 128, 0, s>>>(T, ldt, nI, nF, levelI, EI, levelF, EF, upper_ok, hn, p, out,
-                                  counter, cap, rec, rec_cap);
-  return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------ FP64 GEMM
-// C[z][n*ldc + m] = sum_k A[z][m*lda + k] * B[n*ldb + k] on the FP64 tensor
-// pipe (mma.sync m8n8k4 .f64).  64x64 tile, 4 warps of 32x32, K step 16,
-// cp.async double buffering.  K is a multiple of 16 and lda/ldb are even
-// (the engine pads every K dimension), so each 16-byte copy is aligned.
-namespace {
-constexpr int GBM = 64, GBN = 64, GBK = 16, GPAD = 2;
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  const int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(n));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-}  // namespace
-
-__global__ void __launch_bounds__(128)
-    k_gemm_fp64_nt(const double* __restrict__ A, int lda, size_t strideA,
-                   const double* __restrict__ B, int ldb, double* __restrict__ C, int ldc,
-                   size_t strideC, int M, int Nc, int K) {
-  __shared__ __align__(16) double As[2][GBM][GBK + GPAD];
-  __shared__ __align__(16) double Bs[2][GBN][GBK + GPAD];
-  A += (size_t)blockIdx.z * strideA;
-  C += (size_t)blockIdx.z * strideC;
-  const int m0 = blockIdx.y * GBM, n0 = blockIdx.x * GBN;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-  const int g = lane >> 2, tq = lane & 3;
-
-  double acc[4][4][2];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-
-  auto load = [&](int st, int k0) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int q = tid + 128 * j;
-      const int row = q >> 3, cp = (q & 7) * 2;
-      const int am = m0 + row, bn = n0 + row;
-      const bool va = am < M, vb = bn < Nc;
-      cp_async16(&As[st][row][cp], A + (size_t)(va ? am : 0) * lda + k0 + cp, va);
-      cp_async16(&Bs[st][row][cp], B + (size_t)(vb ? bn : 0) * ldb + k0 + cp, vb);
-    }
-    cp_async_commit();
-  };
-
-  const int nk = K / GBK;
-  load(0, 0);
-  for (int kt = 0; kt < nk; ++kt) {
-    const int st = kt & 1;
-    if (kt + 1 < nk) {
-      load(st ^ 1, (kt + 1) * GBK);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < GBK; kk += 4) {
-      double af[4], bf[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) af[a] = As[st][wm + a * 8 + g][kk + tq];
-#pragma unroll
-      for (int b = 0; b < 4; ++b) bf[b] = Bs[st][wn + b * 8 + g][kk + tq];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          asm volatile(
-              "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-              : "+d"(acc[a][b][0]), "+d"(acc[a][b][1])
-              : "d"(af[a]), "d"(bf[b]));
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int m = m0 + wm + a * 8 + g;
-        const int n = n0 + wn + b * 8 + tq * 2 + e;
-        if (m < M && n < Nc) C[(size_t)n * ldc + m] = acc[a][b][e];
-      }
-}
-
-cudaError_t gemm_fp64_nt(const double* A, int lda, size_t strideA, const double* B, int ldb,
-                         double* C, int ldc, size_t strideC, int M, int Nc, int K, int batch,
-                         cudaStream_t s) {
-  if (M <= 0 || Nc <= 0 || batch <= 0) return cudaSuccess;
-  if (K <= 0 || K % GBK != 0 || (lda & 1) || (ldb & 1)) return cudaErrorInvalidValue;
-  dim3 grid((Nc + GBN - 1) / GBN, (M + GBM - 1) / GBM, batch);
-  k_gemm_fp64_nt<<<grid, 128, 0, s>>>(A, lda, strideA, B, ldb, C, ldc, strideC, M, Nc, K);
+  k_epilogue<<<grid, 128, 0, s>>>(T, ldt, nF, levelI, EI, levelF, EF, upper_ok, hn, p, out, counter,
+                                  cap, rec, rec_cap);
   return cudaGetLastError();
 }
 

@@ -23,7 +23,7 @@
 #include <unordered_map>
 
 #include "engine.h"
-#include "split.h"
+#include "split8.h"
 
 namespace gi {
 
@@ -445,7 +445,13 @@ gi_status gi_serve_start(gi_ctx* h, const gi_serve_config* cfg) {
   if ((size_t)slots * slot_ws >= budget)
     return fail(c, GI_ERR_ARG, "slot workspaces (%d x %zu bytes) leave no room for blocks", slots,
                 slot_ws);
-  // the dipole digits are cut once, before any worker runs
+  // the order of the vibrational functions and the dipole digits are made once,
+  // before any worker runs
+  {
+    const VibPlan* vp;
+    gi_status st = vib_prepare(c, &vp);
+    if (st != GI_OK) return st;
+  }
   if (c->params.precision == GI_PREC_SPLIT) {
     gi_status st = split_prepare(c);
     if (st != GI_OK) return st;

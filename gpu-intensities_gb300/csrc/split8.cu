@@ -548,6 +548,7 @@ __global__ void __launch_bounds__(256) k_cut8_b(const __grid_constant__ CutOps8 
 // transform of the roots of that (slot, function) (k_build_y's arithmetic, from
 // the basis's table), held in shared memory between the exponent and the cut
 // (recomputed when the row does not fit).
+template <bool DIGITS>
 __global__ void __launch_bounds__(256) k_build_y8(const YItem8* __restrict__ items,
                                                   const int32_t* __restrict__ tile_item, int n,
                                                   int cached) {
@@ -580,6 +581,16 @@ __global__ void __launch_bounds__(256) k_build_y8(const YItem8* __restrict__ ite
         if (c[q4] != 0.0) x[q4] = fma(vs[s[q4]], c[q4], x[q4]);
     }
   };
+  if constexpr (!DIGITS) {
+    double* y = reinterpret_cast<double*>(it.out) + (size_t)(it.col0 + j) * K;
+    for (int k = threadIdx.x * 4; k < K; k += 1024) {
+      double x[4];
+      values(k, x);
+      *reinterpret_cast<double2*>(y + k) = make_double2(x[0], x[1]);
+      *reinterpret_cast<double2*>(y + k + 2) = make_double2(x[2], x[3]);
+    }
+    return;
+  }
   unsigned long long mx = 0;
   for (int k = threadIdx.x * 4; k < K; k += 1024) {
     double x[4];
@@ -616,7 +627,7 @@ cudaError_t attributes8() {
     status = cudaFuncSetAttribute(k_split8, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)kSmem);
     if (status == cudaSuccess)
-      status = cudaFuncSetAttribute(k_build_y8, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      status = cudaFuncSetAttribute(k_build_y8<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     kYSmem);
   });
   return status;
@@ -628,14 +639,18 @@ cudaError_t attributes8() {
 struct Split8 {
   bool on = false;
   std::unique_ptr<VibPlan> plan;    // (null in a serving worker)
-  // the dipole's digits: made for `mu_uid`'s order of functions
-  uint64_t mu_uid = 0;
-  bool mu_valid = false;
+  // device tables of the plan `order_uid` for panels of `panel` rows: rowsrc, vk
+  // and zpos in one allocation
+  uint64_t order_uid = 0;
   int panel = 0;
-  DevArray<uint8_t> mu;
-  DevArray<int32_t> mu_exp, tables;  // tables: rowsrc, vk and zpos in one allocation
+  DevArray<int32_t> tables;
   const int32_t *rowsrc = nullptr, *vk = nullptr, *zpos = nullptr;
   std::vector<size_t> panel_tile;   // first row-source tile of each panel, and the end
+  size_t most_tiles = 0;            // of a panel
+  // the dipole's digits in that order
+  bool mu_valid = false;
+  DevArray<uint8_t> mu;
+  DevArray<int32_t> mu_exp;
   DevArray<uint8_t> b;              // B operand workspace
   DevArray<int32_t> b_exp;
   DevArray<int> ctr, err;
@@ -799,12 +814,57 @@ static cudaError_t cut_dipole(Ctx* c, Split8* S, const VibPlan& vp, const double
   return cudaGetLastError();
 }
 
+gi_status vib_prepare(Ctx* c, const VibPlan** out) {
+  gi_status g;
+  const VibPlan* vp = vib_plan(c, &g);
+  *out = vp;
+  if (!vp) return g;
+  if (c->parent) {
+    const Split8* P = c->parent->split8;
+    if (!P || P->order_uid != vp->uid)
+      return fail(c, GI_ERR_STATE, "the serving context's dipole order is not prepared");
+    return GI_OK;
+  }
+  Split8* S = st8(c);
+  const int P = dipole_panel_rows(c);  // 0: the dipole is resident
+  if (S->order_uid == vp->uid && S->panel == P) return GI_OK;
+  S->order_uid = 0;
+  S->mu_valid = false;
+  const int N = c->N, step = P ? P : N;
+  std::vector<int32_t> src;
+  S->panel_tile.assign(1, 0);
+  S->most_tiles = 0;
+  for (int f0 = 0; f0 < N; f0 += step) {
+    const auto tiles = split8_tiles(*vp, f0, std::min(step, N - f0));
+    for (const VibTile& t : tiles)
+      for (int r = 0; r < kBM; r++)
+        src.push_back(r < t.rows ? t.comp * step + vp->members[t.cls][t.i0 + r] - f0 : -1);
+    S->panel_tile.push_back(S->panel_tile.back() + tiles.size());
+    S->most_tiles = std::max(S->most_tiles, tiles.size());
+  }
+  const size_t nsrc = src.size(), nvk = vp->vk.size();
+  src.insert(src.end(), vp->vk.begin(), vp->vk.end());
+  src.insert(src.end(), vp->zpos.begin(), vp->zpos.end());
+  if ((g = check8(c, S->tables.assign(src), "dipole order")) != GI_OK) return g;
+  S->rowsrc = S->tables.p;
+  S->vk = S->rowsrc + nsrc;
+  S->zpos = S->vk + nvk;
+  S->panel = P;
+  S->order_uid = vp->uid;
+  return GI_OK;
+}
+
+const int32_t* vib_rowsrc(const Ctx* c, int panel) {
+  const Split8* S = (c->parent ? c->parent : c)->split8;
+  return S->rowsrc + S->panel_tile[panel] * kBM;
+}
+
 gi_status split8_prepare(Ctx* c) {
   Split8* S = st8(c);
   S->on = true;
-  gi_status g;
-  const VibPlan* vp = vib_plan(c, &g);
-  if (!vp) return g;
+  const VibPlan* vp;
+  gi_status g = vib_prepare(c, &vp);
+  if (g != GI_OK) return g;
   if (!S->err.p) {
     if ((g = check8(c, S->err.reserve(1), "error word")) != GI_OK) return g;
     if ((g = check8(c, S->ctr.reserve(2), "work counter")) != GI_OK) return g;
@@ -821,38 +881,16 @@ gi_status split8_prepare(Ctx* c) {
   if ((g = check8(c, attributes8(), "kernel attributes")) != GI_OK) return g;
   if (c->parent) {
     const Split8* P = c->parent->split8;
-    if (!P || !P->mu_valid || P->mu_uid != vp->uid)
+    if (!P->mu_valid)
       return fail(c, GI_ERR_STATE,
                   "split precision: the dipole digits of the serving context are not prepared");
     return GI_OK;
   }
-  const int P = dipole_panel_rows(c);  // 0: the dipole is resident
-  if (S->mu_valid && S->mu_uid == vp->uid && S->panel == P) return GI_OK;
-  S->mu_valid = false;
-  const int N = c->N, step = P ? P : N;
-  std::vector<int32_t> src;
-  S->panel_tile.assign(1, 0);
-  size_t most = 0;
-  for (int f0 = 0; f0 < N; f0 += step) {
-    const auto tiles = split8_tiles(*vp, f0, std::min(step, N - f0));
-    for (const VibTile& t : tiles)
-      for (int r = 0; r < kBM; r++)
-        src.push_back(r < t.rows ? t.comp * step + vp->members[t.cls][t.i0 + r] - f0 : -1);
-    S->panel_tile.push_back(S->panel_tile.back() + tiles.size());
-    most = std::max(most, tiles.size());
-  }
-  const size_t nsrc = src.size(), nvk = vp->vk.size();
-  src.insert(src.end(), vp->vk.begin(), vp->vk.end());
-  src.insert(src.end(), vp->zpos.begin(), vp->zpos.end());
-  if ((g = check8(c, S->tables.assign(src), "dipole order")) != GI_OK) return g;
-  S->rowsrc = S->tables.p;
-  S->vk = S->rowsrc + nsrc;
-  S->zpos = S->vk + nvk;
-  if ((g = check8(c, S->mu.reserve(a_bytes8(most, vp->nk)), "dipole digits")) != GI_OK) return g;
-  if ((g = check8(c, S->mu_exp.reserve(most * kBM), "dipole exponents")) != GI_OK) return g;
-  S->panel = P;
-  S->mu_uid = vp->uid;
-  if (!P) {
+  if (S->mu_valid) return GI_OK;
+  if ((g = check8(c, S->mu.reserve(a_bytes8(S->most_tiles, vp->nk)), "dipole digits")) != GI_OK)
+    return g;
+  if ((g = check8(c, S->mu_exp.reserve(S->most_tiles * kBM), "dipole exponents")) != GI_OK) return g;
+  if (!S->panel) {
     if ((g = check8(c, cut_dipole(c, S, *vp, c->d_mu.p, 0), "dipole digits")) != GI_OK) return g;
     if ((g = check8(c, cudaStreamSynchronize(c->stream), "dipole digits")) != GI_OK) return g;
   }
@@ -933,7 +971,7 @@ uint8_t* split8_b(Ctx* c) { return st8(c)->b.p; }
 int32_t* split8_b_exp(Ctx* c) { return st8(c)->b_exp.p; }
 
 gi_status split8_build_y(Ctx* c, const YItem8* items, const int32_t* tile_item, int n,
-                         long long blocks) {
+                         long long blocks, bool digits) {
   if (n <= 0 || blocks <= 0) return GI_OK;
   if (blocks > 0x7FFFFFFFll) return check8(c, cudaErrorInvalidValue, "Y digits");
   gi_status g;
@@ -942,8 +980,12 @@ gi_status split8_build_y(Ctx* c, const YItem8* items, const int32_t* tile_item, 
   const size_t row = (size_t)vp->nk * 32 * sizeof(double);
   const int cached = row <= (size_t)kYSmem;
   return check8(c, timed(c, GI_PHASE_CORRELATE, [&] {
-                  k_build_y8<<<(unsigned)blocks, 256, cached ? row : 0, c->stream>>>(
-                      items, tile_item, n, cached);
+                  if (digits)
+                    k_build_y8<true><<<(unsigned)blocks, 256, cached ? row : 0, c->stream>>>(
+                        items, tile_item, n, cached);
+                  else
+                    k_build_y8<false><<<(unsigned)blocks, 256, 0, c->stream>>>(items, tile_item, n,
+                                                                              0);
                   return cudaGetLastError();
                 }),
                 "Y digits");
@@ -1113,7 +1155,7 @@ uint64_t split8_identity(Ctx* c) {
   uint64_t h = 14695981039346656037ull;
   for (uint64_t v : {(uint64_t)(uintptr_t)S->b.p, (uint64_t)(uintptr_t)S->b_exp.p,
                      (uint64_t)(uintptr_t)S->ctr.p, (uint64_t)(uintptr_t)S->err.p,
-                     (uint64_t)(uintptr_t)D->mu.p, (uint64_t)(uintptr_t)D->mu_exp.p, D->mu_uid,
+                     (uint64_t)(uintptr_t)D->mu.p, (uint64_t)(uintptr_t)D->mu_exp.p, D->order_uid,
                      split_tuner_version()})
     h = (h ^ v) * 1099511628211ull;
   return h;

@@ -65,6 +65,10 @@ bool split8_active(const Ctx* c);  // after split_prepare: the run uses it
 // (a serving worker: its parent's).  Null with *st set on failure.
 const VibPlan* vib_plan(Ctx* c, gi_status* st);
 gi_status split8_prepare(Ctx* c);
+// The plan and the device tables of its order (both precisions); a worker uses
+// its parent's.  panel's first row of the row-source table.
+gi_status vib_prepare(Ctx* c, const VibPlan** vp);
+const int32_t* vib_rowsrc(const Ctx* c, int panel);
 // Row tiles of the dipole (or of panel p of a streamed one), in stored order.
 std::vector<VibTile> split8_tiles(const VibPlan& vp, int f0, int rows);
 // B workspace bytes and columns of the largest launch; final blocks' digits.
@@ -75,8 +79,9 @@ uint8_t* split8_b(Ctx* c);
 int32_t* split8_b_exp(Ctx* c);
 // The digits of n column groups; tile_item[b / 64]: the first group of blocks
 // b..b+63 (null: one group, whose first block is the launch's).
+// (digits false: as doubles, out being double[column][32 nk] of the band.)
 gi_status split8_build_y(Ctx* c, const YItem8* items, const int32_t* tile_item, int n,
-                         long long blocks);
+                         long long blocks, bool digits = true);
 // Rows of Z of a basis's roots for the plan (after split_prepare, under the model lock).
 gi_status ensure_root_z(Ctx* c, Basis& b, const VibPlan& vp);
 // Classes a (basis, gamma, slot) has coefficients on; rows of Z that final
@@ -92,6 +97,7 @@ struct Band8 {
   size_t boff = 0;                         // bytes into the B workspace
   int nk = 0;
   const uint16_t* kl = nullptr;            // device list of A slices
+  const int32_t* vl = nullptr;             // and of the functions at their positions
   std::vector<const ATile*> at;            // device row tiles, per panel
   std::vector<int> nA;
 };

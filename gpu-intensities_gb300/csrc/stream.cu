@@ -142,17 +142,6 @@ gi_status for_each_dipole_panel(Ctx* c, cudaStream_t st, const PanelFn& fn) {
   return s;
 }
 
-gi_status dipole_gemm_fp64(Ctx* c, const double* Y, int ldy, double* Z, int ldz, size_t zc,
-                           int ncol, cudaStream_t st) {
-  return for_each_dipole_panel(c, st, [&](const double* mu, size_t mstride, int rows, int f0) {
-    GI_CUDA(c, timed(c, GI_PHASE_HALFLS_GEMM, [&] {
-              return gemm_fp64_nt(mu, c->Kp, mstride, Y, ldy, Z + f0, ldz, zc, rows, ncol, c->Kp,
-                                  3, st);
-            }));
-    return GI_OK;
-  });
-}
-
 }  // namespace gi
 
 extern "C" {
