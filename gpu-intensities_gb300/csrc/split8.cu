@@ -50,6 +50,7 @@ constexpr uint32_t kAS = kS * kAP, kBS = kS * kBP, kStage = kAS + kBS;
 constexpr int kST = 3;            // stages
 constexpr int kSegSlices = 186;   // K = 5952 per exact segment
 constexpr int kHi = 6;            // diagonals 0..5 in the high word of an exact sum
+constexpr int kAhead = 8;         // B slices fetched into L2 ahead of their copies
 constexpr int kRing = 4;          // work items in flight between the roles
 constexpr int kThreads = 320;     // warp 0 copies, warp 1 MMA, warps 2..9 epilogue
 // the earlier segments' sums of a tile (20 per epilogue thread), after the
@@ -92,6 +93,16 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
       "l"(src), "r"(bytes), "r"(sptr(bar))
       : "memory");
 }
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(sptr(b)) : "memory");
 }
@@ -101,21 +112,22 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t* r) {
                : "r"(taddr));
 }
 
-// Every digit product of one K slice: plane p of A with planes 0..10-p of B.
-// The window of j = 11 - p planes is 40 j columns, rounded up to a multiple of
-// 16: the extra 8 fall on columns 440..447, which nothing reads.  Windows past
-// 256 columns take two MMAs.  zero: the first slice of a segment overwrites.
-__device__ __forceinline__ void mma_slice(uint32_t tmem, uint64_t a0, uint64_t b0, bool zero) {
-#pragma unroll
-  for (int j = kS; j >= 1; --j) {
-    const int N = (kBN * j + 15) / 16 * 16;
-    const int N1 = N > 256 ? (N / 2 + 15) / 16 * 16 : N;
-    const uint32_t d = tmem + (uint32_t)(kS - j) * kBN;
-    const uint64_t a = a0 + (uint64_t)((kS - j) * kAP >> 4);
-    const uint32_t acc = (j == kS && zero) ? 0u : 1u;
-    mma_e4m3(d, a, b0, idesc_e4m3(N1), acc);
-    if (N > 256) mma_e4m3(d + N1, a, b0 + (uint64_t)(N1 * 32 >> 4), idesc_e4m3(N - N1), acc);
-  }
+// Plane p = 11 - J of A of one K slice (a0, b0: shared-memory addresses / 16 of
+// its A and B) with planes 0..J-1 of B: a window of 40 J columns, rounded up to
+// a multiple of 16 (the extra 8 fall on columns 440..447, which nothing reads).
+// Windows past 256 columns take two MMAs.
+template <int J>
+__device__ __forceinline__ void mma_window(uint32_t tmem, uint32_t a0, uint32_t b0, uint32_t acc) {
+  constexpr int N = (kBN * J + 15) / 16 * 16;
+  constexpr int N1 = N > 256 ? (N / 2 + 15) / 16 * 16 : N;
+  // sdesc_sw32 without the address: 32-byte rows, 8-row groups 256 bytes apart
+  constexpr uint64_t kDesc = (uint64_t)1 << 16 | (uint64_t)(256 >> 4) << 32 | (uint64_t)1 << 46 |
+                             (uint64_t)6 << 61;
+  const uint32_t d = tmem + (uint32_t)(kS - J) * kBN;
+  const uint64_t a = kDesc | (a0 + (uint32_t)((kS - J) * kAP >> 4));
+  mma_e4m3(d, a, kDesc | b0, idesc_e4m3(N1), acc);
+  if constexpr (N > 256)
+    mma_e4m3(d + N1, a, kDesc | (b0 + (uint32_t)(N1 * 32 >> 4)), idesc_e4m3(N - N1), acc);
 }
 
 // The lines of one thread's four columns: groups of G = ndegI * ndegF
@@ -234,6 +246,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int tile = pr.at ? pr.at[ai].tile : ai;
         const uint8_t* Ab = pr.A + (size_t)tile * pr.nkA * kAS;
         const uint8_t* Bb = pr.B + (size_t)ct * pr.nkB * kBS;
+        // the next tile's first B slices on their way to L2 (no tile in flight
+        // has touched them)
         int ks_next = pr.kl ? pr.kl[0] : 0;
         for (int k = 0; k < pr.nk; ++k, ++it) {
           const int st = it % kST, ks = ks_next;
@@ -241,6 +255,13 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (it >= kST && !mbar_wait(&empty[st], ((it / kST) - 1) & 1, abort_flag, err, 42)) {
             ok = false;
             break;
+          }
+          if (k + kAhead < pr.nk) prefetch_l2(Bb + (size_t)(k + kAhead) * kBS, kBS);
+          if (k == 2 && next < P.nitems) {
+            int pj, aj, cj;
+            decode(next, pj, aj, cj);
+            const Prob8& pn = P.p[pj];
+            prefetch_l2(pn.B + (size_t)cj * pn.nkB * kBS, (uint32_t)min(kAhead, pn.nk) * kBS);
           }
           unsigned char* sa = smem + (size_t)st * kStage;
           const int in_seg = k % kSegSlices;
@@ -269,36 +290,61 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // MMA issuer
-      int it = 0, seg = 0;
-      bool ok = true;
-      for (;; ++it) {
-        const int st = it % kST;
-        ok = mbar_wait(&full[st], (it / kST) & 1, abort_flag, err, 44);
-        if (!ok) break;
-        const int mt = meta[st];
-        if (mt & 8) break;
-        if ((mt & 1) && seg > 0) {  // the epilogue has read the previous segment
-          ok = mbar_wait(tfree, (seg - 1) & 1, abort_flag, err, 45);
-          if (!ok) break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const uint32_t sa = sptr(smem + (size_t)st * kStage);
-        mma_slice(tmem, sdesc_sw32(sa), sdesc_sw32(sa + kAS), (mt & 1) != 0);
+    // MMA issuer.  About four MMAs queue behind the one running, so whatever
+    // the issuer does between MMAs has to fit their time: the whole warp runs the
+    // loop (its control and addresses stay in uniform registers) and one lane
+    // issues; the wait for the next slice comes before the three widest of the
+    // narrow windows.  1667 cycles a slice with one lane looping and the wait
+    // between slices, 1522 this way (1376 of MMAs).
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t sbase = __shfl_sync(0xffffffffu, sptr(smem), 0);
+    int st = 0, seg = 0;
+    uint32_t parity = 0;
+    bool ok = __all_sync(0xffffffffu, mbar_wait(&full[0], 0, abort_flag, err, 44));
+    int mt = ok ? __shfl_sync(0xffffffffu, meta[0], 0) : 8;
+    while (!(mt & 8)) {
+      if ((mt & 1) && seg > 0) {  // the epilogue has read the previous segment
+        if (!__all_sync(0xffffffffu, mbar_wait(tfree, (seg - 1) & 1, abort_flag, err, 45))) break;
+      }
+      if (mt & 1) asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t a0 = (sbase + (uint32_t)st * kStage) >> 4, b0 = a0 + (kAS >> 4);
+      if (elect_one()) {
+        mma_window<11>(tm, a0, b0, (mt & 1) ? 0u : 1u);
+        mma_window<1>(tm, a0, b0, 1u);
+        mma_window<2>(tm, a0, b0, 1u);
+        mma_window<3>(tm, a0, b0, 1u);
+        mma_window<4>(tm, a0, b0, 1u);
+        mma_window<5>(tm, a0, b0, 1u);
+        mma_window<6>(tm, a0, b0, 1u);
+        mma_window<7>(tm, a0, b0, 1u);
+      }
+      __syncwarp();
+      const int nst = st + 1 == kST ? 0 : st + 1;
+      if (nst == 0) parity ^= 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&full[nst], parity, abort_flag, err, 44));
+      const int next = ok ? __shfl_sync(0xffffffffu, meta[nst], 0) : 8;
+      if (elect_one()) {
+        mma_window<8>(tm, a0, b0, 1u);
+        mma_window<9>(tm, a0, b0, 1u);
+        mma_window<10>(tm, a0, b0, 1u);
         mma_commit(&empty[st]);
         if (mt & 2) {
           *seg_last = (mt & 4) ? 1 : 0;
           mma_commit(accf);
           mbar_arrive(accf);
-          ++seg;
         }
       }
-      // every MMA issued has completed before the tensor memory is freed
-      mma_commit(drain);
-      const uint64_t t0 = gtimer();
-      while (!mbar_try(drain, 0) && gtimer() - t0 < 1000000000ull) {
-      }
+      __syncwarp();
+      if (mt & 2) ++seg;
+      st = nst;
+      mt = next;
     }
+    // every MMA issued has completed before the tensor memory is freed
+    if (elect_one()) mma_commit(drain);
+    const uint64_t t0 = gtimer();
+    while (!mbar_try(drain, 0) && gtimer() - t0 < 1000000000ull) {
+    }
+    __syncwarp();
   } else {
     // warps 2..9: tensor-memory lane quadrant (warp % 4), 20 of the 40 columns
     const int q4 = warp & 3, half = (warp - 2) >> 2;
