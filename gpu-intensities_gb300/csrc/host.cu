@@ -402,6 +402,19 @@ static bool degeneracy_ok(const Ctx* c, int gI, int gF, int dI, int dF) {
   return true;
 }
 
+// Digit products per column of Y that the default split scheme's half-ls GEMM
+// forms: of the classes in kset and, per component, rset.
+static double half_products8(const Ctx* c, const VibPlan& vp, const std::vector<VibTile>& tiles,
+                             uint32_t kset, const uint32_t rset[3]) {
+  const auto& products = split8_products(c);
+  double sum = 0.0;
+  for (size_t t = 0; t < tiles.size(); t++)
+    if (rset[tiles[t].comp] >> tiles[t].cls & 1)
+      for (int k = 0; k < vp.ncls; k++)
+        if (kset >> k & 1) sum += products[t * vp.ncls + k] * tiles[t].rows;
+  return sum;
+}
+
 gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   auto t_start = std::chrono::steady_clock::now();
   if (c->nrep == 0) return fail(c, GI_ERR_STATE, "gi_set_symmetry not called");
@@ -687,6 +700,8 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   // (unit, slot) whose Y is non-zero on the same classes of functions and whose
   // Z is read on the same classes, per component.
   std::vector<int32_t> h_slotcol;
+  std::vector<VibTile> all_tiles;
+  if (s8) all_tiles = split8_tiles(*vp, 0, N);
   for (Round& R : rounds) {
     R.ncolZ = R.ncolY;
     if (!vib) continue;
@@ -728,18 +743,10 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       band.col0 = R.ncolZ;
       band.boff = R.bbytes;
       R.ncolZ += (band.ncol + kCols8 - 1) / kCols8 * kCols8;
-      double nv = 0.0, nf = 0.0;
-      for (int k = 0; k < vp->ncls; k++) {
-        const double n = (double)vp->members[k].size();
-        if (band.kset >> k & 1) {
-          band.nk += vp->s0[k + 1] - vp->s0[k];
-          nv += n;
-        }
-        for (int q3 = 0; q3 < 3; q3++)
-          if (band.rset[q3] >> k & 1) nf += n;
-      }
+      for (int k = 0; k < vp->ncls; k++)
+        if (band.kset >> k & 1) band.nk += vp->s0[k + 1] - vp->s0[k];
       R.bbytes += s8 ? b_bytes8(band.ncol, band.nk) : band.ncol * band.nk * 32 * sizeof(double);
-      R.flops8 += (double)kDigits8 * (kDigits8 + 1) / 2 * 2.0 * nv * nf * (double)band.ncol;
+      if (s8) R.flops8 += half_products8(c, *vp, all_tiles, band.kset, band.rset) * 2.0 * (double)band.ncol;
       for (const Group8& g : R.groups8[q])
         h_slotcol[R.units[g.unit].sc + g.slot] = (int32_t)(band.col0 + g.col0);
     }
@@ -1857,13 +1864,8 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
       p.Nc = (int)kv.second.size();
       hp->probs.push_back(p);
     }
-    double nv = 0.0;
-    for (int k = 0; k < vp->ncls; k++)
-      if (kv.first >> k & 1) nv += (double)vp->members[k].size();
-    double rows = 0.0;
-    for (const VibTile& t : tiles) rows += t.rows;
-    hp->flops += (double)kDigits8 * (kDigits8 + 1) / 2 * 2.0 * nv * rows *
-                 (double)kv.second.size();
+    const uint32_t every[3] = {vp->all(), vp->all(), vp->all()};
+    hp->flops += half_products8(c, *vp, tiles, kv.first, every) * 2.0 * (double)kv.second.size();
     col0 += round_up((int)kv.second.size(), kCols8);
     boff += b_bytes8(kv.second.size(), nk);
     nb++;

@@ -181,7 +181,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* tfree = accf + 1;      // ... and have been read
   uint64_t* drain = tfree + 1;
   int* items = reinterpret_cast<int*>(drain + 1);
-  int* meta = items + kRing;       // per stage: bit 0 first, 1 last of a segment, 2 of a tile, 3 quit
+  int* meta = items + kRing;       // per stage: bit 0 first, 1 last of a segment, 2 of a tile,
+                                   // 3 quit; from 4 planes np (windows up to np)
   int* seg_last = meta + kST;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(seg_last + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -227,53 +228,96 @@ __global__ void __launch_bounds__(kThreads, 1)
   };
 
   if (warp == 0) {
-    if (lane == 0) {  // scheduler and copies
-      int it = 0, ic = 0;
-      bool ok = true;
-      int item = atomicAdd(P.ctr, 1);
-      for (; ok; ++ic) {
-        const int slot = ic % kRing;
-        if (ic >= kRing) ok = mbar_wait(&iteme[slot], ((ic / kRing) - 1) & 1, abort_flag, err, 41);
-        if (!ok) break;
-        const bool quit = item >= P.nitems;
+    // scheduler and copies: the warp reads the slice lists, lane 0 copies
+    int it = 0, ic = 0;
+    bool ok = true;
+    int item = lane == 0 ? atomicAdd(P.ctr, 1) : 0;
+    item = __shfl_sync(0xffffffffu, item, 0);
+    for (; ok; ++ic) {
+      const int slot = ic % kRing;
+      if (ic >= kRing)
+        ok = __all_sync(0xffffffffu, mbar_wait(&iteme[slot], ((ic / kRing) - 1) & 1, abort_flag,
+                                               err, 41));
+      if (!ok) break;
+      const bool quit = item >= P.nitems;
+      if (lane == 0) {
         items[slot] = quit ? -1 : item;
         mbar_arrive(&itemf[slot]);
-        if (quit) break;
-        const int next = atomicAdd(P.ctr, 1);  // used after this tile's copies
-        int pi, ai, ct;
-        decode(item, pi, ai, ct);
-        const Prob8& pr = P.p[pi];
-        const int tile = pr.at ? pr.at[ai].tile : ai;
-        const uint8_t* Ab = pr.A + (size_t)tile * pr.nkA * kAS;
-        const uint8_t* Bb = pr.B + (size_t)ct * pr.nkB * kBS;
-        // the next tile's first B slices on their way to L2 (no tile in flight
-        // has touched them)
-        int ks_next = pr.kl ? pr.kl[0] : 0;
-        for (int k = 0; k < pr.nk; ++k, ++it) {
-          const int st = it % kST, ks = ks_next;
-          if (k + 1 < pr.nk) ks_next = pr.kl ? pr.kl[k + 1] : k + 1;  // ahead of the wait
-          if (it >= kST && !mbar_wait(&empty[st], ((it / kST) - 1) & 1, abort_flag, err, 42)) {
-            ok = false;
-            break;
-          }
-          if (k + kAhead < pr.nk) prefetch_l2(Bb + (size_t)(k + kAhead) * kBS, kBS);
-          if (k == 2 && next < P.nitems) {
-            int pj, aj, cj;
-            decode(next, pj, aj, cj);
-            const Prob8& pn = P.p[pj];
-            prefetch_l2(pn.B + (size_t)cj * pn.nkB * kBS, (uint32_t)min(kAhead, pn.nk) * kBS);
-          }
-          unsigned char* sa = smem + (size_t)st * kStage;
-          const int in_seg = k % kSegSlices;
-          const bool last = k + 1 == pr.nk;
-          meta[st] = (in_seg == 0 ? 1 : 0) | ((last || in_seg == kSegSlices - 1) ? 2 : 0) |
-                     (last ? 4 : 0);
-          mbar_expect_tx(&full[st], kStage);
-          bulk_load(sa, Ab + (size_t)ks * kAS, kAS, &full[st]);
-          bulk_load(sa + kAS, Bb + (size_t)k * kBS, kBS, &full[st]);
-        }
-        item = next;
       }
+      if (quit) break;
+      int next = lane == 0 ? atomicAdd(P.ctr, 1) : 0;  // used after this tile's copies
+      int pi, ai, ct;
+      decode(item, pi, ai, ct);
+      const Prob8& pr = P.p[pi];
+      const int tile = pr.at ? pr.at[ai].tile : ai;
+      const uint8_t* Ab = pr.A + (size_t)tile * pr.nkA * kAS;
+      const uint8_t* Bb = pr.B + (size_t)ct * pr.nkB * kBS;
+      const uint8_t* za = pr.za ? pr.za + (size_t)tile * pr.nkA : nullptr;
+      // the slices with a digit in A, and the first of those with the fewest zero
+      // planes: it starts the sums (and must cover every diagonal)
+      int total = pr.nk, kfirst = 0;
+      if (za) {
+        total = 0;
+        unsigned best = ~0u;
+        for (int base = 0; base < pr.nk; base += 32) {
+          const int k = base + lane;
+          const unsigned z = k < pr.nk ? za[pr.kl ? pr.kl[k] : k] : kS;
+          total += __popc(__ballot_sync(0xffffffffu, z < (unsigned)kS));
+          best = min(best, (z << 24) | (unsigned)min(k, pr.nk - 1));
+        }
+        best = __reduce_min_sync(0xffffffffu, best);
+        kfirst = (int)(best & 0xFFFFFFu);
+        total = max(total, 1);  // nothing but zeros: one slice, which writes them
+      }
+      int done = 0;
+      auto slice = [&](int k, int ks, int z) {  // (warp-uniform arguments)
+        const int st = it % kST, in_seg = done % kSegSlices;
+        const bool last = done + 1 == total;
+        const uint32_t np = kS - (in_seg == 0 ? 0 : z);  // planes of A and of B
+        if (lane == 0) {
+          if (it >= kST) ok = mbar_wait(&empty[st], ((it / kST) - 1) & 1, abort_flag, err, 42);
+          if (ok) {
+            unsigned char* sa = smem + (size_t)st * kStage;
+            meta[st] = (in_seg == 0 ? 1 : 0) | ((last || in_seg == kSegSlices - 1) ? 2 : 0) |
+                       (last ? 4 : 0) | (int)(np << 4);
+            mbar_expect_tx(&full[st], np * (kAP + kBP));
+            bulk_load(sa + (kS - np) * kAP, Ab + (size_t)ks * kAS + (kS - np) * kAP, np * kAP,
+                      &full[st]);
+            bulk_load(sa + kAS, Bb + (size_t)k * kBS, np * kBP, &full[st]);
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (!ok) return;
+        ++it;
+        ++done;
+        if (done == 2) {  // the next tile's first B slices on their way to L2
+          const int nx = __shfl_sync(0xffffffffu, next, 0);
+          if (nx < P.nitems) {
+            int pj, aj, cj;
+            decode(nx, pj, aj, cj);
+            const Prob8& pn = P.p[pj];
+            if (lane < min(kAhead, pn.nk))
+              prefetch_l2(pn.B + ((size_t)cj * pn.nkB + lane) * kBS, kBS);
+          }
+        }
+      };
+      if (za) slice(kfirst, pr.kl ? pr.kl[kfirst] : kfirst, 0);
+      for (int base = 0; base < pr.nk && ok; base += 32) {
+        const int k = base + lane;
+        const int ks = k < pr.nk ? (pr.kl ? pr.kl[k] : k) : 0;
+        const int z = k < pr.nk ? (za ? za[ks] : 0) : kS;
+        unsigned mask = __ballot_sync(0xffffffffu, z < kS && !(za && k == kfirst));
+        // the B slices of this stretch: no tile in flight may have touched them
+        if (mask >> lane & 1) prefetch_l2(Bb + (size_t)k * kBS, (kS - z) * kBP);
+        while (mask && ok) {
+          const int b = __ffs(mask) - 1;
+          mask &= mask - 1;
+          slice(base + b, __shfl_sync(0xffffffffu, ks, b), __shfl_sync(0xffffffffu, z, b));
+        }
+      }
+      item = __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (lane == 0) {
       if (ok) {  // the MMA issuer leaves on a stage without copies
         const int st = it % kST;
         if (it < kST || mbar_wait(&empty[st], ((it / kST) - 1) & 1, abort_flag, err, 43)) {
@@ -289,6 +333,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // MMA issuer.  About four MMAs queue behind the one running, so whatever
     // the issuer does between MMAs has to fit their time: the whole warp runs the
@@ -308,15 +353,16 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (mt & 1) asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const uint32_t a0 = (sbase + (uint32_t)st * kStage) >> 4, b0 = a0 + (kAS >> 4);
+      const int np = mt >> 4;  // planes 11 - np.. of A have digits
       if (elect_one()) {
-        mma_window<11>(tm, a0, b0, (mt & 1) ? 0u : 1u);
+        if (np == 11) mma_window<11>(tm, a0, b0, (mt & 1) ? 0u : 1u);
         mma_window<1>(tm, a0, b0, 1u);
-        mma_window<2>(tm, a0, b0, 1u);
-        mma_window<3>(tm, a0, b0, 1u);
-        mma_window<4>(tm, a0, b0, 1u);
-        mma_window<5>(tm, a0, b0, 1u);
-        mma_window<6>(tm, a0, b0, 1u);
-        mma_window<7>(tm, a0, b0, 1u);
+        if (np >= 2) mma_window<2>(tm, a0, b0, 1u);
+        if (np >= 3) mma_window<3>(tm, a0, b0, 1u);
+        if (np >= 4) mma_window<4>(tm, a0, b0, 1u);
+        if (np >= 5) mma_window<5>(tm, a0, b0, 1u);
+        if (np >= 6) mma_window<6>(tm, a0, b0, 1u);
+        if (np >= 7) mma_window<7>(tm, a0, b0, 1u);
       }
       __syncwarp();
       const int nst = st + 1 == kST ? 0 : st + 1;
@@ -324,9 +370,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       ok = __all_sync(0xffffffffu, mbar_wait(&full[nst], parity, abort_flag, err, 44));
       const int next = ok ? __shfl_sync(0xffffffffu, meta[nst], 0) : 8;
       if (elect_one()) {
-        mma_window<8>(tm, a0, b0, 1u);
-        mma_window<9>(tm, a0, b0, 1u);
-        mma_window<10>(tm, a0, b0, 1u);
+        if (np >= 8) mma_window<8>(tm, a0, b0, 1u);
+        if (np >= 9) mma_window<9>(tm, a0, b0, 1u);
+        if (np >= 10) mma_window<10>(tm, a0, b0, 1u);
         mma_commit(&empty[st]);
         if (mt & 2) {
           *seg_last = (mt & 4) ? 1 : 0;
@@ -568,6 +614,22 @@ __global__ void __launch_bounds__(256) k_cut8_a(const double* __restrict__ X, si
           out + (size_t)(b >> 7) * (K >> 5) * kAS, kAP, kAS, b & 127, e_out + b);
 }
 
+// za[tile][slice] = the planes from the top that are zero in all 128 rows (a
+// dipole's elements fall off away from the diagonal, and a slice of elements
+// 2^-5z of their rows' largest has nothing in its first z planes).  Block = one
+// slice of a tile; a full top plane, the usual case, is read and left.
+__global__ void __launch_bounds__(256) k_zero_planes(const uint8_t* __restrict__ A,
+                                                     uint8_t* __restrict__ za) {
+  const uint4* a = reinterpret_cast<const uint4*>(A + (size_t)blockIdx.x * kAS) + threadIdx.x;
+  static_assert(kAP == 256 * sizeof(uint4), "a plane is one load per thread");
+  int z = 0;
+  for (; z < kS; ++z) {
+    const uint4 v = a[z * 256];
+    if (__syncthreads_or((v.x | v.y | v.z | v.w) != 0)) break;
+  }
+  if (threadIdx.x == 0) za[blockIdx.x] = (uint8_t)z;
+}
+
 // Rows of several B operands in one launch: operand j has rows
 // [row0[j], row0[j + 1]) of the grid.
 constexpr int kMaxOps8 = kMaxProb8;
@@ -697,6 +759,8 @@ struct Split8 {
   bool mu_valid = false;
   DevArray<uint8_t> mu;
   DevArray<int32_t> mu_exp;
+  DevArray<uint8_t> za;             // zero planes of every slice of it
+  std::vector<double> products;     // split8_products
   DevArray<uint8_t> b;              // B operand workspace
   DevArray<int32_t> b_exp;
   DevArray<int> ctr, err;
@@ -857,6 +921,7 @@ static cudaError_t cut_dipole(Ctx* c, Split8* S, const VibPlan& vp, const double
   k_cut8_a<<<(unsigned)(nt * kBM), 256, 0, c->stream>>>(mu, (size_t)c->Kp, 0, vp.nk * 32,
                                                         S->rowsrc + t0 * kBM, S->vk, S->mu.p,
                                                         S->mu_exp.p);
+  k_zero_planes<<<(unsigned)(nt * vp.nk), 256, 0, c->stream>>>(S->mu.p, S->za.p);
   return cudaGetLastError();
 }
 
@@ -936,10 +1001,27 @@ gi_status split8_prepare(Ctx* c) {
   if ((g = check8(c, S->mu.reserve(a_bytes8(S->most_tiles, vp->nk)), "dipole digits")) != GI_OK)
     return g;
   if ((g = check8(c, S->mu_exp.reserve(S->most_tiles * kBM), "dipole exponents")) != GI_OK) return g;
+  const size_t nza = S->most_tiles * vp->nk;
+  if ((g = check8(c, S->za.reserve(std::max<size_t>(nza, 1)), "zero planes")) != GI_OK) return g;
+  std::vector<uint8_t> h_za(S->panel ? 0 : nza);
   if (!S->panel) {
     if ((g = check8(c, cut_dipole(c, S, *vp, c->d_mu.p, 0), "dipole digits")) != GI_OK) return g;
+    if (nza)
+      g = check8(c, cudaMemcpyAsync(h_za.data(), S->za.p, nza, cudaMemcpyDeviceToHost, c->stream),
+                 "zero planes");
+    if (g != GI_OK) return g;
     if ((g = check8(c, cudaStreamSynchronize(c->stream), "dipole digits")) != GI_OK) return g;
   }
+  const size_t ntile = split8_tiles(*vp, 0, c->N).size();
+  S->products.assign(ntile * vp->ncls, 0.0);
+  for (size_t t = 0; t < ntile; t++)
+    for (int k = 0; k < vp->ncls; k++) {
+      int left = (int)vp->members[k].size();
+      for (int q = vp->s0[k]; q < vp->s0[k + 1]; q++, left -= 32) {
+        const int np = kS - (h_za.empty() ? 0 : h_za[t * vp->nk + q]);
+        S->products[t * vp->ncls + k] += 0.5 * np * (np + 1) * std::min(left, 32);
+      }
+    }
   S->mu_valid = true;
   return GI_OK;
 }
@@ -1011,7 +1093,11 @@ void split8_dipole_operand(Ctx* c, Prob8* p) {
   const Split8* D = (c->parent ? c->parent : c)->split8;
   p->A = D->mu.p;
   p->ea = D->mu_exp.p;
-  p->nkA = (c->parent ? c->parent : c)->split8->plan->nk;
+  p->za = D->za.p;
+  p->nkA = D->plan->nk;
+}
+const std::vector<double>& split8_products(const Ctx* c) {
+  return (c->parent ? c->parent : c)->split8->products;
 }
 uint8_t* split8_b(Ctx* c) { return st8(c)->b.p; }
 int32_t* split8_b_exp(Ctx* c) { return st8(c)->b_exp.p; }
@@ -1201,7 +1287,8 @@ uint64_t split8_identity(Ctx* c) {
   uint64_t h = 14695981039346656037ull;
   for (uint64_t v : {(uint64_t)(uintptr_t)S->b.p, (uint64_t)(uintptr_t)S->b_exp.p,
                      (uint64_t)(uintptr_t)S->ctr.p, (uint64_t)(uintptr_t)S->err.p,
-                     (uint64_t)(uintptr_t)D->mu.p, (uint64_t)(uintptr_t)D->mu_exp.p, D->order_uid,
+                     (uint64_t)(uintptr_t)D->mu.p, (uint64_t)(uintptr_t)D->mu_exp.p, (uint64_t)(uintptr_t)D->za.p,
+                     D->order_uid,
                      split_tuner_version()})
     h = (h ^ v) * 1099511628211ull;
   return h;

@@ -38,6 +38,7 @@ struct Prob8 {
   long long ldc;
   const ATile* at;      // nA row tiles; null: tile i holds rows [128 i, 128 i + 128) of M
   const uint16_t* kl;   // A slice of each of the nk slices; null: the first nk
+  const uint8_t* za;    // [A tile][nkA] planes that are all zero from the top; null: none known
   int nkA, nkB, nk;     // slices per stored A tile, per stored B tile, contracted
   int M, nA, nB, Nc, GA, first;
   // the fused epilogue (see FusedLines)
@@ -73,6 +74,10 @@ const int32_t* vib_rowsrc(const Ctx* c, int panel);
 std::vector<VibTile> split8_tiles(const VibPlan& vp, int f0, int rows);
 // B workspace bytes and columns of the largest launch; final blocks' digits.
 gi_status split8_reserve(Ctx* c, size_t b_bytes, size_t cols, const std::vector<Block*>& finals);
+// Digit products per row and column that the GEMM forms, for tile t of
+// split8_tiles(vp, 0, N) and class k of the contraction: [t * ncls + k] (the
+// zero planes left out, but for a streamed dipole).
+const std::vector<double>& split8_products(const Ctx* c);
 // The context's dipole digits as a problem's A operand.
 void split8_dipole_operand(Ctx* c, Prob8* p);
 uint8_t* split8_b(Ctx* c);

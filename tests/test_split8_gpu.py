@@ -77,3 +77,43 @@ def test_classes_of_functions(pkg, synth, case):
     assert len(a) > 300 and np.array_equal(a[["level_i", "level_f"]], b[["level_i", "level_f"]])
     scale = np.abs(a["t"]).max()
     assert np.abs(a["t"] - b["t"]).max() <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("case", ["decay", "blocks", "zero_rows", "tiny"])
+def test_zero_planes_of_the_dipole(pkg, synth, case):
+    """K slices of the dipole whose leading digit planes are zero skip those
+    planes' products, and slices without any digit are not contracted at all: a
+    banded dipole, whole zero blocks, rows and components that are zero, and
+    blocks 2^-50 of their rows.  Lines and single vectors as the FP64 path's."""
+    N = 420
+    prob = synth.make_c3v(63, N, [1, 2], nvec_max=20)
+    mu = prob.mu.reshape(3, N, N)
+    rng = np.random.default_rng(1)
+    if case == "blocks":
+        mu[:] = rng.standard_normal(mu.shape)
+        mu[:, :, 200:330] = 0.0
+        mu[:, 100:310, :] = 0.0
+    elif case == "zero_rows":
+        mu[:] = rng.standard_normal(mu.shape)
+        mu[1] = 0.0
+        mu[:, rng.random(N) < 0.6] = 0.0
+    elif case == "tiny":
+        mu[:] = rng.standard_normal(mu.shape)
+        mu[:, :, 64:300] *= 2.0 ** -50
+        mu[:, :, 300:] *= 2.0 ** -30
+    out, vec = [], []
+    for precision, streamed in ((0, None), (1, None), (1, 150)):
+        with pkg.Engine(0) as eng:
+            eng.load(prob, precision=precision, panel_rows=streamed)
+            eng.run()
+            out.append(np.sort(eng.lines(), order=["level_i", "level_f"]))
+            vec.append(eng.half_ls(1, 2, 1, 2, prob.blocks[(1, 2)].vecs[0],
+                                   prob.bases[2].Maxcontracts))
+    assert len(out[0]) > 300
+    scale = np.abs(out[0]["t"]).max()
+    for o in out[1:]:
+        assert np.array_equal(o[["level_i", "level_f"]], out[0][["level_i", "level_f"]])
+        assert np.abs(o["t"] - out[0]["t"]).max() <= 1e-12 * scale
+    assert np.array_equal(out[1], out[2])
+    for v in vec[1:]:
+        assert np.abs(v - vec[0]).max() <= 1e-13 * np.abs(vec[0]).max()
