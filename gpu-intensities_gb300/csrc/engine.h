@@ -161,6 +161,11 @@ struct EpiParams {
 // grp = ndegI * ndegF consecutive columns per level.
 struct EpiPart {
   int c0, c1, grp, pad;
+  // log2 of the thresholds' sides that do not depend on the line (line_below in
+  // epilogue.cuh): of Sum t^2 for S, of Sum t^2 |nu| boltz (1 - exp) for I; and of
+  // the error estimate's factors
+  float lx_s, lx_i, l_err;
+  float beta;
   const double* EI;     // the unit's initial energies
   const double* BI;     // their Boltzmann factors exp(-(E - zpe) beta)
   const int32_t* lvI;   // their line ids

@@ -70,6 +70,59 @@ __device__ __forceinline__ void eval_line(const EpiParams& p, const double* t, c
   for (int q = 0; q < 4; ++q) r.L.t[q] = t[q];
 }
 
+// log2 |x| from the bits of x (FP64 instructions are scarce), to 1e-5 or so;
+// zero and denormals come out below -1021, infinities and NaN at 1024.
+__device__ __forceinline__ float lg2_abs(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
+  const float m = __uint_as_float(0x3F800000u | ((hi & 0xFFFFFu) << 3));
+  return (float)((int)(hi >> 20) - 1023) + __log2f(m);
+}
+
+// Moment index dI + 2 dF of column dI * ndegF + dF of a group of G columns.
+template <int G>
+__device__ __forceinline__ int moment_of(int o, int ndegF) {
+  const int dI = (G == 4) ? (o >> 1) : (G == 2 ? (ndegF == 1 ? o : 0) : 0);
+  const int dF = (G == 4) ? (o & 1) : (G == 2 ? (ndegF == 1 ? 0 : o) : 0);
+  return dI + 2 * dF;
+}
+
+// Whether a line that passes the filters is certainly dropped by its threshold,
+// from single-precision logarithms: its S or I at least 1 % below (the
+// logarithms are good to 0.001), and its estimated relative error small enough
+// (below 0.002, eval_line's estimate bounded by its largest terms) that it is
+// not within that of the threshold.  G moments t, hn their columns' norms.
+// Everything else takes eval_line.
+template <int G>
+__device__ __forceinline__ bool line_below(const EpiPart& pt, const double* t, const double* hn,
+                                           double nu, double boltz_i) {
+  const EpiParams& p = pt.ep;
+  if (!(p.thresh_I > 0.0) && !(p.thresh_S > 0.0)) return false;
+  float l[G], lmax = -3000.0f, hmax = -3000.0f;
+#pragma unroll
+  for (int o = 0; o < G; ++o) {
+    const bool used = p.combo_mask >> moment_of<G>(o, p.ndegF) & 1;
+    l[o] = used ? lg2_abs(t[o]) : -3000.0f;
+    lmax = fmaxf(lmax, l[o]);
+    if (used) hmax = fmaxf(hmax, lg2_abs(hn[o]));
+  }
+  float ls = 2.0f * lmax;
+  if constexpr (G > 1) {
+    float sum = 0.0f;
+#pragma unroll
+    for (int o = 0; o < G; ++o) sum += exp2f(2.0f * (l[o] - lmax));
+    ls += __log2f(sum);
+  }
+  if (!(pt.l_err + hmax - lmax < -9.0f)) return false;
+  const bool has_s = p.thresh_S > 0.0;
+  const float ds = ls - pt.lx_s;
+  if (!(p.thresh_I > 0.0)) return ds < -0.02f;
+  if (has_s && !(fabsf(ds) > 0.02f)) return false;
+  const float lnu = lg2_abs(nu);
+  const float x = exp2f(lnu) * pt.beta;
+  const float li = ls + lnu + lg2_abs(boltz_i) + __log2f(-expm1f(-x));
+  return li - pt.lx_i < -0.02f;
+}
+
 // The warp's lines: counts, appends of kept lines, records of doubtful ones.
 // Every lane of the warp calls it (r.pass false where a lane has no line).
 // counter: [0] kept, [1] passing the filters, [2] handed over, [3] doubtful.

@@ -1067,6 +1067,20 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
             e.lvI = c->w_ivec.p + 2 * u.off + u.nI;
             e.hn = c->w_hn.p + hn_off + T.hcol[k];
             e.ep = rparts[part_of[r][t][k]].ep;
+            {
+              // thresholds as bounds on Sum t^2 (of S) and on Sum t^2 |nu| boltz
+              // (1 - exp) (of I), as eval_line forms S and I
+              const EpiParams& ep = e.ep;
+              const double deg = ep.reduced && ep.ndegF != 1 && ep.ndegI != 1 ? 1.0
+                                                                              : 1.0 / ep.ndegI;
+              const double s_of_t = deg * ep.gns * (2 * ep.jI + 1) * (2 * ep.jF + 1);
+              e.lx_s = (float)(std::log2(std::max(ep.thresh_S, 1e-300)) - std::log2(s_of_t));
+              e.lx_i = (float)(std::log2(std::max(ep.thresh_I, 1e-300)) + std::log2(ep.avogno) +
+                               std::log2(ep.q_stat) - std::log2(s_of_t) -
+                               std::log2(ep.intens_cm_mol));
+              e.l_err = (float)(1.0 + std::log2(ep.err_coef) + std::log2((double)g));
+              e.beta = (float)ep.beta;
+            }
             h_epi.push_back(e);
           }
           hn_off += T.ncolH;

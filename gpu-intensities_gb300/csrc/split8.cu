@@ -53,10 +53,11 @@ constexpr int kHi = 6;            // diagonals 0..5 in the high word of an exact
 constexpr int kAhead = 8;         // B slices fetched into L2 ahead of their copies
 constexpr int kRing = 4;          // work items in flight between the roles
 constexpr int kThreads = 320;     // warp 0 copies, warp 1 MMA, warps 2..9 epilogue
-// the earlier segments' sums of a tile (20 per epilogue thread), after the
+// the earlier segments' sums of a tile, or its moments (20 per epilogue thread), after the
 // stages (256 bytes the junk columns read) and the barriers
 constexpr size_t kSumOff = (size_t)kST * kStage + 256 + 512;
-constexpr size_t kSmem = kSumOff + sizeof(double) * 20 * 256 + 1024;
+constexpr size_t kListOff = kSumOff + sizeof(double) * 20 * 256;  // 640 lines per warp
+constexpr size_t kSmem = kListOff + sizeof(uint16_t) * 640 * 8 + 1024;
 static_assert(kSmem <= 227 * 1024, "shared memory");
 static_assert(kStage % 256 == 0 && kAS % 256 == 0, "swizzle periods");
 static_assert((size_t)kS * kSegSlices * 32 * 256 <= (1u << 24), "exact diagonal sums");
@@ -130,37 +131,68 @@ __device__ __forceinline__ void mma_window(uint32_t tmem, uint32_t a0, uint32_t 
     mma_e4m3(d + N1, a, kDesc | (b0 + (uint32_t)(N1 * 32 >> 4)), idesc_e4m3(N - N1), acc);
 }
 
-// The lines of one thread's four columns: groups of G = ndegI * ndegF
-// consecutive columns are the moments of one initial level.
+// The lines of a warp's 20 columns of 32 final levels (m0.. + lane; sum: this
+// thread's moments).  Groups of G = ndegI * ndegF consecutive columns are the
+// moments of one initial level.  A line costs about a hundred FP64 instructions,
+// 150,000 clocks a tile if every line took them, while most lines end below the
+// threshold: those are told by line_below; the rest are listed (moments and
+// list in shared memory) and evaluated with full warps.
 template <int G>
-__device__ __forceinline__ void lines_of4(const Params8& P, const Prob8& pr, int n0, int m,
-                                          bool row_ok, const double* v) {
+__device__ __forceinline__ void lines_of(const Params8& P, const Prob8& pr, int n0, int m0,
+                                         int lane, int rows_left, const double* sum, double* mom,
+                                         uint16_t* lst) {
+  constexpr int kGroups = 20 / G;
+  const int m = m0 + lane;
+  const bool ok_f = lane < rows_left && pr.upper[m];
+  const double ef = ok_f ? pr.EF[m] : 0.0;
 #pragma unroll
-  for (int g0 = 0; g0 < 4; g0 += G) {
-    const int n = n0 + g0;
-    if (n >= pr.Nc) break;  // the same for every lane of the warp
+  for (int j = 0; j < 20; ++j) mom[j * 256 + lane] = sum[j];
+  auto part_of = [&](int n) {
     int q = 0;
     while (q + 1 < pr.nparts && pr.parts[q + 1].c0 <= n) ++q;
-    const EpiPart& pt = pr.parts[q];
-    const EpiParams& ep = pt.ep;
+    return q;
+  };
+  int cnt = 0, npass = 0;
+#pragma unroll
+  for (int g = 0; g < kGroups; ++g) {
+    const int n = n0 + g * G;
+    if (n >= pr.Nc) break;  // the same for every lane
+    const EpiPart& pt = pr.parts[part_of(n)];
     const int i = (n - pt.c0) / G;
-    // column offset dI * ndegF + dF within the group -> moment index dI + 2 dF
+    const double nu = ef - pt.EI[i];
+    const bool pass = ok_f && nu >= pt.ep.fw0 && nu <= pt.ep.fw1;
+    const bool live = pass && !line_below<G>(pt, sum + g * G, pt.hn + i * G, nu, pt.BI[i]);
+    npass += __popc(__ballot_sync(0xffffffffu, pass));
+    const unsigned mask = __ballot_sync(0xffffffffu, live);
+    if (live) lst[cnt + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)(g * 32 + lane);
+    cnt += __popc(mask);
+  }
+  if (npass && lane == 0) atomicAdd(P.counter + 1, (unsigned long long)npass);
+  __syncwarp();
+  for (int k0 = 0; k0 < cnt; k0 += 32) {
+    const bool on = k0 + lane < cnt;
+    const int code = on ? lst[k0 + lane] : 0;
+    const int g = code >> 5, src = code & 31;
+    const int n = n0 + g * G;
+    const EpiPart& pt = pr.parts[part_of(n)];
+    const EpiParams& ep = pt.ep;
+    const int i = (n - pt.c0) / G, mm = m0 + src;
     double t[4] = {0.0, 0.0, 0.0, 0.0}, hnq[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int o = 0; o < G; ++o) {
-      const int dI = (G == 4) ? (o >> 1) : (G == 2 ? (ep.ndegF == 1 ? o : 0) : 0);
-      const int dF = (G == 4) ? (o & 1) : (G == 2 ? (ep.ndegF == 1 ? 0 : o) : 0);
-      if (ep.combo_mask & (1 << (dI + 2 * dF))) {
-        t[dI + 2 * dF] = v[g0 + o];
-        hnq[dI + 2 * dF] = pt.hn[i * G + o];
+      const int q = moment_of<G>(o, ep.ndegF);
+      if (ep.combo_mask & (1 << q)) {
+        t[q] = mom[(g * G + o) * 256 + src];
+        hnq[q] = pt.hn[i * G + o];
       }
     }
-    const bool ok_f = row_ok && pr.upper[m];
     LineEval r;
-    eval_line(ep, t, hnq, pt.EI[i], ok_f ? pr.EF[m] : 0.0, pt.BI[i], ok_f, pt.lvI[i],
-              ok_f ? pr.lvF[m] : -1, r);
-    append_line(r, ep.part, i, m, P.out, P.counter, P.cap, P.rec, P.rec_cap);
+    eval_line(ep, t, hnq, pt.EI[i], on ? pr.EF[mm] : 0.0, pt.BI[i], on, pt.lvI[i],
+              on ? pr.lvF[mm] : -1, r);
+    r.pass = false;  // counted above
+    append_line(r, ep.part, i, mm, P.out, P.counter, P.cap, P.rec, P.rec_cap);
   }
+  __syncwarp();
 }
 
 // One persistent CTA per SM; work items are 128 x 40 tiles of the launch's
@@ -477,17 +509,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!ok) break;
       if (P.fused) {
-        const int G = pr.parts[0].grp, m = ai * kBM + r;
-#pragma unroll
-        for (int ch = 0; ch < 5; ++ch) {
-          if (n0 + ch * 4 >= pr.Nc) break;  // the same for every lane
-          if (G == 4)
-            lines_of4<4>(P, pr, n0 + ch * 4, m, row_ok, sum + ch * 4);
-          else if (G == 2)
-            lines_of4<2>(P, pr, n0 + ch * 4, m, row_ok, sum + ch * 4);
-          else
-            lines_of4<1>(P, pr, n0 + ch * 4, m, row_ok, sum + ch * 4);
-        }
+        const int G = pr.parts[0].grp, m0 = ai * kBM + q4 * 32, left = at.rows - q4 * 32;
+        double* mom = reinterpret_cast<double*>(smem + kSumOff) + (warp - 2) * 32;
+        uint16_t* lst = reinterpret_cast<uint16_t*>(smem + kListOff) + (warp - 2) * 640;
+        if (G == 4)
+          lines_of<4>(P, pr, n0, m0, lane, left, sum, mom, lst);
+        else if (G == 2)
+          lines_of<2>(P, pr, n0, m0, lane, left, sum, mom, lst);
+        else
+          lines_of<1>(P, pr, n0, m0, lane, left, sum, mom, lst);
       } else if (row_ok) {
         double* dst = pr.C + at.coff + r;
 #pragma unroll

@@ -117,3 +117,33 @@ def test_zero_planes_of_the_dipole(pkg, synth, case):
     assert np.array_equal(out[1], out[2])
     for v in vec[1:]:
         assert np.abs(v - vec[0]).max() <= 1e-13 * np.abs(vec[0]).max()
+
+
+@pytest.mark.parametrize("case", ["c2v", "c3v", "c3v_reduced"])
+@pytest.mark.parametrize("which", ["I", "S", "both"])
+def test_thresholds_keep_exactly_the_lines_above(pkg, synth, case, which):
+    """Lines told to be below a threshold from single-precision logarithms: a
+    run with thresholds keeps bit for bit the lines of a run without that are at
+    or above them, and counts the same lines through the filters."""
+    if case == "c2v":
+        prob = synth.make_c2v(64, 150, [1, 2, 3], nvec_max=60)
+    else:
+        prob = synth.make_c3v(65, 120, [1, 2, 3], nvec_max=50, reduced=case.endswith("reduced"))
+    with pkg.Engine(0) as eng:
+        eng.load(prob, precision=pkg.GI_PREC_SPLIT)
+        eng.run()
+        every, n = np.sort(eng.lines(), order=["level_i", "level_f"]), eng.stats()["nlines_filtered"]
+        avogno = 6.0221415e23
+        tS, tI = np.quantile(every["S"], 0.6), np.quantile(every["I"] / avogno, 0.7)
+        prob.params.thresh_linestrength = float(tS) if which in ("S", "both") else 0.0
+        prob.params.thresh_intensity = float(tI) if which in ("I", "both") else 0.0
+        eng.set_params(prob.params, precision=pkg.GI_PREC_SPLIT)
+        eng.run()
+        kept, m = np.sort(eng.lines(), order=["level_i", "level_f"]), eng.stats()["nlines_filtered"]
+    want = every[(every["S"] >= prob.params.thresh_linestrength) &
+                 (every["I"] / avogno >= prob.params.thresh_intensity)]
+    assert n == m == len(every) > 2000 and 100 < len(want) < len(every)
+    # (a line at the threshold itself is evaluated exactly, its values replaced)
+    assert np.array_equal(kept[["level_i", "level_f"]], want[["level_i", "level_f"]])
+    assert np.allclose(kept["S"], want["S"], rtol=1e-11, atol=0)
+    assert np.count_nonzero(kept["S"] != want["S"]) <= 2
