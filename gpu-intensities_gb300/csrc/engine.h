@@ -213,6 +213,7 @@ struct Basis {
   std::vector<int32_t> v_kind;
   std::vector<uint8_t> kind_mask;
   int nkind = 0;
+  std::vector<int64_t> y_nnz;  // per gamma: (slot, function) places with a coefficient
   // most symmetrised functions with a non-zero coefficient on one root, per
   // gamma, and most roots on one (slot, v)
   std::vector<int32_t> root_ent;

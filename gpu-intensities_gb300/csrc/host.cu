@@ -233,6 +233,14 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
     if (it.second) b.kind_mask.insert(b.kind_mask.end(), key.begin(), key.end());
   }
   b.nkind = (int)kinds.size();
+  std::vector<int64_t> of_kind(b.nkind, 0);
+  for (int kind : b.v_kind)
+    if (kind >= 0) of_kind[kind]++;
+  b.y_nnz.assign(nrep, 0);
+  for (int k = 0; k < b.nkind; k++)
+    for (int slot = 0; slot < b.nslot; slot++)
+      for (unsigned m = b.kind_mask[(size_t)k * b.nslot + slot]; m; m &= m - 1)
+        b.y_nnz[__builtin_ctz(m)] += of_kind[k];
   return GI_OK;
 }
 
@@ -2429,10 +2437,12 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   }
   int32_t* err_word = reinterpret_cast<int32_t*>(c->hls_pin + (c->hls_pin_cap - 1));
   // In the default split scheme a small vector's product goes through FP64,
-  // which is more accurate and, with Y packed to its non-zero values, faster: up
-  // to 2^24 products (half of them zeros at most) cost 30 to 60 us in all, the
-  // digits 65 us at any smaller size.
-  const bool small = split8_selected(c) && 3.0 * c->N * c->N * bI.nslot <= (double)(1 << 24);
+  // which is more accurate, needs no digits of the dipole and, with Y packed to
+  // its non-zero values, is faster up to about 25 million products: 32 million
+  // (C2v, N = 1017, J = 10) took 101 us a call against 92 with digits, 5 million
+  // (N = 555, J = 5) 51 against 68.
+  const bool small =
+      split8_selected(c) && 3.0 * c->N * (double)bI.y_nnz[gammaI] <= (double)(3 << 23);
   const bool split_path =
       c->have_params && c->params.precision == GI_PREC_SPLIT && !c->streamed() && !small;
   if (split_path) {

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("group,N,jlist,precision", [
     ("c2v", 1, [0, 1], 0), ("c2v", 63, [1, 2], 0), ("c2v", 64, [1, 2], 0), ("c3v", 65, [1, 2], 0),
-    ("c3v", 130, [3, 4], 0), ("c2v", 333, [2], 1), ("c2v", 1300, [6, 7], 1), ("c3v", 1250, [6], 1)])
+    ("c3v", 130, [3, 4], 0), ("c2v", 333, [2], 1), ("c2v", 1900, [8, 9], 1), ("c3v", 1250, [6], 1)])
 def test_half_ls_sizes(pkg, synth, oracle, group, N, jlist, precision):
     prob = (synth.make_c2v if group == "c2v" else synth.make_c3v)(N, N, jlist, nvec_max=1)
     with pkg.Engine(0) as eng:
