@@ -2591,6 +2591,8 @@ extern "C" gi_status gi_probe_split_gemm(int device, int slices, int M, int N, i
   Ctx c;
   c.device = device;
   c.params.split_slices = slices;
+  if (cudaDeviceGetAttribute(&c.nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return GI_ERR_CUDA;
   if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess)
     return GI_ERR_CUDA;
   SplitState* S = state(&c);
@@ -2610,10 +2612,12 @@ extern "C" gi_status gi_probe_split_gemm(int device, int slices, int M, int N, i
   ck(dA.alloc((size_t)M * Kp));
   ck(dB.alloc((size_t)N * Kp));
   ck(dC.alloc((size_t)N * M));
-  ck(sa.alloc((size_t)S->s * Mpad * Kp));
-  ck(sb.alloc((size_t)S->s * N * Kp));
-  ck(xa.alloc(Mpad));
-  ck(xb.alloc(N));
+  if (!split8_selected(&c)) {
+    ck(sa.alloc((size_t)S->s * Mpad * Kp));
+    ck(sb.alloc((size_t)S->s * N * Kp));
+    ck(xa.alloc(Mpad));
+    ck(xb.alloc(N));
+  }
   ck(S->err.reserve(1));
   if (g == GI_OK) {
     ck(cudaMemset(dA.p, 0, sizeof(double) * dA.n));
