@@ -50,6 +50,9 @@ constexpr uint32_t kAS = kS * kAP, kBS = kS * kBP, kStage = kAS + kBS;
 constexpr int kST = 3;            // stages
 constexpr int kSegSlices = 186;   // K = 5952 per exact segment
 constexpr int kHi = 6;            // diagonals 0..5 in the high word of an exact sum
+// Planes summed over a segment's slices up to which its sums stay within 2^22: a slice of
+// np planes adds np products per k to diagonal 10, fewer to the others.
+constexpr int kSmallPlanes = (1 << 22) / (32 * 256);
 constexpr int kAhead = 8;         // B slices fetched into L2 ahead of their copies
 constexpr int kRing = 4;          // work items in flight between the roles
 constexpr int kThreads = 320;     // warp 0 copies, warp 1 MMA, warps 2..9 epilogue
@@ -129,6 +132,35 @@ __device__ __forceinline__ void mma_window(uint32_t tmem, uint32_t a0, uint32_t 
   mma_e4m3(d, a, kDesc | b0, idesc_e4m3(N1), acc);
   if constexpr (N > 256)
     mma_e4m3(d + N1, a, kDesc | (b0 + (uint32_t)(N1 * 32 >> 4)), idesc_e4m3(N - N1), acc);
+}
+
+// The exact sums of 20 columns, hi = diagonals 0..5 and lo = 6..10 (below 2^53
+// each).  The tensor memory is held meanwhile, 20 x 11 conversions a thread at 8
+// clocks a warp; a sum within 2^22 is instead read off the bits of itself plus
+// 1.5 2^23, one addition (SMALL: the segments of up to about 46 slices, where
+// this time is the larger part: 2200 clocks a tile instead of 4000; the rounds
+// of half line strengths of a C3v J = 12..13 batch at N = 1500 with 25 slices a tile took
+// 3 % less).
+template <bool SMALL>
+__device__ __forceinline__ void fold_sums(uint32_t t0, long long* hi, long long* lo) {
+  auto whole = [](uint32_t f) {
+    const float x = __uint_as_float(f);
+    return SMALL ? __float_as_int(x + 12582912.0f) - 0x4B400000 : __float2int_rn(x);
+  };
+#pragma unroll
+  for (int ch = 0; ch < 5; ++ch) {
+    uint32_t f[kS][4];
+#pragma unroll
+    for (int d = 0; d < kS; ++d) tmem_ld4(t0 + d * kBN + ch * 4, f[d]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      // pairs of diagonals fit 32 bits (|sum| <= 2^24): 2^29 + 2^24
+      auto pair = [&](int d) { return whole(f[d][j]) * 32 + whole(f[d + 1][j]); };
+      hi[ch * 4 + j] = pair(0) * 1048576ll + (pair(2) * 1024ll + pair(4));
+      lo[ch * 4 + j] = pair(6) * 32768ll + (pair(8) * 32ll + whole(f[10][j]));
+    }
+  }
 }
 
 // The lines of a warp's 20 columns of 32 final levels (m0.. + lane; sum: this
@@ -214,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* drain = tfree + 1;
   int* items = reinterpret_cast<int*>(drain + 1);
   int* meta = items + kRing;       // per stage: bit 0 first, 1 last of a segment, 2 of a tile,
-                                   // 3 quit; from 4 planes np (windows up to np)
+                                   // 3 quit, 4..7 planes np (windows up to np), 8 small sums
   int* seg_last = meta + kST;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(seg_last + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -301,17 +333,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         kfirst = (int)(best & 0xFFFFFFu);
         total = max(total, 1);  // nothing but zeros: one slice, which writes them
       }
-      int done = 0;
+      int done = 0, planes = 0;
       auto slice = [&](int k, int ks, int z) {  // (warp-uniform arguments)
         const int st = it % kST, in_seg = done % kSegSlices;
         const bool last = done + 1 == total;
         const uint32_t np = kS - (in_seg == 0 ? 0 : z);  // planes of A and of B
+        planes = (in_seg == 0 ? 0 : planes) + (int)np;
         if (lane == 0) {
           if (it >= kST) ok = mbar_wait(&empty[st], ((it / kST) - 1) & 1, abort_flag, err, 42);
           if (ok) {
             unsigned char* sa = smem + (size_t)st * kStage;
             meta[st] = (in_seg == 0 ? 1 : 0) | ((last || in_seg == kSegSlices - 1) ? 2 : 0) |
-                       (last ? 4 : 0) | (int)(np << 4);
+                       (last ? 4 : 0) | (int)(np << 4) | (planes <= kSmallPlanes ? 256 : 0);
             mbar_expect_tx(&full[st], np * (kAP + kBP));
             bulk_load(sa + (kS - np) * kAP, Ab + (size_t)ks * kAS + (kS - np) * kAP, np * kAP,
                       &full[st]);
@@ -385,7 +418,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (mt & 1) asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const uint32_t a0 = (sbase + (uint32_t)st * kStage) >> 4, b0 = a0 + (kAS >> 4);
-      const int np = mt >> 4;  // planes 11 - np.. of A have digits
+      const int np = mt >> 4 & 15;  // planes 11 - np.. of A have digits
       if (elect_one()) {
         if (np == 11) mma_window<11>(tm, a0, b0, (mt & 1) ? 0u : 1u);
         mma_window<1>(tm, a0, b0, 1u);
@@ -407,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (np >= 10) mma_window<10>(tm, a0, b0, 1u);
         mma_commit(&empty[st]);
         if (mt & 2) {
-          *seg_last = (mt & 4) ? 1 : 0;
+          *seg_last = mt;
           mma_commit(accf);
           mbar_arrive(accf);
         }
@@ -457,34 +490,16 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (bool last = false, first = true; !last; first = false, ++seg) {
         ok = mbar_wait(accf, seg & 1, abort_flag, err, 47, 128);
         if (!ok) break;
-        last = *seg_last != 0;
+        const int flags = *seg_last;
+        last = (flags & 4) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         // exact sums, hi = diagonals 0..5 and lo = 6..10 (below 2^53 each)
         long long hi[20], lo[20];
-#pragma unroll
-        for (int ch = 0; ch < 5; ++ch) {
-          uint32_t f[kS][4];
-#pragma unroll
-          for (int d = 0; d < kS; ++d)
-            tmem_ld4(tmem + lanes + d * kBN + half * 20 + ch * 4, f[d]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            // pairs of diagonals fit 32 bits (|sum| <= 2^24): 2^29 + 2^24
-            auto pair = [&](int d) {
-              return __float2int_rn(__uint_as_float(f[d][j])) * 32 +
-                     __float2int_rn(__uint_as_float(f[d + 1][j]));
-            };
-            long long h = pair(0);
-            h = h * 1024 + pair(2);
-            h = h * 1024 + pair(4);
-            long long l = pair(6);
-            l = l * 1024 + pair(8);
-            l = l * 32 + __float2int_rn(__uint_as_float(f[10][j]));
-            hi[ch * 4 + j] = h;
-            lo[ch * 4 + j] = l;
-          }
-        }
+        const uint32_t t0 = tmem + lanes + half * 20;
+        if (flags & 256)
+          fold_sums<true>(t0, hi, lo);
+        else
+          fold_sums<false>(t0, hi, lo);
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(tfree);

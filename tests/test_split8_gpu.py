@@ -39,6 +39,20 @@ def test_constant_rows_stay_exact(pkg, value, K):
     assert np.abs(got - want).max() <= 1e-15 * abs(want)
 
 
+@pytest.mark.parametrize("value", [15.0 / 31.0, -15.0 / 31.0, 0.5 - 2.0 ** -54])
+@pytest.mark.parametrize("K", [1409, 1472, 1473])
+def test_short_segments_stay_exact(pkg, value, K):
+    """Sums on both sides of the length up to which they are read off the bits
+    (46 slices): 15/31 is the digit 15 eleven times, 7/8 of the largest sum
+    there is.  Left out of the result are products of 2^-55 of it, about 3e-16;
+    its own roundings and those of the value wanted are as much again."""
+    A = np.full((130, K), value)
+    B = np.full((42, K), 15.0 / 31.0)
+    got = pkg.split_gemm(A, B)
+    want = K * value * (15.0 / 31.0)
+    assert np.abs(got - want).max() <= 1e-15 * abs(want)
+
+
 @pytest.mark.parametrize("case", ["unused", "few_kinds", "many_kinds", "empty_columns"])
 def test_classes_of_functions(pkg, synth, case):
     """The half-line-strength GEMM skips what the symmetries rule out, by
