@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int tile = pr.at ? pr.at[ai].tile : ai;
       const uint8_t* Ab = pr.A + (size_t)tile * pr.nkA * kAS;
       const uint8_t* Bb = pr.B + (size_t)ct * pr.nkB * kBS;
-      const uint8_t* za = pr.za ? pr.za + (size_t)tile * pr.nkA : nullptr;
+      const int32_t* za = pr.za ? pr.za + (size_t)tile * pr.nkA : nullptr;
       // the slices with a digit in A, and the first of those with the fewest zero
       // planes: it starts the sums (and must cover every diagonal)
       int total = pr.nk, kfirst = 0;
@@ -325,9 +325,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         unsigned best = ~0u;
         for (int base = 0; base < pr.nk; base += 32) {
           const int k = base + lane;
-          const unsigned z = k < pr.nk ? za[pr.kl ? pr.kl[k] : k] : kS;
-          total += __popc(__ballot_sync(0xffffffffu, z < (unsigned)kS));
-          best = min(best, (z << 24) | (unsigned)min(k, pr.nk - 1));
+          const int z = k < pr.nk ? za[pr.kl ? pr.kl[k] : k] : kS;
+          total += __popc(__ballot_sync(0xffffffffu, z < kS));
+          best = min(best, ((unsigned)min(z, kS) << 24) | (unsigned)min(k, pr.nk - 1));
         }
         best = __reduce_min_sync(0xffffffffu, best);
         kfirst = (int)(best & 0xFFFFFFu);
@@ -572,21 +572,25 @@ __device__ __forceinline__ uint32_t e4m3x2(uint32_t u0, uint32_t u1) {
                                               __NV_E4M3);
 }
 // The digits of four consecutive elements k..k+3 of a row: one word per plane,
-// planes `ps` bytes apart.
-__device__ __forceinline__ void cut4(const double* x, int e, uint8_t* dst, uint32_t ps) {
+// planes `ps` bytes apart.  Returns the first plane with a digit (kS: none).
+__device__ __forceinline__ int cut4(const double* x, int e, uint8_t* dst, uint32_t ps) {
   unsigned long long b[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) b[i] = (unsigned long long)fixed_point(x[i], e, kW * kS) + kBias;
+  int z = kS;
 #pragma unroll
-  for (int p = 0; p < kS; ++p) {
+  for (int p = kS - 1; p >= 0; --p) {
     uint32_t u[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       u[i] = (uint32_t)(b[i] >> (kW * (kS - 1 - p)));
       if (p > 0) u[i] &= 31u;
     }
-    *reinterpret_cast<uint32_t*>(dst + p * ps) = e4m3x2(u[0], u[1]) | (e4m3x2(u[2], u[3]) << 16);
+    const uint32_t w = e4m3x2(u[0], u[1]) | (e4m3x2(u[2], u[3]) << 16);
+    if (w) z = p;
+    *reinterpret_cast<uint32_t*>(dst + p * ps) = w;
   }
+  return z;
 }
 // Byte of element k (a multiple of 4) of row r within a tile's slices of
 // `ss` bytes: 32-byte rows, 16-byte halves swapped in every other group of
@@ -612,10 +616,11 @@ __device__ __forceinline__ unsigned long long magnitude(double v) {
 
 // One row of K = 4 K4 doubles (null: zeros) into row r of a tile; vk gathers
 // its elements (-1: zero).  Memory bound: 8 B read (twice, the second time
-// from L2) and 11 B written per element.
+// from L2) and 11 B written per element.  za (or null): the first plane with a
+// digit of each slice, taken to the least of the tile's rows.
 __device__ __forceinline__ void cut_row(const double* __restrict__ x, const int32_t* __restrict__ vk,
                                         int K, uint8_t* tile, uint32_t ps, uint32_t ss, int r,
-                                        int32_t* e_out) {
+                                        int32_t* e_out, int32_t* za = nullptr) {
   auto get = [&](int k, double* v) {
     if (!x) {
       v[0] = v[1] = v[2] = v[3] = 0.0;
@@ -643,40 +648,32 @@ __device__ __forceinline__ void cut_row(const double* __restrict__ x, const int3
   for (int k = threadIdx.x * 4; k < K; k += 1024) {
     double v[4];
     get(k, v);
-    cut4(v, e, tile + row_byte(r, k, ss), ps);
+    int z = cut4(v, e, tile + row_byte(r, k, ss), ps);
+    if (za) {  // K is a multiple of 32: the eight threads of a slice are all here
+      const unsigned eight = 0xffu << (threadIdx.x & 24);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) z = min(z, __shfl_xor_sync(eight, z, o));
+      if ((threadIdx.x & 7) == 0 && z < za[k >> 5]) atomicMin(za + (k >> 5), z);
+    }
   }
 }
 
 // Rows of an A operand: block b is row b % 128 of tile b / 128.  rowsrc: source
-// row of each (-1: zeros); null: row b of `rows`.
+// row of each (-1: zeros); null: row b of `rows`.  za[tile][slice] (or null; at
+// least kS before): the planes from the top that are zero in all 128 rows (a
+// dipole's elements fall off away from the diagonal, and a slice of elements
+// 2^-5z of their rows' largest has nothing in its first z planes).  Taken here,
+// where the digits are at hand; reading them back took 27 us at N = 1500.
 __global__ void __launch_bounds__(256) k_cut8_a(const double* __restrict__ X, size_t ldx, int rows,
                                                 int K, const int32_t* __restrict__ rowsrc,
                                                 const int32_t* __restrict__ vk,
                                                 uint8_t* __restrict__ out,
-                                                int32_t* __restrict__ e_out) {
+                                                int32_t* __restrict__ e_out, int32_t* za) {
   const int b = blockIdx.x, src = rowsrc ? rowsrc[b] : (b < rows ? b : -1);
   cut_row(src >= 0 ? X + (size_t)src * ldx : nullptr, vk, K,
-          out + (size_t)(b >> 7) * (K >> 5) * kAS, kAP, kAS, b & 127, e_out + b);
+          out + (size_t)(b >> 7) * (K >> 5) * kAS, kAP, kAS, b & 127, e_out + b, za ? za + (size_t)(b >> 7) * (K >> 5) : nullptr);
 }
 
-// za[tile][slice] = the planes from the top that are zero in all 128 rows (a
-// dipole's elements fall off away from the diagonal, and a slice of elements
-// 2^-5z of their rows' largest has nothing in its first z planes).  Block = one
-// slice of a tile; a full top plane, the usual case, is read and left.
-__global__ void __launch_bounds__(256) k_zero_planes(const uint8_t* __restrict__ A,
-                                                     uint8_t* __restrict__ za) {
-  const uint4* a = reinterpret_cast<const uint4*>(A + (size_t)blockIdx.x * kAS) + threadIdx.x;
-  static_assert(kAP == 256 * sizeof(uint4), "a plane is one load per thread");
-  int z = 0;
-  for (; z < kS; ++z) {
-    const uint4 v = a[z * 256];
-    if (__syncthreads_or((v.x | v.y | v.z | v.w) != 0)) break;
-  }
-  if (threadIdx.x == 0) za[blockIdx.x] = (uint8_t)z;
-}
-
-// Rows of several B operands in one launch: operand j has rows
-// [row0[j], row0[j + 1]) of the grid.
 constexpr int kMaxOps8 = kMaxProb8;
 struct CutOps8 {
   int n;
@@ -804,7 +801,7 @@ struct Split8 {
   bool mu_valid = false;
   DevArray<uint8_t> mu;
   DevArray<int32_t> mu_exp;
-  DevArray<uint8_t> za;             // zero planes of every slice of it
+  DevArray<int32_t> za;             // zero planes of every slice of it
   std::vector<double> products;     // split8_products
   DevArray<uint8_t> b;              // B operand workspace
   DevArray<int32_t> b_exp;
@@ -963,10 +960,12 @@ void vib_rows_needed(const Ctx* c, const VibPlan& vp, const Basis& bI, int gF, i
 static cudaError_t cut_dipole(Ctx* c, Split8* S, const VibPlan& vp, const double* mu, int p) {
   const size_t t0 = S->panel_tile[p], nt = S->panel_tile[p + 1] - t0;
   if (nt == 0) return cudaSuccess;
+  // every byte kS: above kS as a word, the start of the minimum
+  const cudaError_t e = cudaMemsetAsync(S->za.p, kS, nt * vp.nk * sizeof(int32_t), c->stream);
+  if (e != cudaSuccess) return e;
   k_cut8_a<<<(unsigned)(nt * kBM), 256, 0, c->stream>>>(mu, (size_t)c->Kp, 0, vp.nk * 32,
                                                         S->rowsrc + t0 * kBM, S->vk, S->mu.p,
-                                                        S->mu_exp.p);
-  k_zero_planes<<<(unsigned)(nt * vp.nk), 256, 0, c->stream>>>(S->mu.p, S->za.p);
+                                                        S->mu_exp.p, S->za.p);
   return cudaGetLastError();
 }
 
@@ -1048,11 +1047,11 @@ gi_status split8_prepare(Ctx* c) {
   if ((g = check8(c, S->mu_exp.reserve(S->most_tiles * kBM), "dipole exponents")) != GI_OK) return g;
   const size_t nza = S->most_tiles * vp->nk;
   if ((g = check8(c, S->za.reserve(std::max<size_t>(nza, 1)), "zero planes")) != GI_OK) return g;
-  std::vector<uint8_t> h_za(S->panel ? 0 : nza);
+  std::vector<int32_t> h_za(S->panel ? 0 : nza);
   if (!S->panel) {
     if ((g = check8(c, cut_dipole(c, S, *vp, c->d_mu.p, 0), "dipole digits")) != GI_OK) return g;
     if (nza)
-      g = check8(c, cudaMemcpyAsync(h_za.data(), S->za.p, nza, cudaMemcpyDeviceToHost, c->stream),
+      g = check8(c, cudaMemcpyAsync(h_za.data(), S->za.p, nza * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream),
                  "zero planes");
     if (g != GI_OK) return g;
     if ((g = check8(c, cudaStreamSynchronize(c->stream), "dipole digits")) != GI_OK) return g;
@@ -1063,7 +1062,7 @@ gi_status split8_prepare(Ctx* c) {
     for (int k = 0; k < vp->ncls; k++) {
       int left = (int)vp->members[k].size();
       for (int q = vp->s0[k]; q < vp->s0[k + 1]; q++, left -= 32) {
-        const int np = kS - (h_za.empty() ? 0 : h_za[t * vp->nk + q]);
+        const int np = kS - (h_za.empty() ? 0 : std::min(h_za[t * vp->nk + q], kS));
         S->products[t * vp->ncls + k] += 0.5 * np * (np + 1) * std::min(left, 32);
       }
     }
@@ -1092,7 +1091,8 @@ static gi_status block_digits8(Ctx* c, Block& fb, bool wait) {
       g = check8(c, timed(c, GI_PHASE_SLICE, [&] {
                    k_cut8_a<<<vpad, 256, 0, c->stream>>>(
                        fb.d_vecs.p, (size_t)fb.ld, fb.nvec, fb.ld, nullptr, nullptr,
-                       reinterpret_cast<uint8_t*>(fb.d_digits.p), fb.d_digit_exp.p);
+                       reinterpret_cast<uint8_t*>(fb.d_digits.p), fb.d_digit_exp.p,
+                       nullptr);
                    return cudaGetLastError();
                  }),
                  "V digits");
@@ -1369,7 +1369,8 @@ gi_status split8_probe(Ctx* c, int M, int N, int K, const double* dA, const doub
   if (g == GI_OK) g = check8(c, eb.alloc(N + kCols8), "B exponents");
   if (g == GI_OK) g = check8(c, cudaDeviceSynchronize(), "operands");
   if (g != GI_OK) return g;
-  k_cut8_a<<<vpad, 256, 0, c->stream>>>(dA, (size_t)ld, M, ld, nullptr, nullptr, a.p, ea.p);
+  k_cut8_a<<<vpad, 256, 0, c->stream>>>(dA, (size_t)ld, M, ld, nullptr, nullptr, a.p, ea.p,
+                                        nullptr);
   if ((g = check8(c, cudaGetLastError(), "A digits")) != GI_OK) return g;
   CutOps8* ops = new CutOps8();
   ops->n = 1;

@@ -38,7 +38,7 @@ struct Prob8 {
   long long ldc;
   const ATile* at;      // nA row tiles; null: tile i holds rows [128 i, 128 i + 128) of M
   const uint16_t* kl;   // A slice of each of the nk slices; null: the first nk
-  const uint8_t* za;    // [A tile][nkA] planes that are all zero from the top; null: none known
+  const int32_t* za;    // [A tile][nkA] planes that are all zero from the top; null: none known
   int nkA, nkB, nk;     // slices per stored A tile, per stored B tile, contracted
   int M, nA, nB, Nc, GA, first;
   // the fused epilogue (see FusedLines)
