@@ -22,8 +22,8 @@ intensity threshold (1e-30 cm/molecule; the post-threshold rate beside it).
           shards and reads every line back to host memory (40-byte compact
           records); the digit planes of the new blocks are re-cut inside it
   roofline    the half-ls split GEMM (the dominant kernel): tensor-pipe rate of
-          its bf16 digit products against the measured bf16 peak, its FP64-
-          equivalent rate, and its DRAM traffic
+          its digit products against the measured bf16 peak (twice that for
+          the default scheme's 8-bit MMAs) and its FP64-equivalent rate
   fp64_path   the plain FP64 GPU path and the split path on the same batch (one
           fortieth of the job)
   accuracy    per-line error of both paths against the CPU oracle (double-double
@@ -63,14 +63,6 @@ SHARDS = {"c3v_batched": 10}
 # lowest initial levels
 CPU_SAMPLE = {"c3v_batched": ((20, 21), 2), "c2v_plain": ((9, 10), 8),
               "c2v_small": ((0, 1), 4), "c3v_small": ((1, 2), 4)}
-# DRAM traffic of the half-line-strength split GEMM from one ncu capture of its
-# first K segment (K = 2048) on a small case of the same Nvib (profiles/):
-# bytes read per Y column per K element (the digit planes streamed past the
-# tiles) and bytes written per Y column (Z).  A job's K runs in segments of
-# 2048; each later segment re-reads Z to add to it.
-SPLIT_HALFLS_TRAFFIC = {3000: {"read_per_col_k": 44108294656 / (47904 * 2048),
-                               "write_per_col": 4468934656 / 47904,
-                               "capture": "c3v_batched J <= 8, 47904 Y columns, K = 2048"}}
 
 
 def parse(argv=None):
@@ -85,7 +77,7 @@ def parse(argv=None):
                     help="batches per job (a step is one batch); default 10 for c3v_batched")
     ap.add_argument("--precision", default="split", choices=["fp64", "split"])
     ap.add_argument("--seed", type=int, default=1)
-    ap.add_argument("--slices", type=int, default=0, help="bf16 digits per operand (split)")
+    ap.add_argument("--slices", type=int, default=0, help="split: 0 eleven e4m3 digits per operand, 2..10 bf16 digits")
     ap.add_argument("--e2e-steps", type=int, default=2, help="e2e steps (whole jobs)")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-cpu-baseline", action="store_true")
@@ -449,50 +441,48 @@ class Timer:
         return a.elapsed_time(b) * 1e-3, out
 
 
-def split_roofline(prob, ps, peaks):
+def split_roofline(prob, ps, peaks, slices):
     """The dominant kernel of the split path: the half-line-strength digit GEMM
-    (k_split_gemm_g, one launch per round)."""
+    (one launch per round).  The default scheme's flops are the digit products
+    that its symmetries and the dipole's zero planes leave; its MMAs are 8-bit,
+    twice the rate of bf16 ones."""
     sp, lp = ps["seconds_phase"], ps["launches_phase"]
     dom = "halfls_gemm"
-    pairs = ps["flops_tensor"] / max(ps["flops_halfls"] + ps["flops_final"], 1.0)
-    flops = pairs * ps["flops_halfls"]
+    e4m3 = slices == 0
+    kp = -(-prob.N // 64) * 64
+    if e4m3:
+        kernel, elem, rate = "k_split8 (tcgen05 e4m3 digit GEMM, half line strength)", 11, 2.0
+        flops = ps["flops_tensor"] - 66.0 * ps["flops_final"]
+    else:
+        kernel, elem, rate = "k_split_gemm_g (tcgen05 bf16 digit GEMM, half line strength)", \
+            2 * slices, 1.0
+        flops = ps["flops_tensor"] / max(ps["flops_halfls"] + ps["flops_final"], 1.0) \
+            * ps["flops_halfls"]
     ncol = ps["flops_halfls"] / (6.0 * prob.N * prob.N)
-    peak = peaks.get("bf16_tflops", 1900.0)
+    peak = rate * peaks.get("bf16_tflops", 1900.0)
     achieved = flops / sp[dom] / 1e12 if sp[dom] else 0.0
-    tr = SPLIT_HALFLS_TRAFFIC.get(prob.N)
-    traffic = None
-    if tr:
-        kp = -(-prob.N // 64) * 64
-        nseg = -(-kp // 2048)
-        step_bytes = ncol * (tr["read_per_col_k"] * kp + tr["write_per_col"] * (2 * nseg - 1))
-        traffic = step_bytes / max(lp[dom], 1)
-    algo = ncol * (9 * 2 * (-(-prob.N // 64) * 64) + 3 * prob.N * 8) / max(lp[dom], 1)
-    return {"bound": "tensor", "kernel": "k_split_gemm_g (tcgen05 bf16 digit GEMM, grouped digit "
-                                         "layout, half line strength)",
+    algo = ncol * (elem * kp + 3 * prob.N * 8) / max(lp[dom], 1)
+    return {"bound": "tensor", "kernel": kernel,
             "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-            "traffic": traffic,
-            "traffic_source": (f"ncu dram__bytes_read+write of this kernel on {tr['capture']}, "
-                               "scaled to the launch by Y columns and K (reads) and by Y columns "
-                               "(writes, and the re-read of Z by later K segments)")
-            if tr else "not captured for this Nvib",
+            "traffic": None,
+            "traffic_source": "not captured at this size (the operands' slices come from L2)",
             "algorithmic_bytes_per_launch": algo,
-            "algorithmic_bytes_meaning": "Y digit planes (9 x 2 B x Kp per column) read once and "
+            "algorithmic_bytes_meaning": f"Y digits ({elem} B x Kp per column) read once and "
                                          "Z (3 x N doubles per column) written once, per launch "
-                                         "averaged over the step's launches; the dipole's digit "
-                                         "planes (0.5 GB) are re-read per L2 raster group",
-            "achieved_meaning": "bf16 tensor-pipe rate: digit-pair products x 2 x M x N x K",
+                                         "averaged over the step's launches; the dipole's digits "
+                                         "are re-read per L2 raster group",
+            "achieved_meaning": "digit products executed x 2 x M x N x K ÷ device time",
             "tensor_tflop_per_launch": flops / max(lp[dom], 1) / 1e12,
-            "digit_pair_products": pairs,
+            "digit_pair_products": flops / max(ps["flops_halfls"], 1.0),
             "fp64_equivalent_tflops": ps["flops_halfls"] / sp[dom] / 1e12 if sp[dom] else 0.0,
             "fp64_algorithmic_tflop_per_launch": ps["flops_halfls"] / max(lp[dom], 1) / 1e12,
             "both_gemms_tflops": ps["flops_tensor"] / (sp["halfls_gemm"] + sp["final_gemm"]) / 1e12,
-            "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)"
-            if "bf16_tflops" in peaks else "fallback 1.9 PFLOP/s",
+            "peak_source": ("MEASURED_PEAKS.json bf16_tflops (of measured)"
+                            if "bf16_tflops" in peaks else "fallback 1.9 PFLOP/s")
+            + (", twice: 8-bit MMAs" if e4m3 else ""),
             "phase_seconds": {k: round(v, 6) for k, v in sp.items()},
             "phase_launches": lp, "launch_avg_ms": 1e3 * sp[dom] / max(lp[dom], 1),
-            "launch_unit": "one round's half-ls GEMM: its K segments (2048, then the rest) as "
-                           "consecutive kernel launches; achieved, traffic and launch_avg_ms "
-                           "are per such launch"}
+            "launch_unit": "one round's half-ls GEMM; achieved and launch_avg_ms are per launch"}
 
 
 # ---------------------------------------------------------------- legs
@@ -552,9 +542,9 @@ def leg_c2v_precision(pkg, args, device, timer_of):
 def leg_half_ls(pkg, args, device, timer_of, peaks):
     """The kernel-level drop-in for do_1st_half_ls (gi_half_ls): the half line
     strength of one initial vector of C2v J = 10 (Nvib = 2000, 22 (k, tau)
-    slots) towards J = 10, per call.  The split path is one pass over the
-    dipole's digit planes (the narrow digit GEMM, K split over the SMs); the
-    FP64 path is the DMMA GEMM."""
+    slots) towards J = 10, per call.  The split path reads the digits of the
+    dipole blocks that the vector's symmetries meet (K split over the SMs); the
+    FP64 path multiplies the dipole by the vector's non-zero Y values alone."""
     import torch
     prob = make_problem(args, workload="c2v_plain", jlist=[9, 10])
     blk = prob.blocks[(10, 0)]
@@ -562,7 +552,7 @@ def leg_half_ls(pkg, args, device, timer_of, peaks):
     N = prob.N
     Kp = -(-N // 64) * 64
     Mpad = -(-N // 128) * 128
-    digit_bytes = 3 * Mpad * Kp * 9 * 2
+    digit_bytes = 3 * Mpad * Kp * 11
     out = {"workload": f"gi_half_ls: one C2v J=10 vector (nsize {blk.nsize}) towards J=10, Nvib={N}",
            "dipole_fp64_bytes": 3 * N * N * 8, "dipole_digit_bytes": digit_bytes}
     for name, prec in (("split", pkg.GI_PREC_SPLIT), ("fp64", pkg.GI_PREC_FP64)):
@@ -576,12 +566,9 @@ def leg_half_ls(pkg, args, device, timer_of, peaks):
             k = 20
             dt, _ = timer(k, lambda i: eng.half_ls(10, 0, 0, 10, blk.vecs[i % blk.nvec], DF))
             per = dt / k
-            r = {"us_per_call": 1e6 * per, "calls": k,
-                 "note": "device time per call on the engine's stream (Y build, GEMM, stencil, "
-                         "copies of the vector and the result)"}
-            if name == "split":
-                r["digit_gb_per_s_whole_call"] = digit_bytes / per / 1e9
-            out[name] = r
+            out[name] = {"us_per_call": 1e6 * per, "calls": k,
+                         "note": "device time per call on the engine's stream (Y build, GEMM, "
+                                 "stencil, copies of the vector and the result)"}
     out["speedup_split_over_fp64"] = out["fp64"]["us_per_call"] / out["split"]["us_per_call"]
     return out
 
@@ -685,7 +672,8 @@ def main_ours(args):
         for line in open(tune_path).read().splitlines():
             s_, nA, nb, K, layout, kind, ga, ms = line.split()
             autotune.append({"digits": int(s_), "row_tiles": int(nA), "cols_bucket": 2 ** int(nb),
-                             "K": int(K), "kernel": names.get(kind, kind), "l2_group_mb": int(ga),
+                             "K": int(K), "kernel": "k_split8" if s_ == "11" else names.get(kind, kind),
+                             "l2_group_mb": int(ga),
                              "ms": float(ms)})
 
     with ClockSampler(local) as clk:
@@ -709,7 +697,7 @@ def main_ours(args):
     except OSError:
         pass
     if args.precision == "split":
-        roof = split_roofline(prob, ps, peaks)
+        roof = split_roofline(prob, ps, peaks, args.slices)
     else:
         sp, lp = ps["seconds_phase"], ps["launches_phase"]
         fp64_peak = pkg.measure_fp64_peak(local)  # TFLOP/s, DMMA m8n8k4, measured live
@@ -830,10 +818,12 @@ def main_ours(args):
                "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
                "ms_per_step": 1e3 * dt / args.steps, "wall_ms_per_step": 1e3 * wall,
                "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-               "dtype": "split-bf16x9" if args.precision == "split" and args.slices in (0, 9)
-               else (f"split-bf16x{args.slices}" if args.precision == "split" else "f64"),
-               "dtype_note": "bf16 digit products with exact integer accumulation, FP64 "
-                             "epilogue (S, A, I, filters in FP64)" if args.precision == "split"
+               "dtype": ("split-e4m3x11" if args.slices == 0 else f"split-bf16x{args.slices}")
+               if args.precision == "split" else "f64",
+               "dtype_note": ("e4m3" if args.slices == 0 else "bf16")
+               + " digit products (55 bits an operand by default) with exact integer "
+                 "accumulation, FP64 epilogue (S, A, I, filters in FP64)"
+               if args.precision == "split"
                else "FP64 throughout",
                "data": "synthetic", "config": cfg,
                "lines_per_step": lines_pre / args.steps,

@@ -1,4 +1,6 @@
-// Split-precision GEMMs on the tcgen05 tensor pipe (sm_103a).
+// Split-precision GEMMs on the tcgen05 tensor pipe (sm_103a): explicit digit counts
+// (split_slices 2..10) and the forced kernels; the default scheme is split8.cu's,
+// to which the entry points here dispatch.
 //
 // C[z][n*ldc + m] = sum_k A[z][m][k] * B[n][k] in FP64 accuracy from bf16
 // tensor-core products (an Ozaki-style error-free splitting):
