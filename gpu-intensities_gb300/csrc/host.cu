@@ -2438,11 +2438,12 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   int32_t* err_word = reinterpret_cast<int32_t*>(c->hls_pin + (c->hls_pin_cap - 1));
   // In the default split scheme a small vector's product goes through FP64,
   // which is more accurate, needs no digits of the dipole and, with Y packed to
-  // its non-zero values, is faster up to about 25 million products: 32 million
-  // (C2v, N = 1017, J = 10) took 101 us a call against 92 with digits, 5 million
-  // (N = 555, J = 5) 51 against 68.
+  // its non-zero values, is as fast or faster up to about 8 million products (its
+  // first call has no digits to cut).  Microseconds a call in FP64 and with
+  // digits, C2v: N = 555, J = 10 66, 68; 1017, 5 68, 72; 777, 10 (9 million) 80, 81;
+  // 2000, 2 (12 million) 104, 69; 1017, 10 97, 85; 1200, 10 (22 million) 138, 80.
   const bool small =
-      split8_selected(c) && 3.0 * c->N * (double)bI.y_nnz[gammaI] <= (double)(3 << 23);
+      split8_selected(c) && 3.0 * c->N * (double)bI.y_nnz[gammaI] <= (double)(1 << 23);
   const bool split_path =
       c->have_params && c->params.precision == GI_PREC_SPLIT && !c->streamed() && !small;
   if (split_path) {
