@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/gi.h"
+#include "zlayout.h"
 
 namespace gi {
 
@@ -291,6 +292,9 @@ struct JobSel {
   double zpe = 0.0;
   int jmin = 0, jmax = 0;
   double qstat = 0.0;  // partition function of the whole job (when QSTAT <= 0)
+  // the largest final block that jobs of this initial block have: the cut into
+  // rounds (and with it the layout of Z) is the same for all of them
+  FinalSize final;
 };
 
 struct Ctx {
@@ -470,10 +474,11 @@ gi_status refresh_pair_tables(Ctx* c, Basis* only = nullptr);
 // other than `keep` and unused cached half line strengths (least recently
 // used first).  Caller holds model_mu.
 gi_status server_make_room(Ctx* c, size_t bytes, Block* keep);
-// Serving Z cache: the half line strength Z = mu^T Y ([3][ncol][Kp], the run's
-// layout) of an initial block for one selection of its vectors.  acquire
-// (worker context, model lock not held) returns z = null when nothing can be
-// cached; hit: z holds it, else the run writes it there.  release unpins it,
+// Serving Z cache: the half line strength Z = mu^T Y of an initial block for one
+// selection of its vectors, in the run's layout.  An entry serves a job only
+// when its layout is the job's.  acquire (worker context, model lock not held)
+// returns z = null when nothing can be cached; hit: z holds it, else the run
+// writes it there.  release unpins it,
 // keeping it valid after a successful run or dropping it otherwise.
 struct ZEntry;
 struct ZRef {
@@ -482,8 +487,8 @@ struct ZRef {
   bool hit = false;
 };
 // gF: the final symmetry whose rows of Z the run computes (-1: every row).
-gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, size_t elems,
-                         int gF, ZRef* out);
+gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI,
+                         const ZLayout& layout, int gF, ZRef* out);
 void zcache_release(Ctx* w, ZRef& r, bool ok);
 // Stops the serving loop of c (if any): fails queued jobs, joins the workers.
 gi_status server_stop(Ctx* c);

@@ -704,11 +704,11 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     size_t per_vec = (size_t)ndegI * nslot * per_col;
     for (auto* pp : mine) {
       const Block& fb = *pp->F->blk;
-      per_vec += (size_t)ndegI * c->degen[fb.gamma] *
-                 (fb.ld * (8 + digit_bytes) + round_up(fb.nvec, 2) * 8);
+      FinalSize f{fb.ld, fb.nvec};
+      if (c->job.on) f = larger(f, c->job.final);
+      per_vec += (size_t)ndegI * c->degen[fb.gamma] * final_col_bytes(f, digit_bytes);
     }
-    const int chunk =
-        (int)std::min<size_t>(std::max<size_t>(1, ws_limit / per_vec), I.ivec.size());
+    const int chunk = unit_vectors(ws_limit, per_vec, I.ivec.size());
     for (int i0 = 0; i0 < (int)I.ivec.size(); i0 += chunk) {
       const int nI = std::min(chunk, (int)I.ivec.size() - i0);
       if (round_bytes + per_vec * nI > ws_limit && !rounds.back().units.empty()) {
@@ -1132,7 +1132,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   // A serving pair job (one initial block, one unit per round): the half line
   // strength Z of its initial block may come from (or go to) the server's Z
   // cache, shared by every job with the same initial block and selection of
-  // its vectors.  The entry holds the block's whole Z ([3][columns][Kp]); round
+  // its vectors.  The entry holds the block's whole Z ([3][columns][ldz]); round
   // r reads and writes its columns from zoff[r] on.
   ZRef zref;
   std::vector<size_t> zoff(rounds.size(), 0);
@@ -1140,6 +1140,7 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   if (c->job.on && c->parent && !c->streamed()) {
     bool one = true;
     std::vector<int32_t> ids;
+    ZLayout zl;
     const Block* zblk = nullptr;
     for (size_t r = 0; r < rounds.size() && one; r++) {
       if (rounds[r].units.empty()) continue;
@@ -1149,9 +1150,13 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
       zoff[r] = ztotal;
       ztotal += rounds[r].ncolZ;
       ids.insert(ids.end(), h_ivec.begin() + 2 * u.off, h_ivec.begin() + 2 * u.off + u.nI);
+      if (vib) zl.cut.push_back(u.nI);
     }
     if (one && zblk && ztotal) {
-      gi_status s = zcache_acquire(c, zblk, ids.data(), (int)ids.size(), 3 * ztotal * ldz,
+      zl.order = vib ? vp->uid : 0;
+      zl.ldz = ldz;
+      zl.ncol = ztotal;
+      gi_status s = zcache_acquire(c, zblk, ids.data(), (int)ids.size(), zl,
                                    vib ? c->job.gF : -1, &zref);
       if (s != GI_OK) return s;
     }

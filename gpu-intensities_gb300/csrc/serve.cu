@@ -54,6 +54,7 @@ struct ZEntry {
   uint64_t blk_uid = 0, blk_version = 0;
   int precision = 0, slices = 0;
   int gF = -1;                // the final symmetry it serves (-1: any)
+  ZLayout layout;
   std::vector<int32_t> ivec;  // the initial records its columns hold
   DevArray<double> z;
   bool valid = false;         // written by a finished run
@@ -187,8 +188,8 @@ gi_status server_make_room(Ctx* c, size_t bytes, Block* keep) {
 }
 
 // ------------------------------------------------------------------ Z cache
-gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, size_t elems,
-                         int gF, ZRef* out) {
+gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI,
+                         const ZLayout& layout, int gF, ZRef* out) {
   *out = ZRef{};
   Ctx* c = w->parent;
   Server* s = c ? c->server : nullptr;
@@ -198,8 +199,8 @@ gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, 
   for (size_t k = 0; k < s->zcache.size(); k++) {
     ZEntry& e = *s->zcache[k];
     if (e.blk_uid != blk->uid || e.blk_version != blk->version || e.precision != prec ||
-        e.slices != sl || e.gF != gF || (int)e.ivec.size() != nI ||
-        !std::equal(e.ivec.begin(), e.ivec.end(), ivec))
+        e.slices != sl || e.gF != gF || !(e.layout == layout) || e.z.n != layout.elems() ||
+        (int)e.ivec.size() != nI || !std::equal(e.ivec.begin(), e.ivec.end(), ivec))
       continue;
     if (!e.valid) {
       // another job is computing it: its end (or its failure, which drops the
@@ -218,7 +219,7 @@ gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, 
   // and takes at most a quarter of it (one large entry would push out many
   // small ones that are asked for more often)
   s->z_misses++;
-  const size_t bytes = elems * sizeof(double);
+  const size_t bytes = layout.elems() * sizeof(double);
   if (bytes > block_budget(s) / 4) return GI_OK;
   if (server_make_room(c, bytes, nullptr) != GI_OK) {
     c->err.clear();
@@ -230,8 +231,9 @@ gi_status zcache_acquire(Ctx* w, const Block* blk, const int32_t* ivec, int nI, 
   e->precision = prec;
   e->slices = sl;
   e->gF = gF;
+  e->layout = layout;
   e->ivec.assign(ivec, ivec + nI);
-  if (e->z.alloc(elems) != cudaSuccess) {
+  if (e->z.alloc(layout.elems()) != cudaSuccess) {
     cudaGetLastError();
     return GI_OK;
   }
@@ -339,7 +341,12 @@ static void worker_main(Server* s, int slot) {
     w->threej = c->threej;
     w->threej_jmax = c->threej_jmax;
     w->threej_user = c->threej_user;
-    w->job = JobSel{true, j->jI, j->gI, j->jF, j->gF, j->zpe, j->jmin, j->jmax, j->qstat};
+    w->job = JobSel{true, j->jI, j->gI, j->jF, j->gF, j->zpe, j->jmin, j->jmax, j->qstat, {}};
+    for (int jF = j->jI - 1; jF <= j->jI + 1; jF++) {
+      auto it = c->blocks.find({jF, j->gF});
+      if (it != c->blocks.end())
+        w->job.final = larger(w->job.final, FinalSize{it->second->ld, it->second->nvec});
+    }
     lk.unlock();
     int64_t n = 0;
     std::string err;
