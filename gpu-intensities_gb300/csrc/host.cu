@@ -1110,10 +1110,12 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
               const double deg = ep.reduced && ep.ndegF != 1 && ep.ndegI != 1 ? 1.0
                                                                               : 1.0 / ep.ndegI;
               const double s_of_t = deg * ep.gns * (2 * ep.jI + 1) * (2 * ep.jF + 1);
-              e.lx_s = (float)(std::log2(std::max(ep.thresh_S, 1e-300)) - std::log2(s_of_t));
-              e.lx_i = (float)(std::log2(std::max(ep.thresh_I, 1e-300)) + std::log2(ep.avogno) +
-                               std::log2(ep.q_stat) - std::log2(s_of_t) -
-                               std::log2(ep.intens_cm_mol));
+              // a threshold among the smallest numbers is left to eval_line, whose
+              // S and I round there as no logarithm does
+              auto lg = [](double x) { return x < 1e-290 ? -HUGE_VAL : std::log2(x); };
+              e.lx_s = (float)(lg(ep.thresh_S) - std::log2(s_of_t));
+              e.lx_i = (float)(lg(ep.thresh_I) + std::log2(ep.avogno) + std::log2(ep.q_stat) -
+                               std::log2(s_of_t) - std::log2(ep.intens_cm_mol));
               e.l_err = (float)(1.0 + std::log2(ep.err_coef) + std::log2((double)g));
               e.beta = (float)ep.beta;
             }
