@@ -347,6 +347,9 @@ struct Ctx {
   gi_line_compact* h_compact = nullptr;
   size_t h_compact_cap = 0;
   int64_t nlines = 0;
+  // levels that d_lines's level ids count from (0: a run has begun since and
+  // did not end, d_lines and levels are not those of the nlines lines)
+  int lines_nlev = 0;
   // gi_sort_lines: ordered copy and tables (kept up to kSortKeep bytes)
   static constexpr size_t kSortKeep = (size_t)256 << 20;
   DevArray<uint8_t> w_mask;  // set_basis: symmetries of the roots
