@@ -1725,13 +1725,13 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
   }
   const unsigned long long count = counts[0];
   if (count > c->d_lines.n) return fail(c, GI_ERR_DEVICE, "line buffer overflow (%llu lines)", count);
-  c->nlines = (int64_t)count;
   if (!c->lines_on_device && count) {
     gi_status s = host_room(count, copied);
     if (s == GI_OK) s = read_back(copied, count, overlap_d2h ? c->d2h : c->stream);
     if (s != GI_OK) return s;
     GI_CUDA(c, cudaStreamSynchronize(overlap_d2h ? c->d2h : c->stream));
   }
+  c->nlines = (int64_t)count;  // the caller's lines are all there
   float ms = 0.f;
   GI_CUDA(c, cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   for (const auto& r : c->phase_recs) {
