@@ -991,7 +991,10 @@ gi_status run_job(Ctx* c, int flags, int64_t* nlines_out) {
     mixv(grouped_final);
     mixv(fused_y);
     if (P.precision == GI_PREC_SPLIT) mixv(split_identity(c));
-    if (vib) mixv(vp->uid);
+    if (vib) {
+      mixv(vp->uid);
+      mixv(vib_rowsrc(c, 0));  // made again, maybe elsewhere, when the dipole was streamed
+    }
     for (size_t r = 0; r < rounds.size(); r++) {
       mixv(rounds[r].ncolY);
       for (const Unit& u : rounds[r].units) {
