@@ -276,13 +276,15 @@ gi_status ensure_y_table(Ctx* c, Basis& b, int g) {
   b.d_yc.resize(c->nrep);
   if (b.d_ys[g].p) return GI_OK;
   const size_t n = (size_t)b.root_ent[g] * b.y_mult * b.nslot * c->N;
-  GI_CUDA(c, b.d_yc[g].alloc(c->degen[g] * n));
-  GI_CUDA(c, b.d_ys[g].alloc(n));
-  const cudaError_t e = launch_y_table(b, g, c->degen[g], c->N, b.root_ent[g] * b.y_mult,
-                                       b.d_ys[g].p, b.d_yc[g].p, cudaStreamLegacy);
-  if (e == cudaSuccess) GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
-  if (e != cudaSuccess) b.d_ys[g].reset();
-  GI_CUDA(c, e);
+  DevArray<int32_t> ys;
+  DevArray<double> yc;
+  GI_CUDA(c, yc.alloc(c->degen[g] * n));
+  GI_CUDA(c, ys.alloc(n));
+  GI_CUDA(c, launch_y_table(b, g, c->degen[g], c->N, b.root_ent[g] * b.y_mult, ys.p, yc.p,
+                            cudaStreamLegacy));
+  GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
+  b.d_yc[g] = std::move(yc);
+  b.d_ys[g] = std::move(ys);
   return GI_OK;
 }
 
@@ -1793,9 +1795,12 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
   gi_status s;
   const VibPlan* vp = vib_plan(c, &s);
   if (!vp) return s;
-  for (Basis* b : {&bI, &bF})
-    if ((s = ensure_root_z(c, *b, *vp)) != GI_OK) return s;
-  if ((s = ensure_y_table(c, bI, gammaI)) != GI_OK) return s;
+  {
+    std::lock_guard<std::mutex> lk(c->mmu());  // serving workers make them too
+    for (Basis* b : {&bI, &bF})
+      if ((s = ensure_root_z(c, *b, *vp)) != GI_OK) return s;
+    if ((s = ensure_y_table(c, bI, gammaI)) != GI_OK) return s;
+  }
   const int ldz = vp->ldz;
   auto& plans = c->hls_plans8;
   auto sig_of = [&] {
@@ -2412,10 +2417,11 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   cudaSetDevice(c->device);
   Basis& bI = *iI->second;
   Basis& bF = *iF->second;
-  gi_status s = ensure_ycsr(c, bI);
-  if (s != GI_OK) return s;
-  s = ensure_ycsr(c, bF);
-  if (s != GI_OK) return s;
+  gi_status s;
+  {
+    std::lock_guard<std::mutex> lk(c->mmu());
+    if ((s = ensure_ycsr(c, bI)) != GI_OK || (s = ensure_ycsr(c, bF)) != GI_OK) return s;
+  }
   const int jmax = std::max(jI, jF);
   if (c->threej_jmax < jmax) {
     const bool was_user = c->threej_user;
