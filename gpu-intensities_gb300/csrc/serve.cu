@@ -454,8 +454,8 @@ gi_status gi_serve_start(gi_ctx* h, const gi_serve_config* cfg) {
                 slot_ws);
   // the order of the vibrational functions and the dipole digits are made once,
   // before any worker runs
+  const VibPlan* vp;
   {
-    const VibPlan* vp;
     gi_status st = vib_prepare(c, &vp);
     if (st != GI_OK) return st;
   }
@@ -468,6 +468,21 @@ gi_status gi_serve_start(gi_ctx* h, const gi_serve_config* cfg) {
     for (auto& kv : c->bases) {
       gi_status st = ensure_ycsr(c, *kv.second);
       if (st != GI_OK) return st;
+    }
+    // the tables that jobs from the loaded blocks read (a block that comes later
+    // has its own made by its first job)
+    if (c->params.precision == GI_PREC_FP64 || split8_selected(c)) {
+      for (auto& kv : c->bases) {
+        gi_status st = ensure_root_z(c, *kv.second, *vp);
+        if (st != GI_OK) return st;
+      }
+      for (auto& kv : c->blocks) {
+        const Block& b = *kv.second;
+        auto it = c->bases.find(b.J);
+        if (it == c->bases.end() || b.nvec == 0 || !(c->params.gns[b.gamma] > 0.0)) continue;
+        gi_status st = ensure_y_table(c, *it->second, b.gamma);
+        if (st != GI_OK) return st;
+      }
     }
     const int jmax = c->bases.rbegin()->first;
     if (c->threej_jmax < jmax) {
