@@ -218,6 +218,10 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
   const int32_t* ent = reinterpret_cast<const int32_t*>(h.data());
   b.root_ent.assign(ent, ent + nrep);
   const uint8_t* mask = h.data() + 4 * GI_MAX_REP;
+  b.y_nnz.assign(nrep, 0);
+  // an index that no dipole reaches (N of a million takes 24 TB): the calls that
+  // need the functions refuse the basis, and nothing is sized by it here
+  if (b.iroot_max >= (1 << 20)) return GI_OK;
   std::vector<uint8_t> use((size_t)(b.iroot_max + 1) * b.nslot, 0);
   b.v_kind.assign((size_t)b.iroot_max + 1, -1);
   for (int r = 0; r < D; r++) {
@@ -236,7 +240,6 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
   std::vector<int64_t> of_kind(b.nkind, 0);
   for (int kind : b.v_kind)
     if (kind >= 0) of_kind[kind]++;
-  b.y_nnz.assign(nrep, 0);
   for (int k = 0; k < b.nkind; k++)
     for (int slot = 0; slot < b.nslot; slot++)
       for (unsigned m = b.kind_mask[(size_t)k * b.nslot + slot]; m; m &= m - 1)
