@@ -8,10 +8,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "engine.h"
+#include "once.h"
 
 namespace gi {
 
@@ -234,15 +234,18 @@ cudaError_t launch_gemm_f64(std::vector<ProbF> probs, cudaStream_t s) {
 }
 
 static cudaError_t attributes() {
-  static std::once_flag once;
-  static cudaError_t status = cudaSuccess;
-  std::call_once(once, [] {
-    status = cudaFuncSetAttribute(k_pack_y, cudaFuncAttributeMaxDynamicSharedMemorySize, kPackSmem);
-    if (status == cudaSuccess)
-      status = cudaFuncSetAttribute(k_dipole_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kPackSmem);
+  static OncePerDevice once;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return once.run(device, [] {
+    const cudaError_t a =
+        cudaFuncSetAttribute(k_pack_y, cudaFuncAttributeMaxDynamicSharedMemorySize, kPackSmem);
+    return a != cudaSuccess
+               ? a
+               : cudaFuncSetAttribute(k_dipole_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kPackSmem);
   });
-  return status;
 }
 
 cudaError_t launch_pack_y(double* Y, int nslot, int N, int Kp, int32_t* count, cudaStream_t s) {

@@ -50,6 +50,7 @@
 #include "split8.h"
 #include "epilogue.cuh"
 #include "items.cuh"
+#include "once.h"
 #include "tc.cuh"
 #include "../../include/gi_probe.h"
 
@@ -1673,12 +1674,14 @@ cudaError_t set_smem(F a, size_t bytes, F b) {
 template <int S>
 cudaError_t set_attributes() {
   constexpr int BN1 = bn_for(S), BN2 = bn2_of(S), D1 = d1_of(S);
-  static std::once_flag once;
-  static cudaError_t status = cudaSuccess;
-  std::call_once(once, [] {
-    status = cudaFuncSetAttribute(k_split_gemm<S, BN1>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem_bytes(S, BN1));
+  static OncePerDevice once;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return once.run(device, [] {
+    cudaError_t status = cudaFuncSetAttribute(k_split_gemm<S, BN1>,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)smem_bytes(S, BN1));
     if (status == cudaSuccess)
       status = cudaFuncSetAttribute(k_split_gemm2<S, BN2, D1>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1716,8 +1719,8 @@ cudaError_t set_attributes() {
                                         (int)(kFusedYMaxKp * sizeof(double)));
       }
     }
+    return status;
   });
-  return status;
 }
 
 cudaError_t kernel_attributes(int s) {

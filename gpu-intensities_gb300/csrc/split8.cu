@@ -38,6 +38,7 @@
 
 #include "epilogue.cuh"
 #include "items.cuh"
+#include "once.h"
 #include "split8.h"
 #include "tc.cuh"
 
@@ -778,16 +779,18 @@ __global__ void __launch_bounds__(256) k_build_y8(const YItem8* __restrict__ ite
 constexpr int kYSmem = 200 * 1024;  // longest cached row: 25,600 functions
 
 cudaError_t attributes8() {
-  static std::once_flag once;
-  static cudaError_t status = cudaSuccess;
-  std::call_once(once, [] {
-    status = cudaFuncSetAttribute(k_split8, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kSmem);
-    if (status == cudaSuccess)
-      status = cudaFuncSetAttribute(k_build_y8<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kYSmem);
+  static OncePerDevice once;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return once.run(device, [] {
+    const cudaError_t a =
+        cudaFuncSetAttribute(k_split8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
+    return a != cudaSuccess
+               ? a
+               : cudaFuncSetAttribute(k_build_y8<true>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, kYSmem);
   });
-  return status;
 }
 
 }  // namespace
