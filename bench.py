@@ -352,10 +352,13 @@ def serve_stream(pkg, pool, jobs, gaps, device, precision, args):
                                 return
                     time.sleep(0.001)
                     continue
-                info = eng.wait(nxt, check=False)
-                if info["state"] != pkg.GI_JOB_DONE:
-                    errors.append(info["status"])
-                eng.release(nxt)
+                try:
+                    info = eng.wait(nxt, check=False)
+                    if info["state"] != pkg.GI_JOB_DONE:
+                        errors.append(f"status {info['status']}")
+                    eng.release(nxt)
+                except Exception as e:  # the thread goes on: every job is waited for
+                    errors.append(repr(e))
                 k += 1
 
         th = threading.Thread(target=reap, daemon=True)
@@ -375,8 +378,10 @@ def serve_stream(pkg, pool, jobs, gaps, device, precision, args):
         makespan = time.perf_counter() - t0
         st = eng.serve_stats()
         eng.serve_stop()
+    if errors or st["failed"]:
+        raise RuntimeError(f"{max(len(errors), st['failed'])} of {len(jobs)} serving jobs failed"
+                           + (f", the first with {errors[0]}" if errors else ""))
     st["makespan_s"] = makespan
-    st["reaped_failures"] = len(errors)
     return st
 
 
@@ -420,6 +425,28 @@ def serving_leg(pkg, args, device, base):
 
 
 # ---------------------------------------------------------------- helpers
+class Legs:
+    """Runs the workloads beside the headline.  One that fails is an error in the
+    line, not the loss of what was measured; after an error of the device the
+    rest is not run."""
+
+    def __init__(self, pkg):
+        self.pkg, self.dead = pkg, None
+
+    def __call__(self, name, fn, *a):
+        if self.dead:
+            return {"error": f"not run: {self.dead}"}
+        try:
+            return fn(*a)
+        except Exception as e:
+            import traceback
+            traceback.print_exc()
+            if isinstance(e, self.pkg.GiError) and e.status in (self.pkg.GI_ERR_CUDA,
+                                                               self.pkg.GI_ERR_DEVICE):
+                self.dead = f"the device failed in {name}"
+            return {"error": f"{type(e).__name__}: {e}"}
+
+
 class Timer:
     """Device seconds of a callable's launches: CUDA events on the engine's
     stream, bracketed by synchronize and a barrier across ranks."""
@@ -786,9 +813,10 @@ def main_ours(args):
                          f"final level)", "fp64": res["fp64"], "split": res["split"],
                 "speedup_split_over_fp64": res["split"]["value"] / res["fp64"]["value"]}
 
+    run_leg = Legs(pkg)
     streamed = None
     if not args.no_legs and "streamed" in args.legs and world == 1:
-        streamed = leg_streamed(pkg, eng, prob, timer, S, value_rate)
+        streamed = run_leg("streamed", leg_streamed, pkg, eng, prob, timer, S, value_rate)
     eng.close()
     # the serving pool reuses the headline's dipole and bases (blocks regenerated)
     serve_base = None
@@ -801,16 +829,18 @@ def main_ours(args):
     legs = {}
     if not args.no_legs and world == 1:
         if "plain" in args.legs and args.workload != "c2v_plain":
-            legs["c2v_plain"] = leg_c2v_plain(pkg, args, local, timer_of)
+            legs["c2v_plain"] = run_leg("c2v_plain", leg_c2v_plain, pkg, args, local, timer_of)
         if "precision" in args.legs and args.workload != "c2v_precision":
-            legs["c2v_precision"] = leg_c2v_precision(pkg, args, local, timer_of)
+            legs["c2v_precision"] = run_leg("c2v_precision", leg_c2v_precision, pkg, args, local,
+                                            timer_of)
         if "serving" in args.legs:
-            legs["serving"] = serving_leg(pkg, args, local, serve_base)
+            legs["serving"] = run_leg("serving", serving_leg, pkg, args, local, serve_base)
         if "halfls" in args.legs:
-            legs["half_ls_vector"] = leg_half_ls(pkg, args, local, timer_of, peaks)
+            legs["half_ls_vector"] = run_leg("half_ls_vector", leg_half_ls, pkg, args, local,
+                                             timer_of, peaks)
     accuracy = None
     if not args.no_accuracy and world == 1 and args.workload in CPU_SAMPLE:
-        accuracy = accuracy_vs_oracle(pkg, args, local, args.workload)
+        accuracy = run_leg("accuracy", accuracy_vs_oracle, pkg, args, local, args.workload)
 
     dt, lines_all, lines_all_post = across_ranks(dt, lines_pre, lines_post, "cuda")
     if rank == 0:
