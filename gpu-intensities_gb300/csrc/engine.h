@@ -470,7 +470,7 @@ double partition_sum(const Ctx* c, double temperature, double zpe);
 gi_status run_job(Ctx* c, int flags, int64_t* nlines_out);
 // Builds the (slot, v) -> roots table of a basis for the context's dipole size.
 gi_status ensure_ycsr(Ctx* c, Basis& b);
-gi_status ensure_y_table(Ctx* c, Basis& b, int g);
+gi_status ensure_y_table(Ctx* c, Basis& b, int g, bool* pending = nullptr);
 // Device tables of every basis's half-line-strength terms towards J-1, J, J+1
 // (Basis::d_pair_st), from the context's 3j table where it covers the pair.
 gi_status refresh_pair_tables(Ctx* c, Basis* only = nullptr);

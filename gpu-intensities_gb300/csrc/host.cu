@@ -247,16 +247,24 @@ static gi_status derive_basis(Ctx* c, Basis& b) {
   return GI_OK;
 }
 
+// The dipole covers the basis's functions.
+static gi_status check_functions(Ctx* c, const Basis& b) {
+  if (b.iroot_max < c->N) return GI_OK;
+  int r = 0;
+  while (b.iroot[r] < c->N) r++;
+  return fail(c, GI_ERR_ARG, "basis J=%d: iroot_correlat_j0[%d]=%d >= N=%d", b.J, r, b.iroot[r],
+              c->N);
+}
+
 // (slot, v) -> roots, once the dipole size N is known.
 gi_status ensure_ycsr(Ctx* c, Basis& b) {
   if (b.y_N == c->N) return GI_OK;
   const int N = c->N;
+  const gi_status s = check_functions(c, b);
+  if (s != GI_OK) return s;
   std::vector<int32_t> ptr((size_t)b.nslot * N + 1, 0), roots(b.D);
-  for (int r = 0; r < b.D; r++) {
-    if (b.iroot[r] >= N)
-      return fail(c, GI_ERR_ARG, "basis J=%d: iroot_correlat_j0[%d]=%d >= N=%d", b.J, r, b.iroot[r], N);
+  for (int r = 0; r < b.D; r++)
     ptr[(size_t)b.slot_of_key[b.root_key[r]] * N + b.iroot[r] + 1]++;
-  }
   b.y_mult = 0;
   for (size_t i = 0; i + 1 < ptr.size(); i++) {
     b.y_mult = std::max(b.y_mult, ptr[i + 1]);
@@ -273,8 +281,8 @@ gi_status ensure_ycsr(Ctx* c, Basis& b) {
 }
 
 // The basis's Y table of gamma for the default split scheme (after
-// ensure_ycsr, under the model lock).
-gi_status ensure_y_table(Ctx* c, Basis& b, int g) {
+// ensure_ycsr, under the model lock; pending: as for ensure_root_z).
+gi_status ensure_y_table(Ctx* c, Basis& b, int g, bool* pending) {
   b.d_ys.resize(c->nrep);
   b.d_yc.resize(c->nrep);
   if (b.d_ys[g].p) return GI_OK;
@@ -285,7 +293,10 @@ gi_status ensure_y_table(Ctx* c, Basis& b, int g) {
   GI_CUDA(c, ys.alloc(n));
   GI_CUDA(c, launch_y_table(b, g, c->degen[g], c->N, b.root_ent[g] * b.y_mult, ys.p, yc.p,
                             cudaStreamLegacy));
-  GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
+  if (pending)
+    *pending = true;
+  else
+    GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
   b.d_yc[g] = std::move(yc);
   b.d_ys[g] = std::move(ys);
   return GI_OK;
@@ -1798,12 +1809,17 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
   gi_status s;
   const VibPlan* vp = vib_plan(c, &s);
   if (!vp) return s;
-  {
-    std::lock_guard<std::mutex> lk(c->mmu());  // serving workers make them too
-    for (Basis* b : {&bI, &bF})
-      if ((s = ensure_root_z(c, *b, *vp)) != GI_OK) return s;
-    if ((s = ensure_y_table(c, bI, gammaI)) != GI_OK) return s;
-  }
+  // serving workers make the bases' tables too: the lock is held until those made
+  // here are filled, one wait for them and the plan's own
+  std::lock_guard<std::mutex> lk(c->mmu());
+  struct Filled {
+    bool pending = false;
+    ~Filled() {
+      if (pending) cudaStreamSynchronize(cudaStreamLegacy);
+    }
+  } filled;
+  if ((s = ensure_root_z(c, bF, *vp, &filled.pending)) != GI_OK) return s;
+  if ((s = ensure_y_table(c, bI, gammaI, &filled.pending)) != GI_OK) return s;
   const int ldz = vp->ldz;
   auto& plans = c->hls_plans8;
   auto sig_of = [&] {
@@ -1948,6 +1964,7 @@ static gi_status hls_plan8(Ctx* c, Basis& bI, Basis& bF, int gammaI, int ideg, H
   std::memcpy(blob.data() + sc_off, slotcol.data(), slotcol.size() * sizeof(int32_t));
   GI_CUDA(c, cudaMemcpy(hp->blob.p, blob.data(), total, cudaMemcpyHostToDevice));
   GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
+  filled.pending = false;
   hp->items = reinterpret_cast<const YItem8*>(hp->blob.p + it_off);
   hp->tile_item = reinterpret_cast<const int32_t*>(hp->blob.p + ti_off);
   hp->slotcol = reinterpret_cast<const int32_t*>(hp->blob.p + sc_off);
@@ -2423,20 +2440,19 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   gi_status s;
   {
     std::lock_guard<std::mutex> lk(c->mmu());
-    if ((s = ensure_ycsr(c, bI)) != GI_OK || (s = ensure_ycsr(c, bF)) != GI_OK) return s;
+    if ((s = ensure_ycsr(c, bI)) != GI_OK || (s = check_functions(c, bF)) != GI_OK) return s;
   }
   const int jmax = std::max(jI, jF);
-  if (c->threej_jmax < jmax) {
-    const bool was_user = c->threej_user;
+  // the rotational term tables towards jF are the basis's device tables; a caller's
+  // 3j table that does not cover the pair is replaced (the engine's own was never
+  // needed for them: 75 us of a first call at J = 10)
+  if (c->threej_user && c->threej_jmax < jmax) {
     precompute_threej(jmax, c->threej);
     c->threej_jmax = jmax;
     c->threej_user = false;
-    if (was_user) {
-      s = refresh_pair_tables(c);
-      if (s != GI_OK) return s;
-    }
+    s = refresh_pair_tables(c);
+    if (s != GI_OK) return s;
   }
-  // the rotational term tables towards jF are the basis's device tables
   const StencilTerm* dst = bI.d_pair_st[jF - jI + 1].p;
   const int32_t* dstn = bI.d_pair_stn[jF - jI + 1].p;
   if (!dst || !dstn) return fail(c, GI_ERR_STATE, "basis J=%d has no term tables", jI);
@@ -2446,8 +2462,10 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   const int ncol = bI.nslot;
   // grow-only workspaces of the context: repeated calls allocate nothing
   GI_CUDA(c, c->hls_v.reserve(ld));
-  if (!c->hls_iv.p) GI_CUDA(c, c->hls_iv.assign(std::vector<int32_t>{0}));  // the one vector's index
-  GI_CUDA(c, c->hls_y.reserve((size_t)ncol * c->Kp));
+  if (!c->hls_iv.p) {  // the one vector's index
+    GI_CUDA(c, c->hls_iv.reserve(1));
+    GI_CUDA(c, cudaMemsetAsync(c->hls_iv.p, 0, sizeof(int32_t), c->stream));
+  }
   GI_CUDA(c, c->hls_h.reserve(bF.D));
   // the vector and the result pass through pinned staging of the context;
   // one more slot receives the split GEMMs' device error word
@@ -2480,10 +2498,14 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   if (split_path && split8_active(c)) {
     s = hls_plan8(c, bI, bF, gammaI, ideg, &h8);
     if (s != GI_OK) return s;
-  } else if (split_path) GI_CUDA(c, c->hls_z.reserve((size_t)max_parts * ncol * ldz_max));
-  else {
-    GI_CUDA(c, c->hls_z.reserve((size_t)3 * ncol * c->Kp));
-    GI_CUDA(c, c->hls_cnt.reserve(ncol));
+  } else {
+    GI_CUDA(c, c->hls_y.reserve((size_t)ncol * c->Kp));
+    if (split_path) {
+      GI_CUDA(c, c->hls_z.reserve((size_t)max_parts * ncol * ldz_max));
+    } else {
+      GI_CUDA(c, c->hls_z.reserve((size_t)3 * ncol * c->Kp));
+      GI_CUDA(c, c->hls_cnt.reserve(ncol));
+    }
   }
   // the call's device work: the vector in, Y, the dipole GEMM, the stencil,
   // the result out (all on c->stream; capturable)

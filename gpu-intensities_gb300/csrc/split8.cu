@@ -932,12 +932,15 @@ std::vector<VibTile> split8_tiles(const VibPlan& vp, int f0, int rows) {
   return t;
 }
 
-gi_status ensure_root_z(Ctx* c, Basis& b, const VibPlan& vp) {
+gi_status ensure_root_z(Ctx* c, Basis& b, const VibPlan& vp, bool* pending) {
   if (b.z_uid == vp.uid) return GI_OK;
   const Split8* S = (c->parent ? c->parent : c)->split8;
   GI_CUDA(c, b.d_root_z.reserve(std::max(b.D, 1)));
   GI_CUDA(c, launch_root_z(b, S->zpos, b.d_root_z.p, cudaStreamLegacy));
-  GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
+  if (pending)
+    *pending = true;
+  else
+    GI_CUDA(c, cudaStreamSynchronize(cudaStreamLegacy));
   b.z_uid = vp.uid;
   return GI_OK;
 }

@@ -88,7 +88,9 @@ int32_t* split8_b_exp(Ctx* c);
 gi_status split8_build_y(Ctx* c, const YItem8* items, const int32_t* tile_item, int n,
                          long long blocks, bool digits = true);
 // Rows of Z of a basis's roots for the plan (after split_prepare, under the model lock).
-gi_status ensure_root_z(Ctx* c, Basis& b, const VibPlan& vp);
+// pending (or null): set when the table was launched on the legacy stream, for
+// which the caller then waits before it gives up the lock.
+gi_status ensure_root_z(Ctx* c, Basis& b, const VibPlan& vp, bool* pending = nullptr);
 // Classes a (basis, gamma, slot) has coefficients on; rows of Z that final
 // symmetry gF reads of component comp of an initial slot's columns (every final
 // J that the owner's bases allow).
