@@ -2484,6 +2484,8 @@ gi_status gi_half_ls(gi_ctx* h, int jI, int gammaI, int ideg, int jF, const doub
   // first call has no digits to cut).  Microseconds a call in FP64 and with
   // digits, C2v: N = 555, J = 10 66, 68; 1017, 5 68, 72; 777, 10 (9 million) 80, 81;
   // 2000, 2 (12 million) 104, 69; 1017, 10 97, 85; 1200, 10 (22 million) 138, 80.
+  // C3v: 420, 5 (5 million) 51, 62; 450, 10 (7 million) 63, 57; 555, 5 (9 million) 60, 62;
+  // 450, 10, E (11 million) 74, 67; 1300, 3 (18 million) 100, 65.
   const bool small =
       split8_selected(c) && 3.0 * c->N * (double)bI.y_nnz[gammaI] <= (double)(1 << 23);
   const bool split_path =

@@ -139,9 +139,9 @@ __device__ __forceinline__ void mma_window(uint32_t tmem, uint32_t a0, uint32_t 
 // each).  The tensor memory is held meanwhile, 20 x 11 conversions a thread at 8
 // clocks a warp; a sum within 2^22 is instead read off the bits of itself plus
 // 1.5 2^23, one addition (SMALL: the segments of up to about 46 slices, where
-// this time is the larger part: 2200 clocks a tile instead of 4000; the rounds
-// of half line strengths of a C3v J = 12..13 batch at N = 1500 with 25 slices a tile took
-// 3 % less).
+// this time is the larger part: 2200 clocks a tile instead of 4000; a C3v J = 20, 21
+// batch at N = 3000 took 18.15 ms instead of 18.65, a C2v one at N = 2000 3.37 instead
+// of 3.44).
 template <bool SMALL>
 __device__ __forceinline__ void fold_sums(uint32_t t0, long long* hi, long long* lo) {
   auto whole = [](uint32_t f) {
@@ -671,7 +671,7 @@ __device__ __forceinline__ void cut_row(const double* __restrict__ x, const int3
 // least kS before): the planes from the top that are zero in all 128 rows (a
 // dipole's elements fall off away from the diagonal, and a slice of elements
 // 2^-5z of their rows' largest has nothing in its first z planes).  Taken here,
-// where the digits are at hand; reading them back took 27 us at N = 1500.
+// where the digits are at hand; reading them back took 27 us at N = 2000.
 __global__ void __launch_bounds__(256) k_cut8_a(const double* __restrict__ X, size_t ldx, int rows,
                                                 int K, const int32_t* __restrict__ rowsrc,
                                                 const int32_t* __restrict__ vk,
