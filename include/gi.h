@@ -428,8 +428,9 @@ gi_status gi_partition_function(gi_ctx* ctx, double temperature, double* q);
  * evicted together, least recently used first (GI_SERVE_NO_ZCACHE turns the
  * cache off).
  * While serving, gi_set_block / gi_set_block_device / gi_set_params (except
- * precision and split_slices) / gi_submit and the job calls may be used from
- * the context's thread; the other setters and gi_run return GI_ERR_STATE. */
+ * precision and split_slices) / gi_submit, the job calls and the single-vector
+ * calls (gi_half_ls, gi_half_ls_noalloc) may be used from the context's thread;
+ * the other setters and gi_run return GI_ERR_STATE. */
 #define GI_SERVE_NO_ZCACHE 1 /* do not keep initial blocks' half line strengths */
 typedef struct {
   int32_t slots;                /* jobs in flight, one stream each (0: 3) */
